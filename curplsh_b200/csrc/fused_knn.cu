@@ -13,9 +13,9 @@
 // Roles (320 threads, one CTA per SM, persistent over a balanced schedule):
 //   warp 0      TMA producer: query block (resident, or streamed per K chunk)
 //               and database tiles, 128-byte-swizzled, into a stage ring.
-//   warp 1      allocates 512 TMEM columns (two 128x256 f32 accumulators) and,
-//               from one lane, issues tcgen05.mma; commits release stages and
-//               publish accumulators.
+//   warp 1      allocates 512 TMEM columns (two 128x256 f32 accumulators) and
+//               issues tcgen05.mma from one elected lane of a uniform warp;
+//               commits release stages and publish accumulators.
 //   warps 2..9  epilogue: two warpgroups, each owning one 128-column half of
 //               every tile; thread = one query (TMEM lane).  A thread keeps its
 //               own pool and bound; a warp refreshes (radix-selects) a pool that
@@ -544,37 +544,54 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && issuer) {
+    // The whole warp runs this role, so that addresses, descriptors and loop
+    // counters are warp-uniform values (the tensor-core instructions take them
+    // from uniform registers); one elected lane issues.  From a single diverged
+    // lane an MMA took 230-280 cycles of issue, two to four times its
+    // execution, and the issue bound the pass (full pass, diverged -> uniform:
+    // FP8 sphere 28.1 -> 26.8 ms, BF16 integer mixture 3.39 -> 3.22, FP32-exact
+    // 5.89 -> 5.58, d = 960 0.71 -> 0.61).
+    if (issuer) {
+      const bool leader = elect_one();
       constexpr uint32_t fmt = Tr::kFP8 ? 0u : 1u;  // e4m3 : bf16
       // a pair's MMA is 256 rows: this CTA's query block, then the partner's
-      const uint32_t idesc = make_idesc(fmt, fmt, pair ? 2 * kBM : kBM, DUAL ? kBN / 2 : kBN);
+      constexpr uint32_t kM = PAIR ? 2 * kBM : kBM, kN = DUAL ? kBN / 2 : kBN;
+      constexpr uint32_t idesc = make_idesc(fmt, fmt, kM, kN);
       // the FP8 form's BF16 norm tail: the same shape, BF16 operands
-      const uint32_t idesc16 = make_idesc(1u, 1u, pair ? 2 * kBM : kBM, DUAL ? kBN / 2 : kBN);
-      auto mma = [&](uint32_t d_tmem, uint64_t ad, uint64_t bd, uint32_t acc, bool f8) {
-        const uint32_t id = f8 ? idesc : idesc16;
-        if constexpr (PAIR) {
-          if (f8)
-            mma_f8_ss_pair(d_tmem, ad, bd, id, acc);
-          else
-            mma_f16_ss_pair(d_tmem, ad, bd, id, acc);
-        } else {
-          if (f8)
-            mma_f8_ss(d_tmem, ad, bd, id, acc);
-          else
-            mma_f16_ss(d_tmem, ad, bd, id, acc);
-        }
+      constexpr uint32_t idesc16 = make_idesc(1u, 1u, kM, kN);
+      auto mma = [&](uint32_t d_tmem, uint64_t ad, uint64_t bd, uint32_t acc) {
+        if constexpr (PAIR && Tr::kFP8)
+          mma_f8_ss_pair(d_tmem, ad, bd, idesc, acc);
+        else if constexpr (PAIR)
+          mma_f16_ss_pair(d_tmem, ad, bd, idesc, acc);
+        else if constexpr (Tr::kFP8)
+          mma_f8_ss(d_tmem, ad, bd, idesc, acc);
+        else
+          mma_f16_ss(d_tmem, ad, bd, idesc, acc);
+      };
+      auto mma_tail = [&](uint32_t d_tmem, uint64_t ad, uint64_t bd) {
+        if constexpr (PAIR)
+          mma_f16_ss_pair(d_tmem, ad, bd, idesc16, 1u);
+        else
+          mma_f16_ss(d_tmem, ad, bd, idesc16, 1u);
       };
       // completion goes to the barrier at the same offset in both CTAs of a pair
       auto commit = [&](uint64_t* bar) {
-        if constexpr (PAIR)
-          mma_commit_pair(bar);
-        else
-          mma_commit(bar);
+        if (leader) {
+          if constexpr (PAIR)
+            mma_commit_pair(bar);
+          else
+            mma_commit(bar);
+        }
+        __syncwarp();
       };
+      const uint32_t smem_base = smem_u32(smem);
+      const int nreg = L.nkc - (L.tail_narrow ? 1 : 0);
       UnitWalk walk(blockIdx.x, B, rank);
       int ii, qb, t0, t1, u_ord, rot, unit = 0;
       bool gap;
-      uint32_t it = 0, tc = 0;
+      int s = 0;                 // ring stage and its phase
+      uint32_t sphase = 0, tc = 0;
       bool ok = true;
       STAT_DECL(st_full);
       STAT_DECL(st_acc);
@@ -586,6 +603,7 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
           }
           tc_fence_after();
         }
+        const int fp8_tail = Tr::kFP8 ? A.items[ii].fp8_tail : 0;
         for (int t = t0; t < t1 && ok; ++t, ++tc) {
           const uint32_t slot = tc & 1u, use = tc >> 1;
           STAT_BEGIN(ta);
@@ -597,64 +615,57 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
           STAT_END(ta, st_acc);
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + slot * kBN;
-          uint32_t accumulate = 0;
-          const int nreg = L.nkc - (L.tail_narrow ? 1 : 0);
-          const int fp8_tail = Tr::kFP8 ? A.items[ii].fp8_tail : 0;
-          for (int kc = 0; kc < nreg; ++kc, ++it) {
-            const int s = (int)(it % (uint32_t)S);
+          for (int kc = 0; kc < nreg; ++kc) {
             STAT_BEGIN(tf);
-            if (!wait_or_abort(&full[s], (it / S) & 1u, abort_flag)) {
+            if (!wait_or_abort(&full[s], sphase, abort_flag)) {
               raise_abort(abort_flag, B.status, kErrWaitTimeout);
               ok = false;
               break;
             }
             STAT_END(tf, st_full);
             tc_fence_after();
-            const uint32_t st = smem_u32(smem + L.a_bytes + (uint32_t)s * L.stage_bytes);
+            const uint32_t st = smem_base + L.a_bytes + (uint32_t)s * L.stage_bytes;
             const int rem = L.kdim - kc * KC;
-            const int nsteps = rem >= KC ? KC / Tr::kStepElems : (rem + Tr::kStepElems - 1) / Tr::kStepElems;
-            for (int j = 0; j < kQB; ++j) {  // dual: block j accumulates into columns j * 128 of the slot
-              uint32_t acc_j = accumulate;
+            constexpr int kSteps = Tr::kChunkElems / Tr::kStepElems;
+            const int nsteps = (rem + Tr::kStepElems - 1) / Tr::kStepElems;  // >= kSteps: a whole chunk
+            // resident queries: block j's chunk kc; streamed: the stage's own
+            const uint32_t a0 = L.a_stream ? st + stage_a_off<Tr::kAParts, Tr::kBParts>(L, 0)
+                                           : smem_base + a_res_off(L, kc, 0, Tr::kAParts);
+            const bool last = kc == nreg - 1;
+            const uint32_t tl = st + stage_tail_off<Tr::kAParts, Tr::kBParts>(L);
+            const uint32_t at = L.a_stream ? tl + L.b_tail : smem_base + a_res_off(L, nreg, 0, Tr::kAParts);
+            if (leader) {
 #pragma unroll
-              for (int pr = 0; pr < Tr::kProducts; ++pr) {
-                const uint32_t a_addr =
-                    L.a_stream ? st + stage_a_off<Tr::kAParts, Tr::kBParts>(L, Tr::a_part(pr))
-                               : smem_u32(smem + (uint32_t)j * L.a_block + a_res_off(L, kc, Tr::a_part(pr), Tr::kAParts));
-                const uint32_t b_addr = st + Tr::b_part(pr) * L.b_chunk;
-                for (int ks = 0; ks < nsteps; ++ks) {
-                  const uint64_t ad = sw128_kmajor_desc(a_addr + ks * 32);
-                  const uint64_t bd = sw128_kmajor_desc(b_addr + ks * 32);
-                  mma(d_tmem + (uint32_t)j * (kBN / 2), ad, bd, acc_j, Tr::kFP8);
-                  acc_j = 1;
+              for (int j = 0; j < kQB; ++j) {  // dual: block j accumulates into columns j * 128 of the slot
+                const uint32_t dj = d_tmem + (uint32_t)j * (kBN / 2);
+                const uint32_t aj = a0 + (uint32_t)j * L.a_block;
+#pragma unroll
+                for (int pr = 0; pr < Tr::kProducts; ++pr) {
+                  const uint64_t ad = sw128_kmajor_desc(aj + Tr::a_part(pr) * kAChunkBytes);
+                  const uint64_t bd = sw128_kmajor_desc(st + Tr::b_part(pr) * L.b_chunk);
+#pragma unroll
+                  for (int ks = 0; ks < kSteps; ++ks)  // a K step is 32 bytes: descriptor + 2
+                    if (ks < nsteps) mma(dj, ad + 2 * ks, bd + 2 * ks, (pr | ks) ? 1u : (kc ? 1u : 0u));
                 }
+                if (Tr::kFP8 && last && fp8_tail > 0) {
+                  // the BF16 norm tails: one K=16 step at their byte offset in the
+                  // last chunk (a 32-byte K step of the 128-byte swizzled rows, as
+                  // the FP8 steps before it), into the same FP32 accumulator
+                  const uint32_t toff = (uint32_t)(fp8_tail - kc * KC);
+                  mma_tail(dj, sw128_kmajor_desc(aj + toff), sw128_kmajor_desc(st + toff));
+                }
+                // the 16 norm columns: only hi x hi carries them (lo rows are zero
+                // there), so one K step of product 0 with the 32-byte-swizzled tiles
+                if (!Tr::kFP8 && last && L.tail_narrow)
+                  mma_tail(dj, sw32_kmajor_desc(at + (uint32_t)j * L.a_block), sw32_kmajor_desc(tl));
               }
             }
-            accumulate = 1;
-            if (Tr::kFP8 && fp8_tail > 0 && kc == nreg - 1) {
-              // the BF16 norm tails: one K=16 step at their byte offset in the
-              // last chunk (a 32-byte K step of the 128-byte swizzled rows, as
-              // the FP8 steps before it), into the same FP32 accumulator
-              const uint32_t toff = (uint32_t)(fp8_tail - kc * KC);
-              for (int j = 0; j < kQB; ++j) {
-                const uint32_t a_addr =
-                    L.a_stream ? st + stage_a_off<Tr::kAParts, Tr::kBParts>(L, 0)
-                               : smem_u32(smem + (uint32_t)j * L.a_block + a_res_off(L, kc, 0, Tr::kAParts));
-                mma(d_tmem + (uint32_t)j * (kBN / 2), sw128_kmajor_desc(a_addr + toff), sw128_kmajor_desc(st + toff), 1,
-                    false);
-              }
-            }
-            if (L.tail_narrow && kc == nreg - 1) {
-              // the 16 norm columns: only hi x hi carries them (lo rows are zero
-              // there), so one K step of product 0 with the 32-byte-swizzled tiles
-              const uint32_t tl = st + stage_tail_off<Tr::kAParts, Tr::kBParts>(L);
-              for (int j = 0; j < kQB; ++j) {
-                const uint32_t a_addr =
-                    L.a_stream ? tl + L.b_tail
-                               : smem_u32(smem + (uint32_t)j * L.a_block + a_res_off(L, nreg, 0, Tr::kAParts));
-                mma(d_tmem + (uint32_t)j * (kBN / 2), sw32_kmajor_desc(a_addr), sw32_kmajor_desc(tl), 1, false);
-              }
-            }
+            __syncwarp();
             commit(&empty[s]);
+            if (++s == S) {
+              s = 0;
+              sphase ^= 1u;
+            }
           }
           if (!ok) break;
           commit(&acc_full[slot]);
@@ -666,8 +677,10 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
       // both CTAs of a pair: the commit reaches the partner's drain barrier).
       commit(drain);
       mbar_wait(drain, 0);
-      STAT_FLUSH(kStatMmaWaitFull, st_full);
-      STAT_FLUSH(kStatMmaWaitAccEmpty, st_acc);
+      if (lane == 0) {
+        STAT_FLUSH(kStatMmaWaitFull, st_full);
+        STAT_FLUSH(kStatMmaWaitAccEmpty, st_acc);
+      }
     } else if (lane == 0 && pair) {
       // the partner's MMAs also write this CTA's TMEM and read its shared
       // memory: wait for its final commit before the teardown

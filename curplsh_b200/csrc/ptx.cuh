@@ -334,6 +334,13 @@ __device__ __forceinline__ float fmin3(float a, float b, float c) {
   return r;
 }
 
+// One lane of a fully active warp (the same one every time).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
 __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {

@@ -518,7 +518,8 @@ def set_bound_estimate(enabled: bool) -> None:
 
 def estimate_plan_shape(num_rows: int, num_queries: int, kprime: int, num_sms: int = 148):
     """(sample_rows, step, rank) of the sampled bound estimate for a bare search shape
-    (no index or device needed); sample_rows == 0 when that shape uses none."""
+    (no index or device needed); sample_rows == 0 when that shape uses none, or only the
+    light sample of a small k'."""
     a, b, c = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
     _check(_lib.curplsh_estimate_plan_shape(int(num_rows), int(num_queries), int(kprime), int(num_sms),
                                             ctypes.byref(a), ctypes.byref(b), ctypes.byref(c)))

@@ -414,6 +414,15 @@ double binomial_tail(int n, double q, int j) {
 #endif
 constexpr double kEstimateMuMax = CURPLSH_ESTIMATE_MU;
 constexpr double kEstimateMuMin = 8.0;
+// Below kEstimateMuMin expected rows (small k') the rank's relative margin
+// grows (j / mu is 5 at mu = 3, 10 at mu = 1), but 5-20 k' admitted rows are
+// still far fewer than pools without a bound admit: k' (1 + ln(rows / k')) in
+// every unit of the query.  The light sample takes the fraction f of the
+// database that minimises f N + kLightSurvivorRows * (j / f): a survivor costs
+// about as much as this many more sample rows do per query (10^4 queries,
+// 10^6 rows: 0.11 us against 0.2 ns), fewer when the queries do not fill a
+// block.
+constexpr double kLightSurvivorRows = 512.0;
 constexpr double kEstimateFailure = 1e-6;   // per-query failure probability for a uniform sample
 constexpr int kEstimateBlockRows = kHalfN;  // rows per block minimum (one epilogue warp's half tile)
 
@@ -427,17 +436,38 @@ EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms) {
   if (nq < 1 || kp < 1) return e;
   if (n < (1LL << 16) || n < 64LL * kp) return e;  // a short search gains too little
   const long long T = (n + kBN - 1) / kBN;
-  long long tiles = (long long)std::ceil(kEstimateMuMax * (double)n / kp / kBN);
-  tiles = std::min(tiles, T / 10);
-  if ((double)kp * tiles * kBN / (double)n < kEstimateMuMin) return e;  // too small a sample
+  // smallest rank whose failure probability is small enough; 0 if more than
+  // half of the blocks would have to lie under the k'-th distance
+  auto rank_of = [&](long long rows) {
+    const int blocks = (int)(rows / kEstimateBlockRows);
+    const double q0 = -std::expm1(kEstimateBlockRows * std::log1p(-(double)kp / (double)n));
+    int j = 1;
+    while (2 * j <= blocks && binomial_tail(blocks, q0, j) > kEstimateFailure) ++j;
+    return 2 * j > blocks ? 0 : j;
+  };
+  long long tiles = std::min((long long)std::ceil(kEstimateMuMax * (double)n / kp / kBN), T / 10);
+  if ((double)kp * tiles * kBN / (double)n < kEstimateMuMin) {
+    e.light = true;
+    tiles = 0;
+    double best = 0.0;
+    for (int den = 10; den <= 640; den *= 2) {
+      const long long t = T / den;
+      const int j = t > 0 ? rank_of(t * kBN) : 0;
+      if (j == 0) break;  // smaller samples have fewer blocks
+      const double f = (double)t * kBN / (double)n;
+      const double cost = f * (double)n + kLightSurvivorRows * std::min(1.0, nq / (double)kBM) * j / f;
+      if (tiles == 0 || cost < best) {
+        best = cost;
+        tiles = t;
+      }
+    }
+    if (tiles == 0) return e;
+  }
   e.rows = (int)(tiles * kBN);
   e.step = (int)(n / e.rows);  // >= 10; rows j * step < n for every j < rows
   e.blocks = e.rows / kEstimateBlockRows;
-  const double q0 = -std::expm1(kEstimateBlockRows * std::log1p(-(double)kp / (double)n));
-  int j = 1;
-  while (j < e.blocks && binomial_tail(e.blocks, q0, j) > kEstimateFailure) ++j;
-  if (2 * j > e.blocks) return e;
-  e.j = j;
+  e.j = rank_of(e.rows);
+  if (e.j == 0) return e;
   plan_fused(nq, e.rows, num_sms, &e.plan);
   e.on = true;
   return e;
@@ -1255,7 +1285,7 @@ int curplsh_index_estimate_plan(curplsh_index* ix, int64_t num, int k, int preci
   if (ix->n == 0 || !g_bound_estimate.load(std::memory_order_relaxed)) return CURPLSH_OK;
   const bool coarse_on = g_coarse_check.load(std::memory_order_relaxed) != 0;
   const EstimatePlan e = plan_estimate((int)num, ix->n, kprime_for(form, k, rf, ix->n, coarse_on), ix->dres->num_sms);
-  if (e.on) {
+  if (e.on && !e.light) {
     *sample_rows = e.rows;
     *step = e.step;
     *rank = e.j;
@@ -1273,7 +1303,7 @@ int curplsh_estimate_plan_shape(int64_t num_rows, int64_t num_queries, int kprim
   *step = 1;
   *rank = 0;
   const EstimatePlan e = plan_estimate((int)num_queries, num_rows, kprime, num_sms);
-  if (e.on) {
+  if (e.on && !e.light) {
     *sample_rows = e.rows;
     *step = e.step;
     *rank = e.j;

@@ -149,6 +149,7 @@ cudaError_t launch_fused_batch(int form, const FusedItemSpec* specs, const Fused
 // the starting bound of every candidate pool of the full pass.
 struct EstimatePlan {
   bool on = false;
+  bool light = false;  // few expected sample rows: a looser rank from a smaller sample
   int rows = 0;    // sample rows (a multiple of 256)
   int step = 1;    // sample row j is database row j * step
   int blocks = 0;  // B = rows / 128 block minima per query

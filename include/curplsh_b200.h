@@ -300,8 +300,9 @@ int curplsh_tuning_clear(void);
 int curplsh_set_bound_estimate(int enabled);
 int curplsh_get_bound_estimate(int* enabled);
 /* The estimate a search of num_queries queries with this k / precision / rerank factor would
- * use: *sample_rows = 0 when none, else the sample size, its row step and the rank j among the
- * sample_rows / 128 block minima. */
+ * use: the sample size, its row step and the rank j among the sample_rows / 128 block minima;
+ * *sample_rows = 0 when it uses none, or only the light sample of a small k' (fewer than 8
+ * expected rows among the k' nearest). */
 int curplsh_index_estimate_plan(curplsh_index* index, int64_t num_queries, int k, int precision,
                                 int rerank_factor, int* sample_rows, int* step, int* rank);
 /* The same plan for a bare shape (N rows, num_queries queries, k' candidates, num_sms SMs),

@@ -59,16 +59,16 @@ struct MergeArgs {
   MergeItem items[kMergeMaxItems];
   int num_items, d;
   int kp2;      // power of two >= the largest kprime
-  int pre_cap;  // capacity of the prefiltered key buffer (2 * kp2)
-  int lcnt_n;   // room for the largest list count, rounded to 4
+  int pre_cap;  // capacity of the prefiltered key buffer
+  int lcnt_n;   // room for the list offsets, rounded to 4
   int vec4;     // query and database rows allow 16-byte loads
   uint32_t* status;
   const int* run_if;  // non-null: the launch does nothing unless *run_if != 0
 };
 
 // Block-wide radix select: the bound B such that exactly `keep` of the keys
-// visited by `each` are <= B (keys are unique).  `each(f)` calls f(key) for
-// every key of this thread's share.  8-bit digits from the top; stops as soon
+// visited by `each` are <= B (keys are unique).  `each(f)` calls f(key, on) for
+// every key of this thread's share (those with on == false do not count).  8-bit digits from the top; stops as soon
 // as the digit bucket holds exactly the remaining rank.
 template <int T, class Each>
 __device__ uint64_t block_select_bound(Each each, uint32_t keep, uint32_t* hist, uint32_t* warp_tot,
@@ -80,8 +80,8 @@ __device__ uint64_t block_select_bound(Each each, uint32_t keep, uint32_t* hist,
 #pragma unroll
     for (int b = 0; b < (256 / T); ++b) hist[tid * (256 / T) + b] = 0u;
     __syncthreads();
-    each([&](uint64_t key) {
-      if ((key & pmask) == prefix) atomicAdd(&hist[(uint32_t)(key >> shift) & 255u], 1u);
+    each([&](uint64_t key, bool on) {
+      if (on && (key & pmask) == prefix) atomicAdd(&hist[(uint32_t)(key >> shift) & 255u], 1u);
     });
     __syncthreads();
     uint32_t cb[(256 / T)], c = 0;
@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   uint32_t* hist = reinterpret_cast<uint32_t*>(pre + a.pre_cap);  // [256]
   uint32_t* warp_tot = hist + 256;                              // [8]
   uint32_t* misc = warp_tot + 8;                                // [8]
-  int* lcnt = reinterpret_cast<int*>(misc + 8);                 // [lcnt_n]
-  float* qv = reinterpret_cast<float*>(lcnt + a.lcnt_n);        // [d], 16-byte aligned
+  int* loff = reinterpret_cast<int*>(misc + 8);                 // [lcnt_n] list l holds keys [loff[l], loff[l + 1])
+  float* qv = reinterpret_cast<float*>(loff + a.lcnt_n);        // [d], 16-byte aligned
 
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   // smallest k'-th of any pool, or the estimate the pass started from.  When
   // it comes from a pool, every key of the k' smallest has a distance <= it.
   uint32_t qbound = 0xFFFFFFFFu;
-  if (m.q_bound && T > 0 && a.pre_cap > 0) qbound = m.q_bound[prow];
+  if (m.q_bound && T > 0) qbound = m.q_bound[prow];
 
   for (int i = tid; i < d; i += NT) qv[i] = m.queries[(size_t)q * d + i];
   if (tid == 0) {
@@ -167,32 +167,64 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
     misc[6] = 0xFFFFFFFFu;   // min of the same
     misc[7] = 0u;            // largest coarse distance among the candidates, order bits
   }
-  for (int l = tid; l < nlists; l += NT) lcnt[l] = m.pool_counts[list0 + l];
+  // The lists are read as one flattened sequence (list of key i by binary
+  // search in the offsets), four loads in flight per thread: list by list, each
+  // of the up to 148 short lists of a few-query search was a load latency of
+  // its own (merge of 16 queries against 2 x 10^6 rows 164 -> 23 us, of one
+  // query against 10^4 rows 56 -> 19, of 1,000 queries with k = 1,024 312 -> 212).
+  int total = 0;
+  for (int l0 = 0; l0 < nlists; l0 += NT) {
+    const int l = l0 + tid;
+    const uint32_t c = l < nlists ? (uint32_t)m.pool_counts[list0 + l] : 0u;
+    const uint32_t incl = block_incl_scan(c, warp_tot);
+    if (l < nlists) loff[l] = total + (int)(incl - c);
+    if (tid == NT - 1) misc[1] = incl;
+    __syncthreads();
+    total += (int)misc[1];
+    __syncthreads();
+  }
+  if (tid == 0) loff[nlists] = total;
   __syncthreads();
-  auto list_ptr = [&](int l) { return m.pools + (list0 + (size_t)l) * (size_t)m.pool_cap; };
+  constexpr int kLoads = 4;
+  // f(key, on) for this thread's share of the keys, called by whole warps (on =
+  // false past the end and for keys above the final bound)
   auto each_pool_key = [&](auto f) {
-    for (int l = 0; l < nlists; ++l) {
-      const uint64_t* lp = list_ptr(l);
-      for (int o = tid; o < lcnt[l]; o += NT) {
-        const uint64_t key = lp[o];
-        if ((uint32_t)(key >> 32) <= qbound) f(key);
+    for (int i0 = tid; i0 - tid < total; i0 += kLoads * NT) {
+      uint64_t key[kLoads];
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u) {
+        const int i = i0 + u * NT;
+        key[u] = kKeyEmpty;
+        if (i < total) {
+          int l = 0, h = nlists;  // loff[l] <= i < loff[h]
+          while (h - l > 1) {
+            const int mid = (l + h) >> 1;
+            if (loff[mid] <= i)
+              l = mid;
+            else
+              h = mid;
+          }
+          key[u] = m.pools[(list0 + (size_t)l) * (size_t)m.pool_cap + (size_t)(i - loff[l])];
+        }
       }
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u) f(key[u], i0 + u * NT < total && (uint32_t)(key[u] >> 32) <= qbound);
     }
   };
+  // appends `key` of the warp's lanes with `on` to buf (capacity cap), counted in *n
+  auto append = [&](uint64_t key, bool on, uint64_t* buf, int cap, uint32_t* n) {
+    const uint32_t bal = __ballot_sync(0xffffffffu, on);
+    if (!bal) return;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(n, (uint32_t)__popc(bal));
+    const uint32_t pos = __shfl_sync(0xffffffffu, base, 0) + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+    if (on && pos < (uint32_t)cap) buf[pos] = key;
+  };
 
-  // ---- 1. keys under the final bound, compacted into shared memory (when
-  // this launch's pools can carry bounds at all)
-  int cnt = 0;
-  if (a.pre_cap > 0) {
-    each_pool_key([&](uint64_t key) {
-      const uint32_t pos = atomicAdd(&misc[0], 1u);
-      if (pos < (uint32_t)a.pre_cap) pre[pos] = key;
-    });
-    __syncthreads();
-    cnt = (int)misc[0];
-  } else {
-    for (int l = 0; l < nlists; ++l) cnt += lcnt[l];
-  }
+  // ---- 1. keys under the final bound, compacted into shared memory
+  each_pool_key([&](uint64_t key, bool on) { append(key, on, pre, a.pre_cap, &misc[0]); });
+  __syncthreads();
+  const int cnt = (int)misc[0];
   // Started from an estimate E: every row with a key under E was admitted, so
   // k' keys under the final bound (<= E) prove that the k' smallest keys of
   // the whole database are among the candidates (their k'-th is then <= E, and
@@ -210,27 +242,17 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
     if (cnt <= a.pre_cap)
       bound = block_select_bound<NT>(
           [&](auto f) {
-            for (int i = tid; i < cnt; i += NT) f(pre[i]);
+            for (int i = tid; i < cnt; i += NT) f(pre[i], true);
           },
           (uint32_t)keep, hist, warp_tot, misc);
     else
       bound = block_select_bound<NT>(each_pool_key, (uint32_t)keep, hist, warp_tot, misc);
   }
+  auto take = [&](uint64_t key, bool on) { append(key, on && key <= bound, cand, a.kp2, &misc[4]); };
   if (cnt <= a.pre_cap) {
-    for (int i = tid; i < cnt; i += NT) {
-      const uint64_t key = pre[i];
-      if (key <= bound) {
-        const uint32_t pos = atomicAdd(&misc[4], 1u);
-        if (pos < (uint32_t)a.kp2) cand[pos] = key;
-      }
-    }
+    for (int i = tid; i - tid < cnt; i += NT) take(i < cnt ? pre[i] : kKeyEmpty, i < cnt);
   } else {
-    each_pool_key([&](uint64_t key) {
-      if (key <= bound) {
-        const uint32_t pos = atomicAdd(&misc[4], 1u);
-        if (pos < (uint32_t)a.kp2) cand[pos] = key;
-      }
-    });
+    each_pool_key(take);
   }
   __syncthreads();
   int kept = (int)misc[4];
@@ -434,19 +456,11 @@ cudaError_t launch_merge_batch(MergeItem* items, int n, int d, uint32_t* status,
   int kp2 = 32;  // >= 32 keeps the shared-memory carve 16-byte aligned
   while (kp2 < kpmax) kp2 <<= 1;
   a.kp2 = kp2;
-  // A pool can bound the k'-th distance only if a unit covers at least k'
-  // rows; without such pools there is nothing to prefilter with, and the
-  // launch keeps the smaller shared-memory footprint (higher occupancy).
-  bool bounded = false;
-  for (int i = 0; i < n; ++i) {
-    long long len = std::min<long long>(items[i].split_tiles, items[i].work_per_cta);
-    len = std::min<long long>(len, items[i].num_tiles);
-    bounded = bounded || (items[i].q_bound && len * kBN >= items[i].kprime);
-    // the estimate check counts the keys under the final bound
-    bounded = bounded || (items[i].q_bound && (items[i].checks & kCheckEstimate));
-  }
-  a.pre_cap = bounded ? 2 * kp2 : 0;
-  a.lcnt_n = (umax + 3) & ~3;
+  // Room for the keys that pass the final bound: two k', at least 1,024 (8 KB,
+  // which 12 CTAs per SM still have) so that searches with small k' select from
+  // shared memory too.
+  a.pre_cap = std::max(2 * kp2, 1024);
+  a.lcnt_n = (umax + 1 + 3) & ~3;
   bool vec4 = d % 4 == 0;
   for (int i = 0; i < n; ++i)
     vec4 = vec4 && (reinterpret_cast<uintptr_t>(items[i].queries) & 15) == 0 &&

@@ -379,7 +379,7 @@ struct Timing {
 // per pool survive the filter, and appending and selecting survivors is most
 // of the fused pass's time.  A short first pass over a strided sample of the
 // database (rows 0, s, 2s, ...; same form) records, per query, the smallest
-// coarse distance of every 128-row block of the sample (no pools, no
+// coarse distance of every block of 128 (or 8) rows of the sample (no pools, no
 // survivors), and the j-th smallest of those B block minima becomes the
 // starting bound E of every pool of the full pass.  If a fraction p of the
 // database lies under a distance x, a block's minimum is under x with
@@ -390,6 +390,8 @@ struct Timing {
 // k' candidates lie under the final bound, the k' nearest rows are among them
 // (see merge_rerank.cu), otherwise the query is searched again without an
 // estimate.  Results never depend on E.
+
+constexpr double kEstimateFailure = 1e-6;  // per-query failure probability for a uniform sample
 
 // P(X >= j) for X ~ Binomial(n, q).
 double binomial_tail(int n, double q, int j) {
@@ -406,6 +408,25 @@ double binomial_tail(int n, double q, int j) {
   return t;
 }
 
+// Smallest rank j <= most * n with exp(-n KL(j / n || q)) <= kEstimateFailure, a
+// bound of P(X >= j) for j / n >= q that costs two logarithms (one or two ranks
+// above the exact tail's); 0 if there is none.
+int chernoff_rank(int n, double q, double most) {
+  auto small = [&](int j) {
+    const double p = (double)j / n;
+    if (p <= q) return false;
+    const double kl = p * std::log(p / q) + (p < 1.0 ? (1.0 - p) * std::log((1.0 - p) / (1.0 - q)) : 0.0);
+    return n * kl >= -std::log(kEstimateFailure);
+  };
+  int lo = (int)(q * n), hi = (int)(most * n);  // small(hi) and not small(lo)
+  if (hi < 1 || hi <= lo || !small(hi)) return 0;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    (small(mid) ? hi : lo) = mid;
+  }
+  return hi;
+}
+
 // mu = expected sample rows among a query's k' nearest.  A larger sample gives
 // a tighter rank (j / mu falls from ~2.6 at mu = 12 to ~2 at 24) but costs
 // more; the sample pass takes at most a tenth of the full pass's tiles.
@@ -414,17 +435,25 @@ double binomial_tail(int n, double q, int j) {
 #endif
 constexpr double kEstimateMuMax = CURPLSH_ESTIMATE_MU;
 constexpr double kEstimateMuMin = 8.0;
-// Below kEstimateMuMin expected rows (small k') the rank's relative margin
-// grows (j / mu is 5 at mu = 3, 10 at mu = 1), but 5-20 k' admitted rows are
-// still far fewer than pools without a bound admit: k' (1 + ln(rows / k')) in
-// every unit of the query.  The light sample takes the fraction f of the
-// database that minimises f N + kLightSurvivorRows * (j / f): a survivor costs
-// about as much as this many more sample rows do per query (10^4 queries,
-// 10^6 rows: 0.11 us against 0.2 ns), fewer when the queries do not fill a
-// block.
+// Other shapes (small k', few rows, or k' a large share of the rows) take the
+// sample that minimises  f N + kLightSurvivorRows * admitted rows  over
+// fractions f of the database.  The rank's relative margin grows with fewer
+// expected rows (j / mu is 5 at mu = 3, 10 at mu = 1), but even 10 k' admitted
+// rows are far fewer than pools without a bound admit: k' (1 + ln(rows / k'))
+// in every unit of the query.  A survivor costs about as much as this many
+// more sample rows do per query (10^4 queries, 10^6 rows: 0.11 us against
+// 0.2 ns), fewer when the queries do not fill a block.
 constexpr double kLightSurvivorRows = 512.0;
-constexpr double kEstimateFailure = 1e-6;   // per-query failure probability for a uniform sample
 constexpr int kEstimateBlockRows = kHalfN;  // rows per block minimum (one epilogue warp's half tile)
+// Where k' is a large share of the rows most 128-row blocks hold one of the k'
+// nearest and their minima tell little; the filter's minima of eight rows do.
+constexpr int kEstimateFineRows = 8;
+constexpr int kEstimateFineMaxTiles = 64;  // 2,048 minima per query
+// Shorter searches are one or two tiles per CTA either way; from about here on the
+// sample pays (FP32-exact, d = 128, k = 10, with -> without: 3,000 rows 1 query
+// 70 -> 65 us, 16 queries 70 -> 100; 10^4 rows 66 -> 70 and 71 -> 129, 100
+// queries 76 -> 182; 40,000 rows 1 query 76 -> 151).
+constexpr long long kEstimateMinRows = 2048;
 
 }  // namespace
 
@@ -433,41 +462,47 @@ namespace curplsh_b200 {
 // caller reads the process-wide switch once per search).
 EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms) {
   EstimatePlan e;
-  if (nq < 1 || kp < 1) return e;
-  if (n < (1LL << 16) || n < 64LL * kp) return e;  // a short search gains too little
+  if (nq < 1 || kp < 1 || n < kEstimateMinRows || n < 4LL * kp) return e;
   const long long T = (n + kBN - 1) / kBN;
-  // smallest rank whose failure probability is small enough; 0 if more than
-  // half of the blocks would have to lie under the k'-th distance
-  auto rank_of = [&](long long rows) {
-    const int blocks = (int)(rows / kEstimateBlockRows);
-    const double q0 = -std::expm1(kEstimateBlockRows * std::log1p(-(double)kp / (double)n));
-    int j = 1;
-    while (2 * j <= blocks && binomial_tail(blocks, q0, j) > kEstimateFailure) ++j;
-    return 2 * j > blocks ? 0 : j;
-  };
+  auto under = [&](int block_rows) { return -std::expm1(block_rows * std::log1p(-(double)kp / (double)n)); };
   long long tiles = std::min((long long)std::ceil(kEstimateMuMax * (double)n / kp / kBN), T / 10);
-  if ((double)kp * tiles * kBN / (double)n < kEstimateMuMin) {
+  int block_rows = kEstimateBlockRows, j = 0;
+  if (n >= (1LL << 16) && n >= 64LL * kp && (double)kp * tiles * kBN / (double)n >= kEstimateMuMin) {
+    // smallest rank whose failure probability is small enough, among at most half of the blocks
+    const int blocks = (int)(tiles * kBN / block_rows);
+    const double q0 = under(block_rows);
+    j = 1;
+    while (2 * j <= blocks && binomial_tail(blocks, q0, j) > kEstimateFailure) ++j;
+    if (2 * j > blocks) j = 0;
+  }
+  if (j == 0) {
     e.light = true;
-    tiles = 0;
     double best = 0.0;
-    for (int den = 10; den <= 640; den *= 2) {
+    for (int den = 2; den <= 640; den *= 2) {
       const long long t = T / den;
-      const int j = t > 0 ? rank_of(t * kBN) : 0;
-      if (j == 0) break;  // smaller samples have fewer blocks
-      const double f = (double)t * kBN / (double)n;
-      const double cost = f * (double)n + kLightSurvivorRows * std::min(1.0, nq / (double)kBM) * j / f;
-      if (tiles == 0 || cost < best) {
+      if (t < 1) break;
+      int br = kEstimateBlockRows;
+      int r = chernoff_rank((int)(t * kBN / br), under(br), 0.5);
+      if (r == 0 && t <= kEstimateFineMaxTiles)
+        r = chernoff_rank((int)(t * kBN / kEstimateFineRows), under(br = kEstimateFineRows), 0.9);
+      if (r == 0) continue;
+      const double blocks = (double)(t * kBN / br);
+      const double admitted = (double)n * -std::expm1(std::log1p(-r / blocks) / br);
+      const double cost = (double)t * kBN + kLightSurvivorRows * std::min(1.0, nq / (double)kBM) * admitted;
+      if (j == 0 || cost < best) {
         best = cost;
         tiles = t;
+        block_rows = br;
+        j = r;
       }
     }
-    if (tiles == 0) return e;
+    if (j == 0) return e;
   }
   e.rows = (int)(tiles * kBN);
-  e.step = (int)(n / e.rows);  // >= 10; rows j * step < n for every j < rows
-  e.blocks = e.rows / kEstimateBlockRows;
-  e.j = rank_of(e.rows);
-  if (e.j == 0) return e;
+  e.step = (int)(n / e.rows);  // rows i * step < n for every i < rows
+  e.block_rows = block_rows;
+  e.blocks = e.rows / block_rows;
+  e.j = j;
   plan_fused(nq, e.rows, num_sms, &e.plan);
   e.on = true;
   return e;
@@ -500,10 +535,11 @@ SearchShape search_shape(const curplsh_index* ix, int nq, int k, int form, int r
   sh.kp = kprime_for(form, k, rerank_factor, ix->n, coarse_on);
   const TuneParams tp = tune_lookup(form, ix->dim, k, nq);
   sh.P = pool_capacity(sh.kp, tp.headroom);
-  plan_fused(nq, (int)ix->n, ix->dres->num_sms, &sh.plan, default_split_q4(tp, sh.P), form, ix->dim);
+  if (allow_est) sh.est = plan_estimate(nq, ix->n, sh.kp, ix->dres->num_sms);
+  plan_fused(nq, (int)ix->n, ix->dres->num_sms, &sh.plan, default_split_q4(tp, sh.P), form, ix->dim,
+             sh.est.on ? 0 : sh.kp);
   sh.nq_pad = round_up(nq, kBM);
   sh.pool_lists = (size_t)sh.plan.pool_rows() * sh.plan.units_per_block;
-  if (allow_est) sh.est = plan_estimate(nq, ix->n, sh.kp, ix->dres->num_sms);
   sh.coarse = coarse_check_applies(ix, form, sh.kp, coarse_on);
   return sh;
 }
@@ -572,8 +608,7 @@ cudaError_t fused_stats_print(const char* label, const FusedLaunch& f, cudaStrea
 #endif
 
 // The search proper.  Device-side inputs/outputs; `st` orders everything.
-// With `allow_est` a sampled bound estimate may be used, with `coarse_on` the
-// BF16/FP8 forms check their coarse margin; when either applies, *fail_out
+// When the shape has a sampled bound estimate or a coarse-margin check, *fail_out
 // points at the device list of queries that failed a check ([0] count, then
 // indices), which the caller must search again (else *fail_out is null).
 // With `dev_recheck` (and no coarse check) a failed estimate is handled on the
@@ -581,9 +616,8 @@ cudaError_t fused_stats_print(const char* label, const FusedLaunch& f, cudaStrea
 // run again from no bound for the whole batch (rare: the estimate fails with
 // probability ~1e-6 per query), the failures are counted on the device, and
 // *fail_out stays null, so the caller need not synchronise.
-int search_device(curplsh_index* ix, int nq, const float* q_dev, int k, int form, int rerank_factor, int* out_idx,
-                  float* out_dist, cudaStream_t st, char* extra_base, Timing* tm, bool allow_est, bool coarse_on,
-                  int** fail_out, bool dev_recheck) {
+int search_device(curplsh_index* ix, const SearchShape& sh, int nq, const float* q_dev, int k, int form, int* out_idx,
+                  float* out_dist, cudaStream_t st, char* extra_base, Timing* tm, int** fail_out, bool dev_recheck) {
   const int d = ix->dim;
   *fail_out = nullptr;
   if (ix->n == 0) {
@@ -594,7 +628,6 @@ int search_device(curplsh_index* ix, int nq, const float* q_dev, int k, int form
     int rc = build_fp8(ix, st);
     if (rc) return rc;
   }
-  const SearchShape sh = search_shape(ix, nq, k, form, rerank_factor, allow_est, coarse_on);
   const int kp = sh.kp, P = sh.P;
   const FusedPlan& plan = sh.plan;
   const long long nq_pad = sh.nq_pad;
@@ -640,6 +673,7 @@ int search_device(curplsh_index* ix, int nq, const float* q_dev, int k, int form
     e.db_step = sh.est.step;
     e.kprime = 1;
     e.minima = b.minima;
+    e.minima_rows = sh.est.block_rows;
     e.plan = sh.est.plan;
 #ifdef CURPLSH_FUSED_STATS
     CUDA_TRY(fused_stats_begin(&e, st));
@@ -712,10 +746,8 @@ int search_device(curplsh_index* ix, int nq, const float* q_dev, int k, int form
   return CURPLSH_OK;
 }
 
-size_t search_workspace_bytes(const curplsh_index* ix, int nq, int k, int form, int rerank_factor,
-                              bool allow_est, bool coarse_on) {
+size_t search_workspace_bytes(const curplsh_index* ix, const SearchShape& sh, int nq, int form) {
   if (ix->n == 0) return 0;
-  const SearchShape sh = search_shape(ix, nq, k, form, rerank_factor, allow_est, coarse_on);
   Carve c(nullptr);
   SearchBufs b;
   return carve_search(c, ix, sh, nq, form, &b) + 256;
@@ -730,7 +762,8 @@ int search_failed(curplsh_index* ix, int nf, const int* fail_dev, const float* q
   const int form = kFormExact;
   const size_t qbytes = (size_t)round_up((long long)nf * d * sizeof(float), 256);
   const size_t obytes = (size_t)round_up((long long)nf * k * (sizeof(int) + sizeof(float)), 256);
-  const size_t core = search_workspace_bytes(ix, nf, k, form, rerank_factor, false, false);
+  const SearchShape sh = search_shape(ix, nf, k, form, rerank_factor, false, false);
+  const size_t core = search_workspace_bytes(ix, sh, nf, form);
   cudaError_t e = w.fb.ensure(qbytes + obytes + core);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -744,8 +777,7 @@ int search_failed(curplsh_index* ix, int nf, const int* fail_dev, const float* q
   CUDA_TRY(launch_gather_rows(q_dev, d, fail_dev + 2, nf, qf, st));
   Timing none;
   int* again = nullptr;
-  int rc = search_device(ix, nf, qf, k, form, rerank_factor, oif, odf, st, base + qbytes + obytes, &none, false,
-                         false, &again, false);
+  int rc = search_device(ix, sh, nf, qf, k, form, oif, odf, st, base + qbytes + obytes, &none, &again, false);
   if (rc) return rc;
   CUDA_TRY(launch_scatter_results(oif, odf, fail_dev + 2, nf, k, out_idx, out_dist, st));
   return CURPLSH_OK;
@@ -786,10 +818,10 @@ int do_search(curplsh_index* ix, int64_t num, const float* queries, int k, int p
   // is always the host's: a query it lists is searched again in the exact form
   // before the call returns.
   const bool coarse_on = g_coarse_check.load(std::memory_order_relaxed) != 0;
-  const int kp = ix->n > 0 ? kprime_for(form, k, rf, ix->n, coarse_on) : 0;
-  const bool est = g_bound_estimate.load(std::memory_order_relaxed) && ix->n > 0 &&
-                   plan_estimate(nq, ix->n, kp, ix->dres->num_sms).on;
-  const bool coarse = coarse_check_applies(ix, form, kp, coarse_on);
+  SearchShape sh;
+  if (ix->n > 0)
+    sh = search_shape(ix, nq, k, form, rf, g_bound_estimate.load(std::memory_order_relaxed) != 0, coarse_on);
+  const bool est = sh.est.on, coarse = sh.coarse;
   const bool all_dev = q_dev && i_dev && d_dev;
   const bool dev_recheck = est && !coarse && all_dev && !force_sync;
   const bool sync = force_sync || (est && !dev_recheck) || coarse || !all_dev;
@@ -803,7 +835,7 @@ int do_search(curplsh_index* ix, int64_t num, const float* queries, int k, int p
   }
   StreamWorkspace& w = *wp;
   std::lock_guard<std::mutex> wlk(w.mu);
-  const size_t core = search_workspace_bytes(ix, nq, k, form, rf, est, coarse);
+  const size_t core = search_workspace_bytes(ix, sh, nq, form);
   const size_t qbytes = q_dev ? 0 : (size_t)nq * ix->dim * sizeof(float);
   const size_t obytes = (i_dev && d_dev) ? 0 : (size_t)nq * k * (sizeof(int) + sizeof(float));
   const size_t total = (size_t)round_up((long long)qbytes, 256) + (size_t)round_up((long long)obytes, 256) + core;
@@ -836,7 +868,7 @@ int do_search(curplsh_index* ix, int64_t num, const float* queries, int k, int p
   if (!q_dev)
     CUDA_TRY(cudaMemcpyAsync(const_cast<float*>(qd), queries, qbytes, cudaMemcpyDefault, st));
   int* fail = nullptr;
-  int rc = search_device(ix, nq, qd, k, form, rf, oi, od, st, base + off, &tm, est, coarse, &fail, dev_recheck);
+  int rc = search_device(ix, sh, nq, qd, k, form, oi, od, st, base + off, &tm, &fail, dev_recheck);
   if (rc) return rc;
   auto copy_out = [&]() -> int {
     if (!(i_dev && d_dev)) {

@@ -73,18 +73,7 @@ constexpr int kNumThreads = 320;  // warp 0 TMA producer, warp 1 MMA issuer, war
 // terms), query rows (stored as -2q) carry [1 1 1 m1 m2 m3] (||q||^2 = m1+m2+m3),
 // and the accumulator is ||q||^2 + ||x||^2 - 2 q.x directly.
 constexpr int kAugCols = 6;
-constexpr int kEpiWarps = 8;
-// Epilogue warps of the candidate-pool kernel, a build option: 8 or 12 (two or
-// three per TMEM lane group; with 12 the block of 14 warps caps registers at
-// 128 a thread).  The block-minimum kernel keeps 8.
-#ifndef CURPLSH_EPI_WARPS
-#define CURPLSH_EPI_WARPS 8
-#endif
-constexpr int kPoolEpiWarps = CURPLSH_EPI_WARPS;
-static_assert(kPoolEpiWarps == 8 || kPoolEpiWarps == 12, "8 or 12 epilogue warps");
-constexpr int kMaxEpiWarps = 12;
-__host__ __device__ constexpr int epi_warps_for(bool minima) { return minima ? kEpiWarps : kPoolEpiWarps; }
-__host__ __device__ constexpr int threads_for(bool minima) { return 64 + 32 * epi_warps_for(minima); }
+constexpr int kEpiWarps = 8;  // two per TMEM lane group
 constexpr int kPoolRoom = kBN;  // free slots a candidate pool keeps for the next tile (both halves)
 // Tiles between two selection points of a shared candidate pool: two when the
 // capacity leaves room for two tiles of appends above k' + 128, else one.
@@ -120,9 +109,11 @@ struct FusedItem {
   // the tails adds ||x||^2 / (-2 s_q s) to the FP8 accumulator, which then is
   // (||x||^2 - 2 q.x) / (-2 s_q s): no database norm is loaded per tile.
   int fp8_tail;
-  // Non-null: block-minimum mode (no pools): minima[q * 2 * num_tiles + 2 * t + h]
-  // gets the smallest key distance of query q over rows [256 t + 128 h, +128).
+  // Non-null: block-minimum mode (no pools): minima[q * B + b] gets the smallest
+  // key distance of query q over rows [b * minima_rows, +minima_rows) of the
+  // B = 256 num_tiles / minima_rows blocks.
   float* minima;
+  int minima_rows;         // 128 or 8
 };
 
 // Tensor maps of one item, in this order.

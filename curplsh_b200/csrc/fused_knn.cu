@@ -13,16 +13,19 @@
 // Roles (320 threads, one CTA per SM, persistent over a balanced schedule):
 //   warp 0      TMA producer: query block (resident, or streamed per K chunk)
 //               and database tiles, 128-byte-swizzled, into a stage ring.
-//   warp 1      allocates 512 TMEM columns (two 128x256 f32 accumulators) and
-//               issues tcgen05.mma from one elected lane of a uniform warp;
-//               commits release stages and publish accumulators.
-//   warps 2..9  epilogue: two warpgroups, each owning one 128-column half of
-//               every tile; thread = one query (TMEM lane).  A thread keeps its
-//               own pool and bound; a warp refreshes (radix-selects) a pool that
-//               is about to overflow, keeping the k' smallest (distance, row)
-//               keys, and publishes the tightened bound to the shared per-query
-//               bound array so other CTAs working on the same queries filter
-//               harder.
+//   warp 1      allocates 512 TMEM columns (two accumulator slots of 128 x 256,
+//               or with dual blocks of two 128 x 128) and issues tcgen05.mma from
+//               one elected lane of a uniform warp; commits release stages and
+//               publish accumulators.
+//   warps 2..9  epilogue: two warpgroups; thread = one query (TMEM lane).  With
+//               dual blocks each warpgroup owns one query block, else one
+//               128-column half of every tile.  A warp takes the minimum of
+//               every eight columns, and only where one is under its query's
+//               bound looks at the columns and appends survivors to the pool; it
+//               radix-selects a pool that is about to overflow, keeping the k'
+//               smallest (distance, row) keys, and publishes the tightened bound
+//               to the shared per-query bound array so other CTAs working on the
+//               same queries filter harder.
 //
 // Schedule: the (query block, database tile) space is flattened and split into
 // equal contiguous ranges, one per CTA, so the work is balanced to one tile for
@@ -117,8 +120,9 @@ __host__ __device__ inline SmemLayout make_layout(int form, int d, int pair = 0,
   // the tail runs the hi x hi product alone, which is exact only for those
   L.tail_narrow = folded && (d % 64 == 0);
   // everything below the barrier block must fit the 227 KB opt-in limit
-  const uint32_t pool_bytes = dual ? 2048u : 1024u;  // pool counts and bounds of 128 (dual: 256) rows
-  const uint32_t budget = 227u * 1024u - 256u - (uint32_t)epi_warps * 256u * 4u - pool_bytes - 1024u;
+  const uint32_t pool_bytes = dual ? 0u : 1024u;  // counts and bounds of 128 shared pools
+  const uint32_t warp_bytes = (uint32_t)epi_warps * 1024u;  // radix histograms
+  const uint32_t budget = 227u * 1024u - 256u - warp_bytes - pool_bytes - 1024u;
   const int nreg = L.nkc - (L.tail_narrow ? 1 : 0);
   const uint32_t a_one = (uint32_t)nreg * a_parts * kAChunkBytes + (L.tail_narrow ? kATailBytes : 0u);
   L.a_block = (a_one + 1023u) & ~1023u;
@@ -139,7 +143,7 @@ __host__ __device__ inline SmemLayout make_layout(int form, int d, int pair = 0,
   L.stages = s < 2 ? 2 : (s > 8 ? 8 : s);
   L.bar_off = L.a_bytes + (uint32_t)L.stages * L.stage_bytes;
   L.hist_off = L.bar_off + 256;  // barriers: 2*8 + 6 mbarriers + tmem slot + flags < 256 B
-  L.pool_off = L.hist_off + epi_warps * 256 * 4;
+  L.pool_off = L.hist_off + warp_bytes;
   L.total = L.pool_off + pool_bytes + 1024;
   return L;
 }
@@ -229,7 +233,9 @@ struct UnitWalk {
 __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                               bool cl = false) {
   auto poll = [&]() { return cl ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
-  if (poll()) return true;
+  // the timer is read only once a wait has already gone on for a while
+  for (int i = 0; i < 16; ++i)
+    if (poll()) return true;
   const uint64_t t0 = globaltimer_ns();
   for (uint32_t i = 0; i < kWaitPollLimit; ++i) {
     if (poll()) return true;
@@ -279,19 +285,18 @@ __device__ __forceinline__ float thr_from(float dstar, float qn) {
 #define STAT_FLUSH(slot, acc)
 #endif
 
-// Survivor masks from sign bits.  With u = the float just above thr, a column
-// survives iff d < u, i.e. d <= thr.  t = d - u is formed two columns at a time
-// by one packed FMA (d * 1 - u: exact product, one rounding), and its sign bit
-// is exactly the test: rounding never changes the sign of a nonzero difference,
-// d == u gives +0, and a NaN distance gives a NaN with the sign clear, so it
-// never survives, as with a compare.  The sign bits enter the mask by funnel
-// shifts, four consecutive columns per chain, so bit j belongs to column j: a
-// packed FMA per two columns and a shift per column, against a compare, a
-// select and an or per column.
+// The filter admits a column iff its distance is <= thr.  With u = the float just
+// above thr that is d < u, and for the scaled FP8 form (d = km x, km > 0) the sign
+// of fma(km, x, -u): one rounding never changes the sign of a nonzero
+// difference, km x == u gives +0, and a NaN never passes, as with a compare.
 __device__ __forceinline__ float next_above(float x) {
   const uint32_t u = __float_as_uint(x);
   if (u == 0x80000000u) return __uint_as_float(1u);  // -0: the smallest positive subnormal
   return __uint_as_float((int32_t)u >= 0 ? u + 1u : u - 1u);
+}
+template <bool kScaled>
+__device__ __forceinline__ bool passes(float x, float km, float u) {
+  return kScaled ? fmaf(km, x, -u) < 0.f : x < u;
 }
 // (acc << 1) | (t >> 31)
 __device__ __forceinline__ uint32_t shl1_sign(uint32_t acc, uint32_t t) {
@@ -299,74 +304,28 @@ __device__ __forceinline__ uint32_t shl1_sign(uint32_t acc, uint32_t t) {
   asm("shf.l.wrap.b32 %0, %1, %2, 1;" : "=r"(r) : "r"(t), "r"(acc));
   return r;
 }
-// bit j set iff km dv[j] < u, computed exactly (one rounding of km dv[j] - u
-// keeps its sign); u = next_above(thr) makes it km dv[j] <= thr for km = 1.
-// The sign bits are gathered by 32 / L funnel-shift chains of length L and
-// joined: fewer instructions beat the extra chain parallelism at two epilogue
-// warps per sub-partition (chains of 4 -> 16: BF16 pass 3.48 -> 3.37 ms; the
-// FP8 pass gains again from 16 -> 32, 30.1 -> 28.1 ms, BF16 loses 1 %).
-template <int L>
-__device__ __forceinline__ uint32_t survive_mask32(const float (&dv)[32], float km, float u) {
-  float t[32];
+// bit j set iff km x[j] < u, j < N: a packed FMA per two columns, the sign bits
+// gathered by one chain of funnel shifts
+template <int N>
+__device__ __forceinline__ uint32_t survive_mask(const float* x, float km, float u) {
+  float t[N];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) fma2_f32(t[2 * i], t[2 * i + 1], dv[2 * i], dv[2 * i + 1], km, km, -u, -u);
-  // 32 / L independent chains of L funnel shifts, then their L-bit pieces joined
-  uint32_t c[32 / L];
+  for (int i = 0; i < N / 2; ++i) fma2_f32(t[2 * i], t[2 * i + 1], x[2 * i], x[2 * i + 1], km, km, -u, -u);
+  uint32_t a = __float_as_uint(t[N - 1]) >> 31;
 #pragma unroll
-  for (int p = 0; p < 32 / L; ++p) {
-    uint32_t a = __float_as_uint(t[L * p + L - 1]) >> 31;
-#pragma unroll
-    for (int i = L - 2; i >= 0; --i) a = shl1_sign(a, __float_as_uint(t[L * p + i]));
-    c[p] = a;  // bit i = sign of t[L p + i]
-  }
-#pragma unroll
-  for (int w = 1; w < 32 / L; w <<= 1)
-#pragma unroll
-    for (int p = 0; p + w < 32 / L; p += 2 * w) c[p] |= c[p + w] << (L * w);
-  return c[0];
+  for (int i = N - 2; i >= 0; --i) a = shl1_sign(a, __float_as_uint(t[i]));
+  return a;
 }
-
-// bit j set iff dv[j] <= thr, by compare, select and or: eight independent
-// partial masks
-__device__ __forceinline__ uint32_t survive_mask32_cmp(const float (&dv)[32], float thr) {
-  uint32_t pa[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-#pragma unroll
-  for (int j = 0; j < 32; ++j) pa[j & 7] |= (dv[j] <= thr ? 1u : 0u) << j;
-  return ((pa[0] | pa[1]) | (pa[2] | pa[3])) | ((pa[4] | pa[5]) | (pa[6] | pa[7]));
+// smallest of 8 (NaN ignored): four instructions
+__device__ __forceinline__ float min8(const float* x) {
+  return fminf(fmin3(fmin3(fmin3(x[0], x[1], x[2]), x[3], x[4]), x[5], x[6]), x[7]);
 }
-
-// 1: a chunk's masks are built only when some lane's smallest distance of the
-// 64 columns (a three-input min tree, 32 instructions) passes.
-#ifndef CURPLSH_MIN_FIRST
-#define CURPLSH_MIN_FIRST 0
-#endif
-__device__ __forceinline__ float min64(const float (&a)[32], const float (&b)[32]) {
-  float r[22];
-#pragma unroll
-  for (int i = 0; i < 10; ++i) r[i] = fmin3(a[3 * i], a[3 * i + 1], a[3 * i + 2]);
-  r[10] = fmin3(a[30], a[31], b[0]);
-#pragma unroll
-  for (int i = 0; i < 10; ++i) r[11 + i] = fmin3(b[1 + 3 * i], b[2 + 3 * i], b[3 + 3 * i]);
-  r[21] = b[31];
-  float s[8];
-#pragma unroll
-  for (int i = 0; i < 7; ++i) s[i] = fmin3(r[3 * i], r[3 * i + 1], r[3 * i + 2]);
-  s[7] = r[21];
-  return fminf(fmin3(s[0], s[1], s[2]), fmin3(s[3], s[4], fmin3(s[5], s[6], s[7])));
-}
-
-// v[j] for a runtime j in [0, 32) without local memory: a 5-level select tree.
-__device__ __forceinline__ float select32(const float (&v)[32], int j) {
-  float a[16], b[8], c[4], d2[2];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) a[i] = (j & 16) ? v[i + 16] : v[i];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) b[i] = (j & 8) ? a[i + 8] : a[i];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) c[i] = (j & 4) ? b[i + 4] : b[i];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) d2[i] = (j & 2) ? c[i + 2] : c[i];
-  return (j & 1) ? d2[1] : d2[0];
+// x[j] for a runtime j in [0, 8) without local memory: a 3-level select tree
+__device__ __forceinline__ float select8(const float* x, int j) {
+  const float a0 = (j & 4) ? x[4] : x[0], a1 = (j & 4) ? x[5] : x[1];
+  const float a2 = (j & 4) ? x[6] : x[2], a3 = (j & 4) ? x[7] : x[3];
+  const float b0 = (j & 2) ? a2 : a0, b1 = (j & 2) ? a3 : a1;
+  return (j & 1) ? b1 : b0;
 }
 
 // ------------------------------------------------------------------ kernel
@@ -380,7 +339,7 @@ __device__ __forceinline__ float select32(const float (&v)[32], int j) {
 // 128 x 128 MMAs (one per block), so a tile crosses L2 -> SM once per 256
 // queries without coupling CTAs; warp g of a lane group filters block g.
 template <int FORM, int MAXI, bool MINIMA = false, bool PAIR = false, bool DUAL = false>
-__global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const __grid_constant__ FusedArgs<MAXI> A) {
+__global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_constant__ FusedArgs<MAXI> A) {
   static_assert(!(PAIR && DUAL) && !(DUAL && MINIMA), "dual blocks: single CTAs, candidate pools");
   using Tr = FormTraits<FORM>;
   const FusedBatch& B = A.B;
@@ -390,8 +349,7 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
   if (B.run_if && *B.run_if == 0) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int EW = epi_warps_for(MINIMA);  // epilogue warps
-  constexpr int WG = EW / 4;                  // epilogue warps per TMEM lane group
+  constexpr int EW = kEpiWarps;
   const SmemLayout L = make_layout(FORM, B.d, PAIR ? 1 : 0, EW, DUAL ? 1 : 0);
   constexpr int kTileRows = DUAL ? kBN / 2 : kBN;  // database rows per tile
   constexpr int kQB = DUAL ? 2 : 1;                // resident query blocks
@@ -455,7 +413,7 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
   const uint32_t tmem_base = *tmem_slot;
 
   const int KC = Tr::kChunkElems;
-  auto maps_of = [&](int ii) { return &A.maps[ii * kMapsPerItem]; };
+  auto maps_of = [&](int ii) { return &A.maps[(MAXI == 1 ? 0 : ii) * kMapsPerItem]; };
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -509,7 +467,7 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
         }
         const int nreg = L.nkc - (L.tail_narrow ? 1 : 0);
         for (int t = t0; t < t1 && ok; ++t) {
-          const int T_i = A.items[ii].num_tiles;
+          const int T_i = A.items[MAXI == 1 ? 0 : ii].num_tiles;
           const int tx_row = ((t - rot + T_i) % T_i) * kTileRows + half_row;  // database tile of position t
           for (int kc = 0; kc < nreg; ++kc, ++it) {
             const int s = (int)(it % (uint32_t)S);
@@ -603,7 +561,7 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
           }
           tc_fence_after();
         }
-        const int fp8_tail = Tr::kFP8 ? A.items[ii].fp8_tail : 0;
+        const int fp8_tail = Tr::kFP8 ? A.items[MAXI == 1 ? 0 : ii].fp8_tail : 0;
         for (int t = t0; t < t1 && ok; ++t, ++tc) {
           const uint32_t slot = tc & 1u, use = tc >> 1;
           STAT_BEGIN(ta);
@@ -688,24 +646,28 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
     }
   } else {
     // ------------------------------------------------------------ epilogue
-    // The WG warps ew, ew + 4, ... read the same TMEM lanes (queries) and split
-    // each tile's four 64-column chunks between them: with two warps, warp g
-    // takes the 128-column half g; with three, chunk c of the tile counted tc
-    // goes to warp (4 tc + c) mod 3.  They share ONE candidate pool per
-    // (query, unit): appends reserve slots with a shared-memory counter, and at
-    // every S-th tile end the group meets at a named barrier, splits the pools
-    // that need a selection between them, and meets again.  A shared pool sees
-    // all of a tile's rows, so its bound tightens as one pool over the whole
-    // tile would -- about half the survivors and selections of a pool per half.
+    // Warps ew and ew + 4 read the same TMEM lanes (queries); warp g takes the
+    // 64-column chunks 2g and 2g + 1 of an accumulator slot.
+    //   Single blocks: the two warps split each tile's columns and share ONE
+    // candidate pool per (query, unit): appends reserve slots with a
+    // shared-memory counter, and at every S-th tile end the pair meets at a
+    // named barrier, splits the pools that need a selection between them, and
+    // meets again.  A shared pool sees all of a tile's rows, so its bound
+    // tightens as one pool over the whole tile would -- about half the survivors
+    // and selections of a pool per half.
+    //   Dual blocks (OWN): warp g filters query block qb + g alone, so a lane
+    // owns its query's pool: its count and bound live in registers and the
+    // warps meet nowhere.
+    constexpr bool OWN = DUAL;
     const int ew = warp - 2;       // 0..EW-1
     const int g = ew >> 2;         // this warp's index within its lane group
     const int lg = warp & 3;       // TMEM lane group this warp may access
     const int row = lg * 32 + lane;
-    const int pair_bar = 1 + lg;   // named barrier of the WG warps of lane group lg
-    constexpr int kGroupThreads = 32 * WG;
+    const int pair_bar = 1 + lg;   // named barrier of the two warps of lane group lg
+    constexpr int kGroupThreads = 64;
     uint32_t* hist = hist_all + ew * 256;
-    int* cnt_s = reinterpret_cast<int*>(smem + L.pool_off);                   // [128 kQB] pool counts
-    float* thr_s = reinterpret_cast<float*>(smem + L.pool_off) + kQB * kBM;   // [128 kQB] pool bounds
+    int* cnt_s = reinterpret_cast<int*>(smem + L.pool_off);             // [128] pool counts (single blocks)
+    float* thr_s = reinterpret_cast<float*>(smem + L.pool_off) + kBM;   // [128] pool bounds
     const uint32_t lane_base = (uint32_t)(lg * 32) << 16;
     UnitWalk walk(blockIdx.x, B, rank);
     int ii, qb, t0, t1, u_ord, rot;
@@ -725,25 +687,24 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
     if (threadIdx.x == 64 && B.stats) g_radix_pass_counter = &B.stats[kStatRadixPasses];
 #endif
     while (ok && walk.next(A, ii, qb, t0, t1, u_ord, gap, rot)) {
-      const FusedItem& p = A.items[ii];
+      const FusedItem& p = A.items[MAXI == 1 ? 0 : ii];  // one item: constants at fixed addresses
       const int P = p.pool_cap;
       const int U = p.units_per_block;
-      const int S = pool_sync_tiles(P, p.kprime);
+      const int S = OWN ? 1 : MINIMA ? 1024 : pool_sync_tiles(P, p.kprime);
       if (u_ord < 0 || u_ord >= U) {  // identical in every epilogue warp: both of a pair leave here
         raise_abort(abort_flag, B.status, kErrBadSchedule);
         break;
       }
-      // dual: warp g filters query block qb + g and owns its pools alone
-      const int qbw = DUAL ? qb + g : qb;
-      const int crow = DUAL ? g * kBM + row : row;  // this lane's pool count / bound slot
+      const int qbw = OWN ? qb + g : qb;  // this warp's query block
       const int q = qbw * kBM + row;
       const bool valid = q < p.nq;
       const float qn = valid ? p.q_norms[q] : 0.f;
-      float m2s = -2.f;
-      if (Tr::kFP8) m2s = valid ? -2.f * p.q_scale[q] : 0.f;
-      // FP8 with one scale s for every database row: d = ||x||^2 + (-2 s_q s) acc
+      // FP8: d = ||x||^2 + 2 s_q s_x acc (the query codes are stored negated)
+      float s2 = 2.f;
+      if (Tr::kFP8) s2 = valid ? 2.f * p.q_scale[q] : 0.f;
+      // FP8 with one scale s for every database row: d = ||x||^2 + 2 s_q s acc
       const bool uniform = Tr::kFP8 && p.db_scale_uniform > 0.f;
-      const float ku = m2s * p.db_scale_uniform;
+      const float ku = s2 * p.db_scale_uniform;
       // with the norm tails the accumulator is d / ku: the filter compares
       // ku acc with the bound and scales only the survivors (km = 1: the
       // accumulator is d itself or is made d below)
@@ -757,21 +718,23 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
       uint64_t* pool = pool_of(row);
       // a new unit starts with an empty pool (the previous unit's last barrier
       // ordered every use of the old state before this)
-      if (DUAL || g == 0) {
-        cnt_s[crow] = 0;
-        thr_s[crow] = 3.402823466e38f;
-      }
-      if constexpr (DUAL)
-        __syncwarp();
-      else
+      int own_cnt = 0;
+      if constexpr (!OWN) {
+        if (g == 0) {
+          cnt_s[row] = 0;
+          thr_s[row] = 3.402823466e38f;
+        }
         bar_sync_named(pair_bar, kGroupThreads);
-      float thr = 3.402823466e38f;  // FLT_MAX: admits every finite distance until a pool fills
+      }
+      // FLT_MAX admits every finite distance until a pool fills; a padding row
+      // of the last query block admits none
+      float thr = valid ? 3.402823466e38f : -__builtin_huge_valf();
 
-      // Selections of the pools in `need` (lane bits of this lane group; warp g
-      // owns the pools of lanes l with l mod WG = g, so two warps never touch
-      // the same pool's state).  Each keeps `keep` keys, records the pool's new
-      // count and bound in shared memory and publishes a full set's k'-th
-      // distance to q_bound.
+      // Selections of the pools in `need` (lane bits of this lane group; of a
+      // shared pool's two warps, warp g owns those of lanes l with l mod 2 = g,
+      // so two warps never touch the same pool's state).  Each keeps `keep`
+      // keys, records the pool's new count and bound and publishes a full
+      // set's k'-th distance to q_bound.
       auto refresh = [&](uint32_t need, int keep) {
         STAT_BEGIN(tr);
         while (need) {
@@ -779,14 +742,19 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
           need &= need - 1;
           STAT_INC(st_nref, 1);
           const int r = lg * 32 + src;
-          const int cr = (DUAL ? g * kBM : 0) + r;
-          const int n_src = cnt_s[cr];
+          const int n_src = OWN ? __shfl_sync(0xffffffffu, own_cnt, src) : cnt_s[r];
           int kept = 0;
           const uint64_t kmax = warp_select_keep_any(pool_of(r), n_src < P ? n_src : P, keep, P, hist, kept);
           if (lane == src) {
             const uint32_t ord = (uint32_t)(kmax >> 32);
-            cnt_s[cr] = kept;
-            thr_s[cr] = fminf(thr_s[cr], thr_from<Tr::kFolded>(ord2f(ord), qn));
+            const float nt = thr_from<Tr::kFolded>(ord2f(ord), qn);
+            if constexpr (OWN) {
+              own_cnt = kept;
+              thr = fminf(thr, nt);
+            } else {
+              cnt_s[r] = kept;
+              thr_s[r] = fminf(thr_s[r], nt);
+            }
             // only a full set of k' keys bounds the global k'-th distance
             if (kept >= p.kprime) atomicMin(&p.q_bound[q], ord);
           }
@@ -794,52 +762,70 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
         STAT_END(tr, st_refresh);
       };
 
-      // the shared bound is an L2 round trip: load it one tile ahead
+      // takes c slots of this lane's pool; returns the first
+      auto reserve = [&](int c) -> int {
+        if constexpr (OWN) {
+          own_cnt += c;
+          return own_cnt - c;
+        } else {
+          return c ? atomicAdd(&cnt_s[row], c) : 0;
+        }
+      };
+
+      float* colv = reinterpret_cast<float*>(hist);  // FP8 without tails: [128] norms, then [128] scales
+      // Coarse distances of accumulator columns c, c + 1, ... of this warp's 128:
+      // the accumulator itself (BF16 and exact forms), d / ku (FP8 with norm
+      // tails), else from the staged norms and scales.
+      auto dist_of = [&](const uint32_t* v, int c, float* x, int count) {
+#pragma unroll
+        for (int j = 0; j < count; ++j) {
+          x[j] = __uint_as_float(v[j]);
+          if (Tr::kFP8 && !fold)
+            x[j] = uniform ? fmaf(x[j], ku, colv[c + j]) : fmaf(x[j] * colv[kHalfN + c + j], s2, colv[c + j]);
+        }
+      };
+
+      const int T_i = p.num_tiles;
+      int tphys = t0 - rot;  // database tile of position t, kept in [0, T)
+      if (tphys < 0) tphys += T_i;
+      int until_sync = S;    // tiles until the pair meets
+      // The shared bound is an L2 round trip and moves rarely: it is asked for
+      // at one tile and used four tiles later
       uint32_t nb_ob = kOrdInf;
       if (valid) nb_ob = ld_relaxed_u32(&p.q_bound[q]);
       for (int t = t0; t < t1; ++t, ++tc) {
         const uint32_t slot = tc & 1u, use = tc >> 1;
-        const int tphys = (t - rot + p.num_tiles) % p.num_tiles;  // database tile of position t
-        thr = fminf(thr, thr_s[crow]);
-        if (nb_ob != kOrdInf) thr = fminf(thr, thr_from<Tr::kFolded>(ord2f(nb_ob), qn));
-        const float thr_up = next_above(thr);  // d <= thr  <=>  d < thr_up
-        if (valid) nb_ob = ld_relaxed_u32(&p.q_bound[q]);
-        // this warp's 64-column chunks of the tile (-1: none): 2g and 2g + 1
-        // with two warps per lane group; with three, the c with 4 tc + c = g
-        // (mod 3), i.e. c1 = (g - tc) mod 3 and, when c1 = 0, also 3
-        int my_c[2];
-        if constexpr (WG == 2) {
-          my_c[0] = 2 * g;
-          my_c[1] = 2 * g + 1;
-        } else {
-          my_c[0] = (int)(((uint32_t)g + 3u - tc % 3u) % 3u);
-          my_c[1] = my_c[0] == 0 ? 3 : -1;
+        if constexpr (!OWN) thr = fminf(thr, thr_s[row]);
+        if (((t - t0) & 3) == 0) {
+          if (nb_ob != kOrdInf) thr = fminf(thr, thr_from<Tr::kFolded>(ord2f(nb_ob), qn));
+          if (valid) nb_ob = ld_relaxed_u32(&p.q_bound[q]);
         }
-        // FP8: the database norms and scales of these columns, loaded before
-        // the accumulator wait (their latency overlaps it) and staged in the
-        // warp's histogram area, which is free outside a refresh
+        const float thr_up = next_above(thr);  // d <= thr  <=>  d < thr_up
+        const int tile0 = tphys * kTileRows;   // first database row of the tile
+        if (++tphys == T_i) tphys = 0;
+        // FP8 without norm tails: the database norms and scales of this warp's
+        // 128 columns, loaded before the accumulator wait (their latency
+        // overlaps it) and staged in the warp's histogram area, which is free
+        // outside a refresh
         float pxn[4], psx[4];
         if (Tr::kFP8 && !fold) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const int cc = my_c[i >> 1] < 0 ? my_c[0] : my_c[i >> 1];
             // < nb_pad: rows are padded to whole tiles (a strided sample has no padding)
-            const int c0 = tphys * kTileRows + (DUAL ? cc - 2 * g : cc) * 64 + lane + 32 * (i & 1);
+            const int c0 = tile0 + (OWN ? 0 : g * kHalfN) + 32 * i + lane;
             const size_t c = MINIMA ? (size_t)c0 * (size_t)p.db_step : (size_t)c0;
             pxn[i] = __ldg(p.db_norms + c);
             psx[i] = uniform ? 0.f : __ldg(p.db_scale + c);
           }
         }
         STAT_BEGIN(tw);
-        bool got = wait_or_abort(&acc_full[slot], use & 1u, abort_flag);
+        const bool got = wait_or_abort(&acc_full[slot], use & 1u, abort_flag);
         if (!got) raise_abort(abort_flag, B.status, kErrWaitTimeout);
         STAT_END(tw, st_wait);
         // an aborting warp skips the tile but still meets its partner below
         if (got) {
         STAT_BEGIN(tfl);
         tc_fence_after();
-        float bmin = 3.402823466e38f;  // block-minimum mode: smallest distance of this half tile
-        float* colv = reinterpret_cast<float*>(hist);  // [128] norms, then [128] scales
         if (Tr::kFP8 && !fold) {
           __syncwarp();
 #pragma unroll
@@ -849,174 +835,98 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
           }
           __syncwarp();
         }
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          const int ch = my_c[h];
-          if (ch < 0) break;
+        const uint32_t t_src = tmem_base + lane_base + slot * kBN + g * kHalfN;
+        const int tcol = tile0 + (OWN ? 0 : g * kHalfN);  // database row of the warp's first column
+        // Smallest distance of every 8 of the warp's 128 columns: half an
+        // instruction a column (the masks of every column took 1.5) decides
+        // whether anything of the tile survives, and which eights hold it.  The
+        // warp's cost is latency -- about six cycles an instruction at two
+        // warps per sub-partition -- so fewer instructions are the gain (full
+        // pass: FP8 sphere 26.8 -> 16.9 ms, BF16 integer mixture 3.22 -> 2.84
+        // and FP32-exact 5.58 -> 4.70 with dual blocks).
+        float gm[16];
+        {
           uint32_t v[64];
-          STAT_BEGIN(ttm);
-          tmem_ld_32x32b_x64(tmem_base + lane_base + slot * kBN + ch * 64, v);
+          float x[32];
+          auto mins = [&](const uint32_t* v, int i) {
+            dist_of(v, 32 * i, x, 32);
+            if (MINIMA && tcol + 32 * i + 32 > p.nb) {  // columns past nb do not count
+#pragma unroll
+              for (int j = 0; j < 32; ++j) x[j] = tcol + 32 * i + j < p.nb ? x[j] : __builtin_huge_valf();
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) gm[4 * i + e] = min8(x + 8 * e);
+          };
+          tmem_ld_32x32b_x64(t_src, v);
           tmem_ld_wait();
-          STAT_END(ttm, st_tmem);
-          const int col0 = tphys * kTileRows + (DUAL ? ch - 2 * g : ch) * 64;
-          // coarse distances of the 64 columns (two independent 32-column halves)
-          float da[32], db[32];
-          if (Tr::kFolded || fold) {
-            // the accumulator already is ||q||^2 + ||x||^2 - 2 q.x (BF16 and
-            // exact forms) or (||x||^2 - 2 q.x) / ku (FP8 with norm tails)
+          mins(v, 0);
+          mins(v + 32, 1);
+          tmem_ld_32x32b_x64(t_src + 64, v);
+          tmem_ld_wait();
+          mins(v, 2);
+          mins(v + 32, 3);
+        }
+        const float dmin = fminf(min8(gm), min8(gm + 8));
+        if (MINIMA) {
+          if (valid) {
+            const int br = p.minima_rows, per = kHalfN / br;  // 1 or 16 blocks of this warp's columns
+            float* o = p.minima + (size_t)q * (2 * (size_t)T_i * per) + (size_t)(2 * (tile0 / kTileRows) + g) * per;
+            auto key = [&](float x) { return Tr::kFolded ? x : (fold ? km * x : x) + qn; };
+            if (br == kHalfN) {
+              *o = key(dmin);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              da[j] = __uint_as_float(v[j]);
-              db[j] = __uint_as_float(v[32 + j]);
+              for (int e = 0; e < 16; e += 4)
+                *reinterpret_cast<float4*>(o + e) =
+                    make_float4(key(gm[e]), key(gm[e + 1]), key(gm[e + 2]), key(gm[e + 3]));
             }
-            if (MINIMA && fold) {
+          }
+        } else if (__any_sync(0xffffffffu, passes<Tr::kFP8>(dmin, km, thr_up))) {
+          STAT_INC(st_slow, 1);
+          // the eights in which some lane has a survivor (uniform), one at a
+          // time, fetched again from TMEM: one copy of the survivor code, which
+          // holds no tile registers (unrolled over register-held columns it
+          // missed the instruction caches)
+          uint32_t hit = __reduce_or_sync(
+              0xffffffffu, survive_mask<8>(gm, km, thr_up) | survive_mask<8>(gm + 8, km, thr_up) << 8);
+#pragma unroll 1
+          while (hit) {
+            const int e = __ffs(hit) - 1;
+            hit &= hit - 1u;
+            uint32_t w[8];
+            float x[8];
+            tmem_ld_32x32b_x8(t_src + 8 * e, w);
+            tmem_ld_wait();
+            dist_of(w, 8 * e, x, 8);
+            const int c8 = tcol + 8 * e;
+            uint32_t m = survive_mask<8>(x, km, thr_up);
+            // database rows beyond nb (padding of the last tile) never survive
+            if (c8 + 8 > p.nb) m &= c8 >= p.nb ? 0u : (1u << (p.nb - c8)) - 1u;
+            const int c = __popc(m);
+            int n = reserve(c);
+            STAT_INC(st_surv, c);
+            if (__any_sync(0xffffffffu, c > 2)) {
+              // dense (a pool without a tight bound yet): every column in order
 #pragma unroll
-              for (int j = 0; j < 32; j += 2) {
-                mul2_f32(da[j], da[j + 1], da[j], da[j + 1], ku, ku);
-                mul2_f32(db[j], db[j + 1], db[j], db[j + 1], ku, ku);
+              for (int j = 0; j < 8; ++j) {
+                const bool take = (m >> j) & 1u;
+                if (take && n < P) pool[n] = make_key(key_d(x[j]), (uint32_t)(c8 + j));
+                n += take ? 1 : 0;
               }
+              continue;
             }
-          } else {
-            const float4* xn4 = reinterpret_cast<const float4*>(colv + h * 64);
-            const float4* sx4 = reinterpret_cast<const float4*>(colv + kHalfN + h * 64);
-            if (uniform) {
-#pragma unroll
-              for (int j4 = 0; j4 < 16; ++j4) {
-                const float4 xn = xn4[j4];
-                float* dst = j4 < 8 ? da : db;
-                const int o = (j4 & 7) * 4;
-                fma2_f32(dst[o + 0], dst[o + 1], __uint_as_float(v[4 * j4 + 0]), __uint_as_float(v[4 * j4 + 1]), ku,
-                         ku, xn.x, xn.y);
-                fma2_f32(dst[o + 2], dst[o + 3], __uint_as_float(v[4 * j4 + 2]), __uint_as_float(v[4 * j4 + 3]), ku,
-                         ku, xn.z, xn.w);
-              }
-            } else
-#pragma unroll
-            for (int j4 = 0; j4 < 16; ++j4) {
-              const float4 xn = xn4[j4];
-              const float4 sx = sx4[j4];
-              float* dst = j4 < 8 ? da : db;
-              const int o = (j4 & 7) * 4;
-              // fmaf(acc * s_x, -2 s_q, ||x||^2) on column pairs
-              float p0, p1, p2, p3;
-              mul2_f32(p0, p1, __uint_as_float(v[4 * j4 + 0]), __uint_as_float(v[4 * j4 + 1]), sx.x, sx.y);
-              mul2_f32(p2, p3, __uint_as_float(v[4 * j4 + 2]), __uint_as_float(v[4 * j4 + 3]), sx.z, sx.w);
-              fma2_f32(dst[o + 0], dst[o + 1], p0, p1, m2s, m2s, xn.x, xn.y);
-              fma2_f32(dst[o + 2], dst[o + 3], p2, p3, m2s, m2s, xn.z, xn.w);
-            }
-          }
-          if (MINIMA) {
-            // block-minimum mode: no survivors, only the half tile's smallest
-            // distance (columns past nb excluded)
-            const int lim = p.nb - col0;
-            float mm[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {  // a tree, not one dependent chain
-              const float a0 = j < lim ? da[j] : 3.402823466e38f;
-              const float a1 = 16 + j < lim ? da[16 + j] : 3.402823466e38f;
-              const float b0 = 32 + j < lim ? db[j] : 3.402823466e38f;
-              const float b1 = 48 + j < lim ? db[16 + j] : 3.402823466e38f;
-              mm[j] = fminf(fminf(a0, a1), fminf(b0, b1));
-            }
-#pragma unroll
-            for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-              for (int j = 0; j < w; ++j) mm[j] = fminf(mm[j], mm[j + w]);
-            bmin = fminf(bmin, mm[0]);
-            continue;
-          }
-#if CURPLSH_MIN_FIRST
-          if (!__any_sync(0xffffffffu, valid && min64(da, db) < thr_up)) continue;
-#endif
-          // survivor masks: bit j of ma / mb for column j of da / db
-          uint32_t ma, mb;
-          // the FP32-exact form keeps compare masks: with three products per
-          // tile it is bound by the tensor pipe, and the packed-FMA masks
-          // measured slower there (10M-row sphere: 70.9 vs 77.0 ms)
-          if (Tr::kProducts == 3) {
-            ma = survive_mask32_cmp(da, thr);
-            mb = survive_mask32_cmp(db, thr);
-          } else {
-            constexpr int kChain = Tr::kFP8 ? 32 : 16;
-            ma = survive_mask32<kChain>(da, km, thr_up);
-            mb = survive_mask32<kChain>(db, km, thr_up);
-          }
-          if (!valid) ma = mb = 0u;
-          // database rows beyond nb (padding of the last tile) never survive
-          if (col0 + 64 > p.nb) {
-            const int lim = p.nb - col0;
-            ma &= lim <= 0 ? 0u : (lim >= 32 ? ~0u : ((1u << lim) - 1u));
-            mb &= lim <= 32 ? 0u : (lim >= 64 ? ~0u : ((1u << (lim - 32)) - 1u));
-          }
-          if (__any_sync(0xffffffffu, (ma | mb) != 0u)) {
-            STAT_INC(st_slow, 1);
-#ifdef CURPLSH_FUSED_STATS
-            {
-              int mx = __popc(ma) + __popc(mb);
-#pragma unroll
-              for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-              STAT_INC(st_iters, mx);
-            }
-#endif
-            // A lane rarely has more than one survivor per 32 columns: take the
-            // first of each half with a register select tree (no local memory),
-            // a second one the same way, and stash only for the rare rest.
-            // slots for this lane's survivors of the 64 columns, reserved at
-            // once by every lane (most add 0): no branch, so the select trees
-            // below run while the shared atomic is in flight
-            int n = atomicAdd(&cnt_s[crow], __popc(ma) + __popc(mb));
-            if ((ma & mb) == ~0u) {
-              // every column survives (a pool with no bound yet): append all
-              // 64 keys in column order, no extraction
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (n + j < P) pool[n + j] = make_key(key_d(da[j]), (uint32_t)(col0 + j));
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (n + 32 + j < P)
-                  pool[n + 32 + j] = make_key(key_d(db[j]), (uint32_t)(col0 + 32 + j));
-              n += 64;
-              ma = mb = 0u;
-              STAT_INC(st_surv, 64);
-            }
-            // the first survivor of each half, straight-line (j = -1: none)
-            auto take2 = [&]() {
-              const int ja = __ffs(ma) - 1, jb = __ffs(mb) - 1;
-              const float xa = select32(da, ja & 31), xb = select32(db, jb & 31);
-              ma &= ma - 1u;
-              mb &= mb - 1u;
-              const bool ha = ja >= 0, hb = jb >= 0;
-              if (ha && n < P) pool[n] = make_key(key_d(xa), (uint32_t)(col0 + ja));
-              n += ha ? 1 : 0;
-              if (hb && n < P) pool[n] = make_key(key_d(xb), (uint32_t)(col0 + 32 + jb));
-              n += hb ? 1 : 0;
-              STAT_INC(st_surv, (ha ? 1 : 0) + (hb ? 1 : 0));
-            };
-            take2();
-            if (__any_sync(0xffffffffu, (ma | mb) != 0u)) {
-              take2();
-              if (__any_sync(0xffffffffu, (ma | mb) != 0u)) {
-                float stash[64];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                  stash[j] = da[j];
-                  stash[32 + j] = db[j];
-                }
-                uint64_t mm = ((uint64_t)mb << 32) | ma;
-                while (mm) {
-                  const int j = __ffsll((long long)mm) - 1;
-                  mm &= mm - 1;
-                  if (n < P) pool[n] = make_key(key_d(stash[j]), (uint32_t)(col0 + j));
-                  ++n;
-                  STAT_INC(st_surv, 1);
-                }
-              }
-            }
+            // mostly one survivor, in one lane
+#pragma unroll 1
+            do {
+              STAT_INC(st_iters, 1);
+              const int j = __ffs(m) - 1;  // -1: none left
+              const float xs = select8(x, j);
+              m &= m - 1u;
+              if (j >= 0 && n < P) pool[n] = make_key(key_d(xs), (uint32_t)(c8 + j));
+              ++n;
+            } while (__any_sync(0xffffffffu, m != 0u));
           }
         }
-        if (MINIMA && valid)
-          p.minima[(size_t)q * (2 * (size_t)p.num_tiles) + 2 * (size_t)tphys + g] =
-              Tr::kFolded ? bmin : bmin + qn;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
@@ -1027,47 +937,53 @@ __global__ void __launch_bounds__(threads_for(MINIMA), 1) fused_knn_kernel(const
         }
         STAT_END(tfl, st_filter);
         }  // got
+        if constexpr (OWN) {
+          if (!got) {
+            ok = false;
+            break;
+          }
+          // pools that may not have room for the next tile, or, at the unit's
+          // end, every pool above k' (the merge pass reads at most k' keys'
+          // worth beyond what it needs)
+          const int lim = t + 1 < t1 ? P - kTileRows : p.kprime;
+          const uint32_t need = __ballot_sync(0xffffffffu, valid && own_cnt > lim);
+          if (need) {
+            if (own_cnt > P) atomicOr(B.status, kErrPoolOverflow);
+            __syncwarp();  // the other lanes read this lane's keys
+            refresh(need, p.kprime);
+          }
+          continue;
+        }
         // every S tiles (and at the unit's end) meet the partner warp; leave
         // together if either aborted
-        if ((t - t0 + 1) % S != 0 && t + 1 < t1) continue;
+        if (--until_sync != 0 && t + 1 < t1) continue;
+        until_sync = S;
         STAT_BEGIN(tb1);
-        bool leave;
-        if constexpr (DUAL)
-          leave = __any_sync(0xffffffffu, !got || *abort_flag != 0);
-        else
-          leave = bar_red_or(pair_bar, kGroupThreads, !got || *abort_flag != 0);
+        const bool leave = bar_red_or(pair_bar, kGroupThreads, !got || *abort_flag != 0);
         STAT_END(tb1, st_bar);
         if (leave) {
           ok = false;
           break;
         }
-        // pools that may not have room for the next S tiles (both halves),
-        // or, at the unit's end, every pool above k' (the merge pass reads at
-        // most k' keys' worth beyond what it needs)
+        // as above, for the next S tiles (both halves)
         const int lim = t + 1 < t1 ? P - S * kTileRows : p.kprime;
-        const bool mine = DUAL || (lane % WG) == g;
-        const int cn = mine ? cnt_s[crow] : 0;
+        const bool mine = (lane & 1) == g;
+        const int cn = mine ? cnt_s[row] : 0;
         if (cn > P) atomicOr(B.status, kErrPoolOverflow);
         refresh(__ballot_sync(0xffffffffu, mine && valid && cn > lim), p.kprime);
         STAT_BEGIN(tb2);
-        if constexpr (DUAL)
-          __syncwarp();
-        else
-          bar_sync_named(pair_bar, kGroupThreads);
+        bar_sync_named(pair_bar, kGroupThreads);
         STAT_END(tb2, st_bar);
       }
       if (!ok) break;
       // a refresh may keep a few more than k' keys (unsorted): record them all;
       // the merge pass selects exactly
-      if (!MINIMA && valid && (DUAL || g == 0)) {
-        const int cn = cnt_s[crow];
+      if (!MINIMA && valid && (OWN || g == 0)) {
+        const int cn = OWN ? own_cnt : cnt_s[row];
         p.pool_counts[(pool_row0 + row) * U + u_ord] = cn < P ? cn : P;
         if (gap) p.pool_counts[(pool_row0 + row) * U + u_ord - 1] = 0;
       }
-      if constexpr (DUAL)
-        __syncwarp();
-      else
-        bar_sync_named(pair_bar, kGroupThreads);  // the counts are read before the next unit resets them
+      if constexpr (!OWN) bar_sync_named(pair_bar, kGroupThreads);  // the counts are read before the next unit resets them
     }
     if (lane == 0) {
       STAT_FLUSH(kStatEpiWaitAccFull, st_wait);
@@ -1161,7 +1077,7 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
                         const int* run_if) {
   cudaError_t e = ensure_attributes<FORM, MAXI, MINIMA, PAIR, DUAL>();
   if (e != cudaSuccess) return e;
-  smem = make_layout(FORM, specs[0].d, PAIR ? 1 : 0, epi_warps_for(MINIMA), DUAL ? 1 : 0).total;  // this instance's
+  smem = make_layout(FORM, specs[0].d, PAIR ? 1 : 0, kEpiWarps, DUAL ? 1 : 0).total;  // this instance's
   FusedArgs<MAXI> a;
   memset(&a, 0, sizeof(a));
   a.B.num_items = n;
@@ -1201,6 +1117,7 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
     it.db_scale_uniform = f.xs_uniform;
     it.fp8_tail = (fp8 && f.xs_uniform > 0.f) ? (int)fp8_tail_offset(f.d, f.ld8) : 0;
     it.minima = f.minima;
+    it.minima_rows = f.minima_rows;
     CUtensorMap* m = &a.maps[i * kMapsPerItem];
     const void* qh = fp8 ? (const void*)f.q8 : (const void*)f.qh;
     const void* xh = fp8 ? (const void*)f.x8 : (const void*)f.xh;
@@ -1227,13 +1144,13 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
     }
   }
   if (!PAIR) {
-    fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL><<<bp.grid, threads_for(MINIMA), smem, st>>>(a);
+    fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL><<<bp.grid, kNumThreads, smem, st>>>(a);
     return cudaGetLastError();
   }
   if (bp.grid % 2) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)bp.grid, 1, 1);
-  cfg.blockDim = dim3(threads_for(MINIMA), 1, 1);
+  cfg.blockDim = dim3(kNumThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -1255,14 +1172,10 @@ cudaError_t launch_form_any(const FusedItemSpec* specs, const FusedItemPlan* pla
                    : launch_form<FORM, 1, true>(specs, plans, n, bp, status, stats, smem, st, run_if);
   for (int i = 0; i < n; ++i)
     if (specs[i].minima) return cudaErrorInvalidValue;  // block-minimum mode is single-item
-  if constexpr (FORM != kFormExact) {
-    if (bp.dual)
-      return n == 1 ? launch_form<FORM, 1, false, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
+  if (bp.dual)
+    return n == 1 ? launch_form<FORM, 1, false, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
                     : launch_form<FORM, kFusedMaxItems, false, false, true>(specs, plans, n, bp, status, stats, smem,
                                                                           st, run_if);
-  } else {
-    if (bp.dual) return cudaErrorInvalidValue;  // dual blocks are planned for BF16 / FP8 only
-  }
   if (n == 1)
     return bp.pair ? launch_form<FORM, 1, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
                    : launch_form<FORM, 1>(specs, plans, n, bp, status, stats, smem, st, run_if);
@@ -1286,6 +1199,8 @@ std::atomic<int> g_dual{CURPLSH_DUAL_DEFAULT};
 // 3.43, 192 4.75 -> 4.36, 256 6.10 -> 5.55, 512 11.5 -> 9.9 (identical results).
 constexpr int kPairMinDimBF16 = 320;
 constexpr int kPairMinDimExact = 192;
+// Dual blocks need units of this many times k' rows when pools start unbounded.
+constexpr int kDualFillRows = 64;
 }  // namespace
 
 void set_cta_pairs(int mode) {
@@ -1308,12 +1223,34 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
     odd += g & 1;
   }
   const bool grouped = blocks >= 4 && odd * 8 <= blocks;
-  // dual blocks need both query blocks resident in shared memory
-  const bool dual_fits = n > 0 && specs[0].d > 0 && !make_layout(form, specs[0].d, 0, kPoolEpiWarps, 1).a_stream;
-  // FP8 only: its MMAs are light, so halving the tile bytes per query pays
-  // (sphere 39.6 -> 37.7 ms); the BF16 pass got slower (3.50 -> 4.52 ms on the
-  // integer mixture: twice the MMA instructions and shared-memory A reads)
-  const int dual = (grouped && dual_fits && get_dual_blocks() && form == kFormFP8) ? 1 : 0;
+  // dual blocks need both query blocks resident in shared memory, and a ring
+  // whose stages cover the load latency: three, or two of the FP32-exact form's,
+  // each of which feeds three products (BF16 with two stages, d = 320: 4.26 ms
+  // against 3.53 as CTA pairs)
+  bool dual_fits = false;
+  if (n > 0 && specs[0].d > 0 && form >= 0) {
+    const SmemLayout DL = make_layout(form, specs[0].d, 0, kEpiWarps, 1);
+    dual_fits = !DL.a_stream && DL.stages >= (form == kFormExact ? 2 : 3);
+  }
+  // Pools that start without a bound fill to k' keys in every unit; a dual
+  // unit has half the rows at the same CTA range, so there are twice as many.
+  // With an estimate (fill_kprime = 0), or with units of many times k' rows,
+  // that is nothing; where it is not, single blocks stay (1,000 queries,
+  // k = 1,024, 300,000 rows without an estimate: 5.7 against 8.4 ms).
+  bool short_units = false;
+  {
+    long long work = 0;
+    for (int i = 0; i < n; ++i)
+      if (specs[i].nb > 0)
+        work += (long long)((specs[i].nq + 2 * kBM - 1) / (2 * kBM)) * ((specs[i].nb + kBN / 2 - 1) / (kBN / 2));
+    const long long w = std::max<long long>(1, work / std::max(1, max_ctas));
+    for (int i = 0; i < n; ++i)
+      short_units = short_units || w * (kBN / 2) < (long long)kDualFillRows * specs[i].fill_kprime;
+  }
+  // Two query blocks per CTA: a database tile crosses L2 -> SM once per 256
+  // queries, and every query's pool belongs to one lane (full pass, single ->
+  // dual blocks: BF16 integer mixture 3.50 -> 2.84 ms, FP32-exact 5.64 -> 4.70)
+  const int dual = (grouped && dual_fits && !short_units && get_dual_blocks()) ? 1 : 0;
   const int pm = get_cta_pairs();
   const int d0 = n > 0 ? specs[0].d : 0;
   const bool want_pair = pm == 1 || (pm == kPairsAuto && ((form == kFormBF16 && d0 >= kPairMinDimBF16) ||
@@ -1355,11 +1292,12 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
   }
 }
 
-void plan_fused(int nq, int nb, int num_sms, FusedPlan* out, int split_q4, int form, int d) {
+void plan_fused(int nq, int nb, int num_sms, FusedPlan* out, int split_q4, int form, int d, int fill_kprime) {
   FusedItemSpec s{};
   s.nq = nq;
   s.nb = nb;
   s.d = d;
+  s.fill_kprime = fill_kprime;
   FusedItemPlan ip;
   FusedBatchPlan bp;
   plan_fused_batch(&s, 1, num_sms, &ip, &bp, form);
@@ -1388,6 +1326,8 @@ cudaError_t prepare_fused_kernels(int form) {
       if (e == cudaSuccess) e = ensure_attributes<kFormExact, 1, false, true>();
       if (e == cudaSuccess) e = ensure_attributes<kFormExact, 1, true, true>();
       if (e == cudaSuccess) e = ensure_attributes<kFormExact, kFusedMaxItems, false, true>();
+      if (e == cudaSuccess) e = ensure_attributes<kFormExact, 1, false, false, true>();
+      if (e == cudaSuccess) e = ensure_attributes<kFormExact, kFusedMaxItems, false, false, true>();
       return e != cudaSuccess ? e : ensure_attributes<kFormExact, kFusedMaxItems>();
     case kFormBF16:
       e = ensure_attributes<kFormBF16, 1>();
@@ -1460,6 +1400,7 @@ cudaError_t launch_fused(const FusedLaunch& f, cudaStream_t st) {
   s.q_bound = f.q_bound;
   s.db_step = f.db_step;
   s.minima = f.minima;
+  s.minima_rows = f.minima_rows;
   FusedItemPlan ip;
   ip.num_qblocks = f.plan.num_qblocks;
   ip.num_tiles = f.plan.num_tiles;

@@ -62,6 +62,7 @@ struct FusedLaunch {
   int db_step = 1;
   // non-null: block-minimum mode, see FusedItem::minima (pools are not used)
   float* minima = nullptr;
+  int minima_rows = 128;
   // outputs / scratch
   uint64_t* pools;
   int* pool_counts;
@@ -74,8 +75,11 @@ struct FusedLaunch {
 
 // One search over at most num_sms CTAs.  split_q4 < 4 cuts units shorter than
 // the CTA ranges (split_tiles_for(W, split_q4)); >= 4 leaves the ranges whole.
-// `form` (-1: unknown) decides whether dual blocks may be used (BF16 and FP8).
-void plan_fused(int nq, int nb, int num_sms, FusedPlan* out, int split_q4 = 4, int form = -1, int d = 0);
+// `form` (-1: unknown) decides whether dual blocks may be used, and
+// `fill_kprime` > 0 says that pools start without a bound and fill to that many
+// keys first (FusedItemSpec::fill_kprime).
+void plan_fused(int nq, int nb, int num_sms, FusedPlan* out, int split_q4 = 4, int form = -1, int d = 0,
+                int fill_kprime = 0);
 uint32_t fused_smem_bytes(int form, int d);
 cudaError_t launch_fused(const FusedLaunch& f, cudaStream_t st);
 
@@ -88,6 +92,7 @@ constexpr int kFusedMaxItems = 16;
 
 struct FusedItemSpec {
   int nq, nb, d, kprime, pool_cap;
+  int fill_kprime;  // planning: k' when the pools start without a bound, 0 when an estimate bounds them
   int split_tiles;  // max tiles per unit (<= 0: no limit beyond the CTA ranges)
   long long nq_pad, nb_pad, ld16, ld8;
   const __nv_bfloat16* qh;
@@ -106,6 +111,7 @@ struct FusedItemSpec {
   uint32_t* q_bound;        // [nq_pad], initialised to all ones (or to estimated bounds)
   int db_step;              // database row j is stored row j * db_step (0 or 1: contiguous)
   float* minima;            // non-null: block-minimum mode (FusedItem::minima)
+  int minima_rows;          // its block rows: 128 or 8
 };
 struct FusedItemPlan {
   int num_qblocks, num_tiles, units_per_block;  // num_qblocks: groups of 128 << pair query rows
@@ -126,11 +132,11 @@ struct FusedBatchPlan {
 constexpr int kPairsAuto = 2;
 void set_cta_pairs(int mode);
 int get_cta_pairs();
-// Dual query blocks (BF16 / FP8) on or off for the plans made after the call.
+// Dual query blocks on or off for the plans made after the call.
 void set_dual_blocks(int on);
 int get_dual_blocks();
-// Plans `n` items over at most `max_ctas` CTAs.  Only nq, nb and split_tiles
-// of the specs are read, so pool sizes (which depend on units_per_block) can be computed
+// Plans `n` items over at most `max_ctas` CTAs.  Only nq, nb, d, fill_kprime and
+// split_tiles of the specs are read, so pool sizes (which depend on units_per_block) can be computed
 // from the plan before the pools are carved.
 void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItemPlan* plans, FusedBatchPlan* out,
                       int form = -1);
@@ -145,14 +151,15 @@ cudaError_t launch_fused_batch(int form, const FusedItemSpec* specs, const Fused
 
 // ---- sampled bound estimate (capi.cpp): a short fused pass over a strided
 // sample of the database records per query the smallest distance of every
-// 128-row block of the sample; the j-th smallest of those B block minima is
+// block of the sample's rows; the j-th smallest of those B block minima is
 // the starting bound of every candidate pool of the full pass.
 struct EstimatePlan {
   bool on = false;
-  bool light = false;  // few expected sample rows: a looser rank from a smaller sample
+  bool light = false;  // sized by cost, not by expected rows (see capi.cpp)
   int rows = 0;    // sample rows (a multiple of 256)
   int step = 1;    // sample row j is database row j * step
-  int blocks = 0;  // B = rows / 128 block minima per query
+  int block_rows = 128;  // or 8
+  int blocks = 0;  // B = rows / block_rows block minima per query
   int j = 0;       // rank of the estimate among the block minima
   FusedPlan plan;
 };
@@ -169,7 +176,7 @@ bool bound_estimate_enabled();
 // database rows get [n1 n2 n3 1 1 1] after column d, query rows are stored as -2q
 // followed by [1 1 1 m1 m2 m3]; lo rows get zeros there.  kAugF8Query /
 // kAugF8Database write the FP8 rows' BF16 norm tail (see fp8_tail_offset):
-// query rows [a_h a_h a_l] with a = 1/s_q (a zero row takes scale 1), database
+// query rows (codes stored negated) [a_h a_h a_l] with a = -1/s_q (a zero row takes scale 1), database
 // rows [b_h b_l b_h] with b = -||x||^2 / (2 fixed_scale) (zeros without a
 // fixed scale).
 enum AugMode : int { kAugNone = 0, kAugDatabase = 1, kAugQuery = 2, kAugF8Query = 3, kAugF8Database = 4 };

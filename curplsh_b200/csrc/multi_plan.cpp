@@ -155,10 +155,13 @@ int MultiPlan::build(const curplsh_batch_item* items, int n, const std::vector<c
       std::vector<FusedItemSpec> specs(FL.fitems.size());
       std::vector<FusedItemPlan> plans(FL.fitems.size());
       for (size_t j = 0; j < FL.fitems.size(); ++j) {
-        const FItem& x = fitems_[FL.fitems[j]];
+        FItem& x = fitems_[FL.fitems[j]];
         specs[j].nq = x.nq;
         specs[j].nb = (int)views[x.slot].n;
         specs[j].d = G.d;
+        if (use_est) x.est = plan_estimate(x.nq, views[x.slot].n, x.kp, num_sms);
+        FL.est_any = FL.est_any || x.est.on;
+        specs[j].fill_kprime = x.est.on ? 0 : x.kp;
         // units as long as the item's own CTA ranges would be if it were
         // searched alone (scaled by the tuned split, at most the whole range,
         // as alone), so its in-pool selection work stays what it is alone
@@ -172,8 +175,6 @@ int MultiPlan::build(const curplsh_batch_item* items, int n, const std::vector<c
         x.plan = plans[j];
         x.W = FL.bp.work_per_cta;
         x.launch = (int)(&FL - G.launches.data());
-        if (use_est) x.est = plan_estimate(x.nq, views[x.slot].n, x.kp, num_sms);
-        FL.est_any = FL.est_any || x.est.on;
       }
     }
   }
@@ -348,6 +349,7 @@ int MultiPlan::enqueue(cudaStream_t main, const std::vector<cudaStream_t>* branc
       e.xs_uniform = s.xs_uniform;
       e.db_step = x.est.step;
       e.minima = reinterpret_cast<float*>(base_ + x.o_minima);
+      e.minima_rows = x.est.block_rows;
       e.pools = s.pools;
       e.pool_counts = s.pool_counts;
       e.q_bound = s.q_bound;

@@ -98,11 +98,14 @@ __device__ __forceinline__ void prep_row(const float* __restrict__ x, long long 
   if (f8) {
     m = warp_max(m);
     // an all-zero row gets scale 0 (its codes are 0 whatever the scale); a
-    // zero query row with a norm tail gets 1, so its tail 1/s_q is finite
+    // zero query row with a norm tail gets 1, so its tail -1/s_q is finite
     float sc = fixed_scale > 0.f ? fixed_scale : m / kE4M3Max;
     const bool q_tail = aug == kAugF8Query;
     if (q_tail && !(sc > 0.f)) sc = 1.f;
     inv = sc > 0.f ? 1.f / sc : 0.f;
+    // query codes (and their norm tail) are stored negated, so that the FP8
+    // accumulator grows with the distance; every rounding is symmetric
+    if (q_tail) inv = -inv;
     if (scale && lane == 0) scale[r] = (m > 0.f || q_tail) ? sc : 0.f;
   }
   if (vec4) {
@@ -179,7 +182,7 @@ __device__ __forceinline__ void prep_row(const float* __restrict__ x, long long 
       __syncwarp();  // after the zero fill above, which covers these bytes
       float v = 0.f;
       if (aug == kAugF8Query)
-        v = inv;  // 1 / s_q
+        v = inv;  // -1 / s_q
       else if (fixed_scale > 0.f)
         v = -0.5f * s / fixed_scale;  // -||x||^2 / (2 s)
       const float vh = __bfloat162float(__float2bfloat16_rn(v));

@@ -119,16 +119,30 @@ struct DevRes {
 // the next index or workspace and goes back to the driver with the resources.
 // cudaMalloc, cudaFree and the pinned read-back took most of a one-shot search
 // (200,000 rows, 1,000 queries: 3.4 to 30 ms a call; 0.39 ms from the pool).
+// Larger buffers come from cudaMalloc: the pool maps and unmaps them at every
+// index (10 GB in 100 to 200 ms, against 25 to 100).
 constexpr uint64_t kPoolKeep = 512ull << 20;
+constexpr size_t kPoolMaxBytes = 256ull << 20;
 
 // `st` orders the allocation; only work after it on `st` (or synchronised with
 // it) may use the memory.
-static cudaError_t pool_alloc(DevRes* d, void** p, size_t bytes, cudaStream_t st) {
+static cudaError_t pool_alloc(DevRes* d, void** p, size_t bytes, cudaStream_t st, bool* pooled) {
+  *pooled = false;
+  if (bytes > kPoolMaxBytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {  // give back what the pool keeps, once
+      cudaGetLastError();
+      cudaMemPoolTrimTo(d->pool, 0);
+      e = cudaMalloc(p, bytes);
+    }
+    return e;
+  }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
     return cudaMalloc(p, bytes);  // an allocation recorded into a graph would belong to the graph
   }
+  *pooled = true;
   cudaError_t e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
   if (e == cudaErrorMemoryAllocation) {  // give back what the pool keeps, once
     cudaGetLastError();
@@ -142,12 +156,13 @@ static cudaError_t pool_alloc(DevRes* d, void** p, size_t bytes, cudaStream_t st
 struct DevBuf {
   void* ptr = nullptr;
   size_t cap = 0;
+  bool pooled = false;
   // all use of the buffer is on `st`, so the old memory is freed in its order
   cudaError_t ensure(size_t bytes, DevRes* d, cudaStream_t st) {
     if (bytes <= cap) return cudaSuccess;
     if (ptr) release(st);
     size_t want = std::max(bytes, (size_t)1 << 20);
-    cudaError_t e = pool_alloc(d, &ptr, want, st);
+    cudaError_t e = pool_alloc(d, &ptr, want, st, &pooled);
     if (e == cudaSuccess)
       cap = want;
     else
@@ -155,10 +170,7 @@ struct DevBuf {
     return e;
   }
   void release(cudaStream_t st) {
-    if (ptr && cudaFreeAsync(ptr, st) != cudaSuccess) {  // memory of a capturing call, or a capturing stream
-      cudaGetLastError();
-      cudaFree(ptr);
-    }
+    if (ptr && (!pooled || cudaFreeAsync(ptr, st) != cudaSuccess)) cudaFree(ptr);
     ptr = nullptr;
     cap = 0;
   }
@@ -296,6 +308,27 @@ struct curplsh_index {
   std::atomic<long long> coarse_queries{0};    // queries re-searched after their coarse margin failed
   std::map<cudaStream_t, std::unique_ptr<StreamWorkspace>> ws;
 
+  // Device arrays of the index; `direct` lists those that cudaMalloc gave.
+  std::vector<void*> direct;
+  template <class T>
+  cudaError_t alloc(T** p, size_t bytes, cudaStream_t st) {
+    bool pooled = false;
+    cudaError_t e = pool_alloc(dres, reinterpret_cast<void**>(p), bytes, st, &pooled);
+    if (e == cudaSuccess && !pooled) direct.push_back(*p);
+    return e;
+  }
+  void free_array(void* p) {
+    if (!p) return;
+    for (size_t i = 0; i < direct.size(); ++i)
+      if (direct[i] == p) {
+        direct[i] = direct.back();
+        direct.pop_back();
+        cudaFree(p);
+        return;
+      }
+    cudaFreeAsync(p, dres->def);
+  }
+
   // Searches, batch graphs and servers on any stream may still read the rows,
   // so freeing them waits for the device (once, where the arrays had a
   // synchronising cudaFree each).
@@ -304,12 +337,11 @@ struct curplsh_index {
     if (rows || xn || xh || xl || x8 || xs) cudaDeviceSynchronize();
     if (rows && x32_managed)
       cudaFree(rows);
-    else if (rows)
-      cudaFreeAsync(rows, dres->def);
+    else
+      free_array(rows);
     x32 = nullptr;
     x32_owned = false;
-    for (void* p : {(void*)xn, (void*)xh, (void*)xl, (void*)x8, (void*)xs})
-      if (p) cudaFreeAsync(p, dres->def);
+    for (void* p : {(void*)xn, (void*)xh, (void*)xl, (void*)x8, (void*)xs}) free_array(p);
     xn = nullptr;
     xh = xl = nullptr;
     x8 = nullptr;
@@ -340,8 +372,8 @@ int build_fp8(curplsh_index* ix, cudaStream_t st) {
   if (ix->n == 0) return CURPLSH_OK;
   std::lock_guard<std::mutex> lk(ix->fp8_mu);  // concurrent searches build it once
   if (!ix->x8) {
-    CUDA_TRY(pool_alloc(ix->dres, (void**)&ix->x8, (size_t)ix->n_pad * ix->ld8, st));
-    CUDA_TRY(pool_alloc(ix->dres, (void**)&ix->xs, (size_t)ix->n_pad * sizeof(float), st));
+    CUDA_TRY(ix->alloc(&ix->x8, (size_t)ix->n_pad * ix->ld8, st));
+    CUDA_TRY(ix->alloc(&ix->xs, (size_t)ix->n_pad * sizeof(float), st));
     CUDA_TRY(launch_prep_rows(ix->x32, ix->dim, (int)ix->n, ix->n_pad, ix->dim, nullptr, 0.f, nullptr, nullptr,
                               ix->ld16, ix->x8, ix->xs, ix->ld8, st));
     uint32_t range[2] = {0xFFFFFFFFu, 0u};
@@ -453,19 +485,42 @@ struct Timing {
 
 constexpr double kEstimateFailure = 1e-6;  // per-query failure probability for a uniform sample
 
-// P(X >= j) for X ~ Binomial(n, q).
+// P(X >= j) for X ~ Binomial(n, q), q in (0, 1): the first term from log gammas,
+// the others by their ratio.
 double binomial_tail(int n, double q, int j) {
   if (j <= 0) return 1.0;
   if (j > n) return 0.0;
-  const double lq = std::log(q), l1q = std::log1p(-q);
+  const double odds = q / (1.0 - q);
+  double term = std::exp(std::lgamma(n + 1.0) - std::lgamma(j + 1.0) - std::lgamma(n - j + 1.0) + j * std::log(q) +
+                         (n - j) * std::log1p(-q));
   double t = 0.0;
   for (int i = j; i <= n; ++i) {
-    const double term =
-        std::exp(std::lgamma(n + 1.0) - std::lgamma(i + 1.0) - std::lgamma(n - i + 1.0) + i * lq + (n - i) * l1q);
     t += term;
     if (term < t * 1e-12) break;
+    term *= (double)(n - i) / (i + 1) * odds;
   }
   return t;
+}
+
+// Smallest j with P(X >= j) <= kEstimateFailure, or n / 2 + 1.  The tail falls
+// with j and is above 0.4 up to the mean, so the search starts there.
+int binomial_rank(int n, double q) {
+  int lo = std::max(0, (int)(n * q) - 1), hi = n / 2 + 1;  // the answer is in (lo, hi]
+  for (int step = 8; lo + step < hi; step *= 2) {
+    if (binomial_tail(n, q, lo + step) <= kEstimateFailure) {
+      hi = lo + step;
+      break;
+    }
+    lo += step;
+  }
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (binomial_tail(n, q, mid) <= kEstimateFailure)
+      hi = mid;
+    else
+      lo = mid;
+  }
+  return hi;
 }
 
 // Smallest rank j <= most * n with exp(-n KL(j / n || q)) <= kEstimateFailure, a
@@ -520,7 +575,7 @@ constexpr long long kEstimateMinRows = 2048;
 namespace curplsh_b200 {
 // The plan a search of this shape uses when the estimate is enabled (the
 // caller reads the process-wide switch once per search).
-EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms) {
+EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms, bool lean) {
   EstimatePlan e;
   if (nq < 1 || kp < 1 || n < kEstimateMinRows || n < 4LL * kp) return e;
   const long long T = (n + kBN - 1) / kBN;
@@ -531,10 +586,10 @@ EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms) {
     // smallest rank whose failure probability is small enough, among at most half of the blocks
     const int blocks = (int)(tiles * kBN / block_rows);
     const double q0 = under(block_rows);
-    j = 1;
-    while (2 * j <= blocks && binomial_tail(blocks, q0, j) > kEstimateFailure) ++j;
+    j = q0 < 1.0 ? binomial_rank(blocks, q0) : 0;
     if (2 * j > blocks) j = 0;
   }
+  if (j == 0 && lean) return e;
   if (j == 0) {
     e.light = true;
     double best = 0.0;
@@ -590,16 +645,16 @@ bool coarse_check_applies(const curplsh_index* ix, int form, int kp, bool enable
 }
 
 SearchShape search_shape(const curplsh_index* ix, int nq, int k, int form, int rerank_factor, bool allow_est,
-                         bool coarse_on) {
+                         bool coarse_on, bool lean = false) {
   SearchShape sh;
   sh.kp = kprime_for(form, k, rerank_factor, ix->n, coarse_on);
   const TuneParams tp = tune_lookup(form, ix->dim, k, nq);
   sh.P = pool_capacity(sh.kp, tp.headroom);
-  if (allow_est) sh.est = plan_estimate(nq, ix->n, sh.kp, ix->dres->num_sms);
+  if (allow_est) sh.est = plan_estimate(nq, ix->n, sh.kp, ix->dres->num_sms, lean);
   plan_fused(nq, (int)ix->n, ix->dres->num_sms, &sh.plan, default_split_q4(tp, sh.P), form, ix->dim,
-             sh.est.on ? 0 : sh.kp);
+             lean ? kFillSingle : sh.est.on ? 0 : sh.kp);
   sh.nq_pad = round_up(nq, kBM);
-  sh.pool_lists = (size_t)sh.plan.pool_rows() * sh.plan.units_per_block;
+  sh.pool_lists = (size_t)sh.plan.pool_rows() * sh.plan.units_per_block * sh.plan.lists_per_unit();
   sh.coarse = coarse_check_applies(ix, form, sh.kp, coarse_on);
   return sh;
 }
@@ -878,14 +933,6 @@ int do_search(curplsh_index* ix, int64_t num, const float* queries, int k, int p
   // is always the host's: a query it lists is searched again in the exact form
   // before the call returns.
   const bool coarse_on = g_coarse_check.load(std::memory_order_relaxed) != 0;
-  SearchShape sh;
-  if (ix->n > 0)
-    sh = search_shape(ix, nq, k, form, rf, g_bound_estimate.load(std::memory_order_relaxed) != 0, coarse_on);
-  const bool est = sh.est.on, coarse = sh.coarse;
-  const bool all_dev = q_dev && i_dev && d_dev;
-  const bool dev_recheck = est && !coarse && all_dev && !force_sync;
-  const bool sync = force_sync || (est && !dev_recheck) || coarse || !all_dev;
-
   StreamWorkspace* wp;
   {
     std::lock_guard<std::mutex> wl(ix->ws_mu);
@@ -895,15 +942,25 @@ int do_search(curplsh_index* ix, int64_t num, const float* queries, int k, int p
   }
   StreamWorkspace& w = *wp;
   std::lock_guard<std::mutex> wlk(w.mu);
-  const size_t core = search_workspace_bytes(ix, sh, nq, form);
+  const bool est_on = g_bound_estimate.load(std::memory_order_relaxed) != 0;
   const size_t qbytes = q_dev ? 0 : (size_t)nq * ix->dim * sizeof(float);
   const size_t obytes = (i_dev && d_dev) ? 0 : (size_t)nq * k * (sizeof(int) + sizeof(float));
-  const size_t total = (size_t)round_up((long long)qbytes, 256) + (size_t)round_up((long long)obytes, 256) + core;
-  cudaError_t e = w.dev.ensure(total, ix->dres, st);
-  if (e != cudaSuccess) {
+  SearchShape sh;
+  for (int lean = 0;; ++lean) {  // short of memory, a plan with less working memory is tried
+    if (ix->n > 0) sh = search_shape(ix, nq, k, form, rf, est_on, coarse_on, lean != 0);
+    const size_t core = search_workspace_bytes(ix, sh, nq, form);
+    const size_t total = (size_t)round_up((long long)qbytes, 256) + (size_t)round_up((long long)obytes, 256) + core;
+    const cudaError_t e = w.dev.ensure(total, ix->dres, st);
+    if (e == cudaSuccess) break;
     cudaGetLastError();
-    return set_error(CURPLSH_ERR_OOM, "workspace of %zu bytes: %s", total, cudaGetErrorString(e));
+    if (lean || ix->n == 0)
+      return set_error(CURPLSH_ERR_OOM, "workspace of %zu bytes: %s", total, cudaGetErrorString(e));
   }
+  const bool est = sh.est.on, coarse = sh.coarse;
+  const bool all_dev = q_dev && i_dev && d_dev;
+  const bool dev_recheck = est && !coarse && all_dev && !force_sync;
+  const bool sync = force_sync || (est && !dev_recheck) || coarse || !all_dev;
+
   if (!w.host) w.host = ix->res->pinned.take();
   if (!w.host) return set_error(CURPLSH_ERR_OOM, "pinned host memory");
   char* base = static_cast<char*>(w.dev.ptr);
@@ -1171,7 +1228,7 @@ int curplsh_index_bf_create(curplsh_resources* r, int dim, const curplsh_bf_conf
   ix->ld8 = (round_up(dim, 32) % 128 != 0) ? round_up(dim, 32) + 32 : round_up(dim, 16);
   r->refs.fetch_add(1);
   DeviceScope scope(c.device);
-  cudaError_t e = pool_alloc(d, (void**)&ix->status, 6 * sizeof(uint32_t), d->def);
+  cudaError_t e = ix->alloc(&ix->status, 6 * sizeof(uint32_t), d->def);
   if (e == cudaSuccess) e = cudaMemsetAsync(ix->status, 0, 6 * sizeof(uint32_t), d->def);
   if (e == cudaSuccess) e = cudaStreamSynchronize(d->def);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ix->order_ev, cudaEventDisableTiming);
@@ -1198,7 +1255,7 @@ int curplsh_index_destroy(curplsh_index* ix) {
       ix->res->pinned.give(kv.second->host);
     }
     ix->free_db();
-    if (ix->status) cudaFreeAsync(ix->status, def);
+    ix->free_array(ix->status);
     if (ix->order_ev) cudaEventDestroy(ix->order_ev);
     if (ix->fp8_ev) cudaEventDestroy(ix->fp8_ev);
   }
@@ -1242,15 +1299,15 @@ int curplsh_index_add(curplsh_index* ix, int64_t num, const float* data) {
     if (ix->cfg.memory_space == CURPLSH_MEMORY_UNIFIED)
       CUDA_TRY(cudaMallocManaged(&x32, (size_t)n_new * d * sizeof(float)));
     else
-      CUDA_TRY(pool_alloc(ix->dres, (void**)&x32, (size_t)n_new * d * sizeof(float), st));
+      CUDA_TRY(ix->alloc(&x32, (size_t)n_new * d * sizeof(float), st));
     if (n_old) CUDA_TRY(cudaMemcpyAsync(x32, ix->x32, (size_t)n_old * d * sizeof(float), cudaMemcpyDeviceToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(x32 + (size_t)n_old * d, data, (size_t)num * d * sizeof(float), cudaMemcpyDefault, st));
   }
   float* xn = nullptr;
   __nv_bfloat16 *xh = nullptr, *xl = nullptr;
-  CUDA_TRY(pool_alloc(ix->dres, (void**)&xn, (size_t)pad_new * sizeof(float), st));
-  CUDA_TRY(pool_alloc(ix->dres, (void**)&xh, (size_t)pad_new * ix->ld16 * sizeof(__nv_bfloat16), st));
-  CUDA_TRY(pool_alloc(ix->dres, (void**)&xl, (size_t)pad_new * ix->ld16 * sizeof(__nv_bfloat16), st));
+  CUDA_TRY(ix->alloc(&xn, (size_t)pad_new * sizeof(float), st));
+  CUDA_TRY(ix->alloc(&xh, (size_t)pad_new * ix->ld16 * sizeof(__nv_bfloat16), st));
+  CUDA_TRY(ix->alloc(&xl, (size_t)pad_new * ix->ld16 * sizeof(__nv_bfloat16), st));
   // rows [0, n_old) keep their prepared copies; rows from n_old on (and padding) are prepared now
   if (n_old) {
     CUDA_TRY(cudaMemcpyAsync(xn, ix->xn, (size_t)n_old * sizeof(float), cudaMemcpyDeviceToDevice, st));

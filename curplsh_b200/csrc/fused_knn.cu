@@ -657,8 +657,10 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
     // and selections of a pool per half.
     //   Dual blocks (OWN): warp g filters query block qb + g alone, so a lane
     // owns its query's pool: its count and bound live in registers and the
-    // warps meet nowhere.
-    constexpr bool OWN = DUAL;
+    // warps meet nowhere.  CTA pairs do the same with two pools per query, one
+    // per warp (kLists); block minima need no pool at all.
+    constexpr bool OWN = DUAL || PAIR || MINIMA;
+    constexpr int kLists = PAIR ? 2 : 1;
     const int ew = warp - 2;       // 0..EW-1
     const int g = ew >> 2;         // this warp's index within its lane group
     const int lg = warp & 3;       // TMEM lane group this warp may access
@@ -690,12 +692,12 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       const FusedItem& p = A.items[MAXI == 1 ? 0 : ii];  // one item: constants at fixed addresses
       const int P = p.pool_cap;
       const int U = p.units_per_block;
-      const int S = OWN ? 1 : MINIMA ? 1024 : pool_sync_tiles(P, p.kprime);
+      const int S = OWN ? 1 : pool_sync_tiles(P, p.kprime);
       if (u_ord < 0 || u_ord >= U) {  // identical in every epilogue warp: both of a pair leave here
         raise_abort(abort_flag, B.status, kErrBadSchedule);
         break;
       }
-      const int qbw = OWN ? qb + g : qb;  // this warp's query block
+      const int qbw = DUAL ? qb + g : qb;  // this warp's query block
       const int q = qbw * kBM + row;
       const bool valid = q < p.nq;
       const float qn = valid ? p.q_norms[q] : 0.f;
@@ -712,8 +714,11 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       const float km = fold ? ku : 1.f;
       auto key_d = [&](float x) -> float { return Tr::kFolded ? x : fmaf(km, x, qn); };
       const size_t pool_row0 = (size_t)qbw * kBM;  // pool index of lane-group row 0 is added per lane
+      auto list_of = [&](int r) -> size_t {
+        return ((pool_row0 + (size_t)r) * U + (size_t)u_ord) * kLists + (kLists > 1 ? g : 0);
+      };
       auto pool_of = [&](int r) -> uint64_t* {
-        return p.pools + ((pool_row0 + (size_t)r) * U + (size_t)u_ord) * (size_t)P;
+        return p.pools + list_of(r) * (size_t)P;
       };
       uint64_t* pool = pool_of(row);
       // a new unit starts with an empty pool (the previous unit's last barrier
@@ -812,7 +817,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             // < nb_pad: rows are padded to whole tiles (a strided sample has no padding)
-            const int c0 = tile0 + (OWN ? 0 : g * kHalfN) + 32 * i + lane;
+            const int c0 = tile0 + (DUAL ? 0 : g * kHalfN) + 32 * i + lane;
             const size_t c = MINIMA ? (size_t)c0 * (size_t)p.db_step : (size_t)c0;
             pxn[i] = __ldg(p.db_norms + c);
             psx[i] = uniform ? 0.f : __ldg(p.db_scale + c);
@@ -836,7 +841,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
           __syncwarp();
         }
         const uint32_t t_src = tmem_base + lane_base + slot * kBN + g * kHalfN;
-        const int tcol = tile0 + (OWN ? 0 : g * kHalfN);  // database row of the warp's first column
+        const int tcol = tile0 + (DUAL ? 0 : g * kHalfN);  // database row of the warp's first column
         // Smallest distance of every 8 of the warp's 128 columns: half an
         // instruction a column (the masks of every column took 1.5) decides
         // whether anything of the tile survives, and which eights hold it.  The
@@ -945,7 +950,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
           // pools that may not have room for the next tile, or, at the unit's
           // end, every pool above k' (the merge pass reads at most k' keys'
           // worth beyond what it needs)
-          const int lim = t + 1 < t1 ? P - kTileRows : p.kprime;
+          const int lim = t + 1 < t1 ? P - kHalfN : p.kprime;
           const uint32_t need = __ballot_sync(0xffffffffu, valid && own_cnt > lim);
           if (need) {
             if (own_cnt > P) atomicOr(B.status, kErrPoolOverflow);
@@ -980,8 +985,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       // the merge pass selects exactly
       if (!MINIMA && valid && (OWN || g == 0)) {
         const int cn = OWN ? own_cnt : cnt_s[row];
-        p.pool_counts[(pool_row0 + row) * U + u_ord] = cn < P ? cn : P;
-        if (gap) p.pool_counts[(pool_row0 + row) * U + u_ord - 1] = 0;
+        p.pool_counts[list_of(row)] = cn < P ? cn : P;
+        if (gap) p.pool_counts[list_of(row) - kLists] = 0;
       }
       if constexpr (!OWN) bar_sync_named(pair_bar, kGroupThreads);  // the counts are read before the next unit resets them
     }
@@ -1255,7 +1260,9 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
   const int d0 = n > 0 ? specs[0].d : 0;
   const bool want_pair = pm == 1 || (pm == kPairsAuto && ((form == kFormBF16 && d0 >= kPairMinDimBF16) ||
                                                           (form == kFormExact && d0 >= kPairMinDimExact)));
-  const int pair = (!dual && grouped && want_pair && max_ctas >= 2) ? 1 : 0;
+  bool lean = false;
+  for (int i = 0; i < n; ++i) lean = lean || specs[i].fill_kprime >= kFillSingle;
+  const int pair = (!dual && !lean && grouped && want_pair && max_ctas >= 2) ? 1 : 0;
   const int rows = kBM << (pair | dual);
   const int tile_rows = dual ? kBN / 2 : kBN;
   long long total = 0;

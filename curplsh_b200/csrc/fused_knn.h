@@ -18,6 +18,7 @@ struct FusedPlan {
   int dual = 0;               // 1: one CTA holds two query blocks against 128-row database tiles
   // pool rows of the plan (pools and counts are indexed by query row)
   long long pool_rows() const { return (long long)num_qblocks * (128LL << (pair | dual)); }
+  int lists_per_unit() const { return pair ? 2 : 1; }  // candidate pools of one query in one unit
 };
 
 // Tuned launch parameters for one (form, d, k, Q) bucket (tuning.cpp).
@@ -165,7 +166,13 @@ struct EstimatePlan {
 };
 // The estimate a search of nq queries with k' candidates against n rows uses
 // (on == false: none), whatever the process-wide switch says.
-EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms);
+// `lean`: only the estimates of at most a tenth of the rows among 128-row blocks,
+// for callers short of working memory.
+EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms, bool lean = false);
+// FusedItemSpec::fill_kprime of a lean plan, which keeps single query blocks:
+// dual blocks and CTA pairs round the pools up to 256 queries and pairs have two
+// pools per query and unit.
+constexpr int kFillSingle = 1 << 30;
 // The process-wide switch (curplsh_set_bound_estimate).
 bool bound_estimate_enabled();
 
@@ -251,6 +258,7 @@ constexpr int kMergeMaxItems = 128;
 struct MergeItem {
   int nq, k, kprime, pool_cap, num_tiles, units_per_block;
   int pair;                // the fused launch ran CTA pairs (query groups of 256 rows)
+  int lists;               // pools of one query in one unit (2 with CTA pairs)
   int row0;                // first pool row of this item within its fused item
   int split_tiles;         // the fused item's resolved split length L
   long long work_begin;    // the fused item's offset in its launch's flattened work space

@@ -151,8 +151,8 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   const long long first = (m.work_begin + (long long)qb * T) / W;
   const long long last = (m.work_begin + (long long)(qb + 1) * T - 1) / W;
   // an empty database has no pools; otherwise one list per unit
-  const int nlists = T > 0 ? (int)(last - first + 1 + (T - 1) / m.split_tiles) : 0;
-  const size_t list0 = (size_t)prow * U;  // pool-list index of unit 0
+  const int nlists = T > 0 ? (int)(last - first + 1 + (T - 1) / m.split_tiles) * m.lists : 0;
+  const size_t list0 = (size_t)prow * U * m.lists;  // pool-list index of unit 0
   // Final bound of the fused pass on this query's k'-th coarse distance: the
   // smallest k'-th of any pool, or the estimate the pass started from.  When
   // it comes from a pool, every key of the k' smallest has a distance <= it.
@@ -445,7 +445,7 @@ cudaError_t launch_merge_batch(MergeItem* items, int n, int d, uint32_t* status,
     items[i].q_begin = qsum;
     qsum += items[i].nq > 0 ? items[i].nq : 0;
     if (items[i].kprime > kpmax) kpmax = items[i].kprime;
-    if (items[i].units_per_block > umax) umax = items[i].units_per_block;
+    umax = std::max(umax, items[i].units_per_block * items[i].lists);
     a.items[i] = items[i];
   }
   if (qsum == 0) return cudaSuccess;
@@ -487,6 +487,7 @@ cudaError_t launch_merge_rerank(const MergeLaunch& m, cudaStream_t st) {
   it.num_tiles = m.plan.num_tiles;
   it.units_per_block = m.plan.units_per_block;
   it.pair = m.plan.pair | m.plan.dual;
+  it.lists = m.plan.lists_per_unit();
   it.row0 = 0;
   it.split_tiles = m.plan.split_tiles > 0 ? m.plan.split_tiles : 1;
   it.work_begin = 0;

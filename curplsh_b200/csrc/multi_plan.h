@@ -34,9 +34,9 @@ class MultiPlan {
  public:
   // `uniq` are the distinct indexes (sorted by address), `views` their locked
   // views (updated when an FP8 copy has to be built).  Requests with num == 0
-  // are skipped.
+  // are skipped.  `lean` plans for less working memory (see plan_estimate).
   int build(const curplsh_batch_item* items, int n, const std::vector<curplsh_index*>& uniq,
-            std::vector<IndexView>& views, int precision, int rerank_factor, int num_sms);
+            std::vector<IndexView>& views, int precision, int rerank_factor, int num_sms, bool lean = false);
   size_t bytes() const { return bytes_; }
   void bind(void* base);
   uint32_t* status() const { return status_; }

@@ -174,8 +174,13 @@ int build_step(curplsh_server* s, const std::vector<int64_t>& tickets, std::vect
     if (!r.o_dev) st_bytes += rup((size_t)r.num * r.k * (sizeof(int32_t) + sizeof(float)), 256);
   }
   *staging = st_bytes;
-  return plan.build(items.data(), (int)items.size(), uniq, views, s->cfg.precision, s->cfg.rerank_factor,
-                    s->num_sms);
+  int rc = plan.build(items.data(), (int)items.size(), uniq, views, s->cfg.precision, s->cfg.rerank_factor,
+                      s->num_sms);
+  // a step over the whole budget is planned again for less working memory
+  if (!rc && rup(plan.bytes(), 256) + st_bytes > (size_t)s->cfg.memory_budget)
+    rc = plan.build(items.data(), (int)items.size(), uniq, views, s->cfg.precision, s->cfg.rerank_factor,
+                    s->num_sms, true);
+  return rc;
 }
 
 void finish_step(curplsh_server* s, Step& st) {
@@ -503,12 +508,18 @@ int curplsh_server_submit(curplsh_server* s, int64_t num, const float* queries, 
     it.indices = indices;
     it.distances = distances;
     MultiPlan p;
-    int rc = p.build(&it, 1, uniq, views, s->cfg.precision, s->cfg.rerank_factor, s->num_sms);
+    size_t staging = 0;
+    if (!r.q_dev) staging += rup((size_t)num * s->dim * sizeof(float), 256);
+    if (!r.o_dev) staging += rup((size_t)num * k * (sizeof(int32_t) + sizeof(float)), 256);
+    int rc = 0;
+    size_t need = 0;
+    for (int lean = 0; lean < 2 && !rc; ++lean) {  // as build_step plans it
+      rc = p.build(&it, 1, uniq, views, s->cfg.precision, s->cfg.rerank_factor, s->num_sms, lean != 0);
+      need = rup(p.bytes(), 256) + staging;
+      if (need <= (size_t)s->cfg.memory_budget) break;
+    }
     index_unlock(s->index);
     if (rc) return rc;
-    size_t need = rup(p.bytes(), 256);
-    if (!r.q_dev) need += rup((size_t)num * s->dim * sizeof(float), 256);
-    if (!r.o_dev) need += rup((size_t)num * k * (sizeof(int32_t) + sizeof(float)), 256);
     if (need > (size_t)s->cfg.memory_budget)
       return fail(CURPLSH_ERR_INVALID_ARG, "request needs %zu bytes of working memory, more than the budget %lld",
                   need, (long long)s->cfg.memory_budget);

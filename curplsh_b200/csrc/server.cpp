@@ -277,6 +277,13 @@ bool issue_step(curplsh_server* s, std::unique_lock<std::mutex>& lk) {
   }
   st->tickets = take;
   slot.busy = true;
+  // Requests may be submitted while this step is enqueued (some 100 us of
+  // launches): held through it, the lock let one request at a time in and a
+  // burst of small ones ran one per step.  The step's requests stay where they
+  // are until they are done.
+  std::vector<Request*> rq;
+  for (int64_t t : take) rq.push_back(&s->reqs[t]);
+  lk.unlock();
   // ---- bind memory: [plan][staging...]; host inputs go through the pinned slot buffer
   char* dbase = static_cast<char*>(s->arena_mem) + st->off;
   st->plan.bind(dbase);
@@ -285,7 +292,7 @@ bool issue_step(curplsh_server* s, std::unique_lock<std::mutex>& lk) {
   size_t po = pinned_query_bytes(s);     // pinned output cursor
   cudaError_t e = cudaEventRecord(slot.ev_begin, slot.st);
   for (size_t i = 0; i < take.size(); ++i) {
-    Request& r = s->reqs[take[i]];
+    Request& r = *rq[i];
     curplsh_batch_item& it = items[i];
     if (!r.q_dev) {
       const size_t qb = (size_t)r.num * s->dim * sizeof(float);
@@ -312,7 +319,7 @@ bool issue_step(curplsh_server* s, std::unique_lock<std::mutex>& lk) {
   index_unlock(s->index);
   if (!rc && e == cudaSuccess) {
     for (size_t i = 0; i < take.size(); ++i) {
-      Request& r = s->reqs[take[i]];
+      Request& r = *rq[i];
       if (r.o_dev) continue;
       const size_t ni = (size_t)r.num * r.k;
       e = cudaMemcpyAsync(slot.pinned + po, items[i].indices, ni * sizeof(int32_t), cudaMemcpyDeviceToHost, slot.st);
@@ -329,6 +336,7 @@ bool issue_step(curplsh_server* s, std::unique_lock<std::mutex>& lk) {
                         cudaMemcpyDeviceToHost, slot.st);
   if (!rc && e == cudaSuccess) e = cudaEventRecord(slot.ev_end, slot.st);
   if (!rc && e == cudaSuccess) e = cudaLaunchHostFunc(slot.st, on_step_done, s);
+  lk.lock();
   if (rc || e != cudaSuccess) {
     if (e != cudaSuccess) {
       cudaGetLastError();

@@ -1223,9 +1223,7 @@ int curplsh_index_bf_create(curplsh_resources* r, int dim, const curplsh_bf_conf
   ix->cfg = c;
   ix->dres = d;
   ix->ld16 = round_up(dim + kAugCols, 8);  // BF16 rows carry the augmented norm columns
-  // FP8 rows: the codes, then, when round_up(d, 32) leaves 32 bytes of the
-  // last 128-byte K chunk free, the BF16 norm tail there
-  ix->ld8 = (round_up(dim, 32) % 128 != 0) ? round_up(dim, 32) + 32 : round_up(dim, 16);
+  ix->ld8 = round_up(dim, 32) + 32;  // FP8 rows: the codes, then the BF16 norm tail
   r->refs.fetch_add(1);
   DeviceScope scope(c.device);
   cudaError_t e = ix->alloc(&ix->status, 6 * sizeof(uint32_t), d->def);

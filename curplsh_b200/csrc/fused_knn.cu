@@ -51,7 +51,7 @@ template <>
 struct FormTraits<kFormExact> {
   static constexpr int kAParts = 2, kBParts = 2, kProducts = 3;
   static constexpr int kChunkElems = 64, kStepElems = 16;  // bf16
-  static constexpr bool kFP8 = false;
+  static constexpr bool kFP8 = false, kRowScales = false;
   static constexpr bool kFolded = true;  // norms ride in the augmented K columns
   // products: hi*hi, hi*lo, lo*hi  (the lo*lo term, O(2^-16) relative, is dropped)
   __device__ static constexpr int a_part(int p) { return p == 2 ? 1 : 0; }
@@ -61,19 +61,31 @@ template <>
 struct FormTraits<kFormBF16> {
   static constexpr int kAParts = 1, kBParts = 1, kProducts = 1;
   static constexpr int kChunkElems = 64, kStepElems = 16;
-  static constexpr bool kFP8 = false;
+  static constexpr bool kFP8 = false, kRowScales = false;
   static constexpr bool kFolded = true;
   __device__ static constexpr int a_part(int) { return 0; }
   __device__ static constexpr int b_part(int) { return 0; }
 };
-template <>
-struct FormTraits<kFormFP8> {
+// The FP8 form's kernels for databases with per-row scales: no norm tails, the
+// norms and scales are applied in the epilogue.  A form of its own at compile
+// time: as a run-time branch it cost the tiles with tails a sixth of their pass
+// (FP8 sphere 17.5 -> 14.8 ms).
+constexpr int kFormFP8Rows = 3;
+struct FP8Traits {
   static constexpr int kAParts = 1, kBParts = 1, kProducts = 1;
   static constexpr int kChunkElems = 128, kStepElems = 32;  // e4m3
   static constexpr bool kFP8 = true;
-  static constexpr bool kFolded = false;  // per-row scales: norms are applied in the epilogue
+  static constexpr bool kFolded = false;  // the accumulator is d / (2 s_q s), or needs norms and scales
   __device__ static constexpr int a_part(int) { return 0; }
   __device__ static constexpr int b_part(int) { return 0; }
+};
+template <>
+struct FormTraits<kFormFP8> : FP8Traits {
+  static constexpr bool kRowScales = false;
+};
+template <>
+struct FormTraits<kFormFP8Rows> : FP8Traits {
+  static constexpr bool kRowScales = true;
 };
 
 constexpr uint32_t kAChunkBytes = kBM * kChunkBytes;  // 16 KB
@@ -110,15 +122,19 @@ __host__ __device__ inline SmemLayout make_layout(int form, int d, int pair = 0,
   SmemLayout L{};
   L.b_chunk = (pair || dual) ? kBChunkBytes / 2 : kBChunkBytes;
   L.b_tail = (pair || dual) ? kBTailBytes / 2 : kBTailBytes;
-  const bool folded = form != kFormFP8;
+  const bool folded = form != kFormFP8 && form != kFormFP8Rows;
   const int chunk_elems = folded ? 64 : 128;
   const int a_parts = (form == kFormExact) ? 2 : 1;
   const int b_parts = (form == kFormExact) ? 2 : 1;
   L.kdim = folded ? d + kAugCols : d;
   L.nkc = (L.kdim + chunk_elems - 1) / chunk_elems;
   // narrow tail only when it holds nothing but the norm columns (d % 64 == 0):
-  // the tail runs the hi x hi product alone, which is exact only for those
-  L.tail_narrow = folded && (d % 64 == 0);
+  // the tail runs the hi x hi product alone, which is exact only for those.
+  // FP8 rows: the norm tail, when the 32-byte steps of the codes fill the chunks
+  // (without a tail such dimensions loaded norms in the epilogue: 4,096 queries,
+  // 10^6 rows, d = 256 2.81 -> 1.46 ms, d = 512 2.98 -> 1.87).
+  L.tail_narrow = folded ? d % 64 == 0 : form == kFormFP8 && (d + 31) / 32 % 4 == 0;
+  if (!folded && L.tail_narrow) ++L.nkc;
   // everything below the barrier block must fit the 227 KB opt-in limit
   const uint32_t pool_bytes = dual ? 0u : 1024u;  // counts and bounds of 128 shared pools
   const uint32_t warp_bytes = (uint32_t)epi_warps * 1024u;  // radix histograms
@@ -515,41 +531,44 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       // a pair's MMA is 256 rows: this CTA's query block, then the partner's
       constexpr uint32_t kM = PAIR ? 2 * kBM : kBM, kN = DUAL ? kBN / 2 : kBN;
       constexpr uint32_t idesc = make_idesc(fmt, fmt, kM, kN);
-      // the FP8 form's BF16 norm tail: the same shape, BF16 operands
+      // the norm columns' step: the same shape, BF16 operands
       constexpr uint32_t idesc16 = make_idesc(1u, 1u, kM, kN);
-      auto mma = [&](uint32_t d_tmem, uint64_t ad, uint64_t bd, uint32_t acc) {
-        if constexpr (PAIR && Tr::kFP8)
-          mma_f8_ss_pair(d_tmem, ad, bd, idesc, acc);
-        else if constexpr (PAIR)
-          mma_f16_ss_pair(d_tmem, ad, bd, idesc, acc);
-        else if constexpr (Tr::kFP8)
-          mma_f8_ss(d_tmem, ad, bd, idesc, acc);
+      constexpr int kSteps = Tr::kChunkElems / Tr::kStepElems;
+      static_assert(kSteps == 4, "K steps of a chunk");
+      auto steps = [&](int n, uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t acc) {
+        if (n >= 4)
+          mma_steps<Tr::kFP8, PAIR, 4>(d, a_lo, b_lo, kDescHiSw128, idesc, acc);
+        else if (n == 3)
+          mma_steps<Tr::kFP8, PAIR, 3>(d, a_lo, b_lo, kDescHiSw128, idesc, acc);
+        else if (n == 2)
+          mma_steps<Tr::kFP8, PAIR, 2>(d, a_lo, b_lo, kDescHiSw128, idesc, acc);
         else
-          mma_f16_ss(d_tmem, ad, bd, idesc, acc);
+          mma_steps<Tr::kFP8, PAIR, 1>(d, a_lo, b_lo, kDescHiSw128, idesc, acc);
       };
-      auto mma_tail = [&](uint32_t d_tmem, uint64_t ad, uint64_t bd) {
-        if constexpr (PAIR)
-          mma_f16_ss_pair(d_tmem, ad, bd, idesc16, 1u);
-        else
-          mma_f16_ss(d_tmem, ad, bd, idesc16, 1u);
-      };
-      // completion goes to the barrier at the same offset in both CTAs of a pair
+      // (leader only) completion goes to the barrier at the same offset in both
+      // CTAs of a pair
       auto commit = [&](uint64_t* bar) {
-        if (leader) {
-          if constexpr (PAIR)
-            mma_commit_pair(bar);
-          else
-            mma_commit(bar);
-        }
-        __syncwarp();
+        if constexpr (PAIR)
+          mma_commit_pair(bar);
+        else
+          mma_commit(bar);
       };
+      // Everything a tile's issue needs, in descriptor units of 16 bytes
       const uint32_t smem_base = smem_u32(smem);
       const int nreg = L.nkc - (L.tail_narrow ? 1 : 0);
+      const int last_steps = (L.kdim - (nreg - 1) * KC + Tr::kStepElems - 1) / Tr::kStepElems;  // >= 4: whole
+      const uint32_t b_first = desc_lo(smem_base + L.a_bytes), stage16 = L.stage_bytes >> 4;
+      const uint32_t a_block16 = L.a_block >> 4;
+      constexpr uint32_t kA16 = kAChunkBytes >> 4;
+      const uint32_t b_chunk16 = L.b_chunk >> 4;
+      // queries: resident at a_first + chunk, or in the stage at b + a_in_stage
+      const uint32_t a_first = desc_lo(smem_base), a_in_stage = stage_a_off<Tr::kAParts, Tr::kBParts>(L, 0) >> 4;
+      const uint32_t tail16 = stage_tail_off<Tr::kAParts, Tr::kBParts>(L) >> 4;
       UnitWalk walk(blockIdx.x, B, rank);
       int ii, qb, t0, t1, u_ord, rot, unit = 0;
       bool gap;
-      int s = 0;                 // ring stage and its phase
-      uint32_t sphase = 0, tc = 0;
+      int s = 0;                 // ring stage, its phase and descriptor
+      uint32_t sphase = 0, tc = 0, b_lo = b_first;
       bool ok = true;
       STAT_DECL(st_full);
       STAT_DECL(st_acc);
@@ -561,7 +580,19 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
           }
           tc_fence_after();
         }
+        // The norm columns' K step (hi x hi alone carries them: lo rows are zero
+        // there): the 32-byte-swizzled narrow tail after the last chunk, or the
+        // FP8 rows' 32 bytes inside it (a K step of its 128-byte swizzled rows, as
+        // the FP8 steps before it), into the same FP32 accumulator.  A norm tail
+        // is BF16 in every form.
         const int fp8_tail = Tr::kFP8 ? A.items[MAXI == 1 ? 0 : ii].fp8_tail : 0;
+        const bool tail = Tr::kFP8 ? !Tr::kRowScales : L.tail_narrow != 0;
+        const uint32_t tail_hi = L.tail_narrow ? kDescHiSw32 : kDescHiSw128;
+        const uint32_t in_chunk16 = (uint32_t)(fp8_tail - (nreg - 1) * KC) >> 4;
+        const uint32_t tail_b = L.tail_narrow ? tail16 : in_chunk16;
+        const uint32_t tail_a = L.a_stream ? (L.tail_narrow ? tail16 + (L.b_tail >> 4) : a_in_stage + in_chunk16)
+                                : L.tail_narrow ? (a_res_off(L, nreg, 0, Tr::kAParts) >> 4)
+                                                : (a_res_off(L, nreg - 1, 0, Tr::kAParts) >> 4) + in_chunk16;
         for (int t = t0; t < t1 && ok; ++t, ++tc) {
           const uint32_t slot = tc & 1u, use = tc >> 1;
           STAT_BEGIN(ta);
@@ -573,6 +604,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
           STAT_END(ta, st_acc);
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + slot * kBN;
+          uint32_t a_lo = a_first;
           for (int kc = 0; kc < nreg; ++kc) {
             STAT_BEGIN(tf);
             if (!wait_or_abort(&full[s], sphase, abort_flag)) {
@@ -582,58 +614,42 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
             }
             STAT_END(tf, st_full);
             tc_fence_after();
-            const uint32_t st = smem_base + L.a_bytes + (uint32_t)s * L.stage_bytes;
-            const int rem = L.kdim - kc * KC;
-            constexpr int kSteps = Tr::kChunkElems / Tr::kStepElems;
-            const int nsteps = (rem + Tr::kStepElems - 1) / Tr::kStepElems;  // >= kSteps: a whole chunk
-            // resident queries: block j's chunk kc; streamed: the stage's own
-            const uint32_t a0 = L.a_stream ? st + stage_a_off<Tr::kAParts, Tr::kBParts>(L, 0)
-                                           : smem_base + a_res_off(L, kc, 0, Tr::kAParts);
+            if (L.a_stream) a_lo = b_lo + a_in_stage;
             const bool last = kc == nreg - 1;
-            const uint32_t tl = st + stage_tail_off<Tr::kAParts, Tr::kBParts>(L);
-            const uint32_t at = L.a_stream ? tl + L.b_tail : smem_base + a_res_off(L, nreg, 0, Tr::kAParts);
+            const int n = last ? last_steps : kSteps;
             if (leader) {
 #pragma unroll
               for (int j = 0; j < kQB; ++j) {  // dual: block j accumulates into columns j * 128 of the slot
                 const uint32_t dj = d_tmem + (uint32_t)j * (kBN / 2);
-                const uint32_t aj = a0 + (uint32_t)j * L.a_block;
 #pragma unroll
-                for (int pr = 0; pr < Tr::kProducts; ++pr) {
-                  const uint64_t ad = sw128_kmajor_desc(aj + Tr::a_part(pr) * kAChunkBytes);
-                  const uint64_t bd = sw128_kmajor_desc(st + Tr::b_part(pr) * L.b_chunk);
-#pragma unroll
-                  for (int ks = 0; ks < kSteps; ++ks)  // a K step is 32 bytes: descriptor + 2
-                    if (ks < nsteps) mma(dj, ad + 2 * ks, bd + 2 * ks, (pr | ks) ? 1u : (kc ? 1u : 0u));
-                }
-                if (Tr::kFP8 && last && fp8_tail > 0) {
-                  // the BF16 norm tails: one K=16 step at their byte offset in the
-                  // last chunk (a 32-byte K step of the 128-byte swizzled rows, as
-                  // the FP8 steps before it), into the same FP32 accumulator
-                  const uint32_t toff = (uint32_t)(fp8_tail - kc * KC);
-                  mma_tail(dj, sw128_kmajor_desc(aj + toff), sw128_kmajor_desc(st + toff));
-                }
-                // the 16 norm columns: only hi x hi carries them (lo rows are zero
-                // there), so one K step of product 0 with the 32-byte-swizzled tiles
-                if (!Tr::kFP8 && last && L.tail_narrow)
-                  mma_tail(dj, sw32_kmajor_desc(at + (uint32_t)j * L.a_block), sw32_kmajor_desc(tl));
+                for (int pr = 0; pr < Tr::kProducts; ++pr)
+                  steps(n, dj, a_lo + (uint32_t)j * a_block16 + (uint32_t)Tr::a_part(pr) * kA16,
+                        b_lo + (uint32_t)Tr::b_part(pr) * b_chunk16, pr ? 1u : (uint32_t)kc);
+                if (last && tail)
+                  mma_steps<false, PAIR, 1>(dj, (L.a_stream ? b_lo : a_first) + tail_a + (uint32_t)j * a_block16,
+                                            b_lo + tail_b, tail_hi, idesc16, 1u);
               }
+              commit(&empty[s]);
+              if (last) commit(&acc_full[slot]);
             }
             __syncwarp();
-            commit(&empty[s]);
+            a_lo += Tr::kAParts * kA16;
+            b_lo += stage16;
             if (++s == S) {
               s = 0;
               sphase ^= 1u;
+              b_lo = b_first;
             }
           }
-          if (!ok) break;
-          commit(&acc_full[slot]);
         }
-        if (!L.a_stream) commit(a_empty);
+        if (ok && leader && !L.a_stream) commit(a_empty);
+        __syncwarp();
         ++unit;
       }
       // Make sure every issued MMA has retired before TMEM is released (in
       // both CTAs of a pair: the commit reaches the partner's drain barrier).
-      commit(drain);
+      if (leader) commit(drain);
+      __syncwarp();
       mbar_wait(drain, 0);
       if (lane == 0) {
         STAT_FLUSH(kStatMmaWaitFull, st_full);
@@ -658,7 +674,9 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
     //   Dual blocks (OWN): warp g filters query block qb + g alone, so a lane
     // owns its query's pool: its count and bound live in registers and the
     // warps meet nowhere.  CTA pairs do the same with two pools per query, one
-    // per warp (kLists); block minima need no pool at all.
+    // per warp (kLists): an accumulator waits for both CTAs' warps, so what the
+    // warps wait for each other is paid twice (FP32-exact integer mixture as
+    // pairs: full pass 5.30 -> 4.72 ms).  Block minima need no pool at all.
     constexpr bool OWN = DUAL || PAIR || MINIMA;
     constexpr int kLists = PAIR ? 2 : 1;
     const int ew = warp - 2;       // 0..EW-1
@@ -704,13 +722,12 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       // FP8: d = ||x||^2 + 2 s_q s_x acc (the query codes are stored negated)
       float s2 = 2.f;
       if (Tr::kFP8) s2 = valid ? 2.f * p.q_scale[q] : 0.f;
-      // FP8 with one scale s for every database row: d = ||x||^2 + 2 s_q s acc
-      const bool uniform = Tr::kFP8 && p.db_scale_uniform > 0.f;
+      // FP8 with one scale s for every database row and the norm tails: the
+      // accumulator is d / ku, ku = 2 s_q s; the filter compares ku acc with the
+      // bound and scales only the survivors (km = 1: the accumulator is d itself
+      // or is made d below)
+      constexpr bool fold = Tr::kFP8 && !Tr::kRowScales;
       const float ku = s2 * p.db_scale_uniform;
-      // with the norm tails the accumulator is d / ku: the filter compares
-      // ku acc with the bound and scales only the survivors (km = 1: the
-      // accumulator is d itself or is made d below)
-      const bool fold = Tr::kFP8 && p.fp8_tail > 0;
       const float km = fold ? ku : 1.f;
       auto key_d = [&](float x) -> float { return Tr::kFolded ? x : fmaf(km, x, qn); };
       const size_t pool_row0 = (size_t)qbw * kBM;  // pool index of lane-group row 0 is added per lane
@@ -778,15 +795,23 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       };
 
       float* colv = reinterpret_cast<float*>(hist);  // FP8 without tails: [128] norms, then [128] scales
-      // Coarse distances of accumulator columns c, c + 1, ... of this warp's 128:
-      // the accumulator itself (BF16 and exact forms), d / ku (FP8 with norm
-      // tails), else from the staged norms and scales.
+      // Coarse distances of `count` (a multiple of 4) accumulator columns from c
+      // on of this warp's 128: the accumulator itself (BF16 and exact forms),
+      // d / ku (FP8 with norm tails), else from the staged norms and scales.
       auto dist_of = [&](const uint32_t* v, int c, float* x, int count) {
 #pragma unroll
-        for (int j = 0; j < count; ++j) {
-          x[j] = __uint_as_float(v[j]);
-          if (Tr::kFP8 && !fold)
-            x[j] = uniform ? fmaf(x[j], ku, colv[c + j]) : fmaf(x[j] * colv[kHalfN + c + j], s2, colv[c + j]);
+        for (int j = 0; j < count; ++j) x[j] = __uint_as_float(v[j]);
+        if (Tr::kRowScales) {
+          const float4* xn4 = reinterpret_cast<const float4*>(colv + c);
+          const float4* sx4 = reinterpret_cast<const float4*>(colv + kHalfN + c);
+#pragma unroll
+          for (int j = 0; j < count; j += 4) {  // fma(acc * s_x, 2 s_q, ||x||^2)
+            const float4 xn = xn4[j / 4], sx = sx4[j / 4];
+            x[j] = fmaf(x[j] * sx.x, s2, xn.x);
+            x[j + 1] = fmaf(x[j + 1] * sx.y, s2, xn.y);
+            x[j + 2] = fmaf(x[j + 2] * sx.z, s2, xn.z);
+            x[j + 3] = fmaf(x[j + 3] * sx.w, s2, xn.w);
+          }
         }
       };
 
@@ -813,14 +838,14 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
         // overlaps it) and staged in the warp's histogram area, which is free
         // outside a refresh
         float pxn[4], psx[4];
-        if (Tr::kFP8 && !fold) {
+        if (Tr::kRowScales) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             // < nb_pad: rows are padded to whole tiles (a strided sample has no padding)
             const int c0 = tile0 + (DUAL ? 0 : g * kHalfN) + 32 * i + lane;
             const size_t c = MINIMA ? (size_t)c0 * (size_t)p.db_step : (size_t)c0;
             pxn[i] = __ldg(p.db_norms + c);
-            psx[i] = uniform ? 0.f : __ldg(p.db_scale + c);
+            psx[i] = __ldg(p.db_scale + c);
           }
         }
         STAT_BEGIN(tw);
@@ -831,7 +856,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
         if (got) {
         STAT_BEGIN(tfl);
         tc_fence_after();
-        if (Tr::kFP8 && !fold) {
+        if (Tr::kRowScales) {
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -1096,7 +1121,7 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
   a.B.status = status;
   a.B.stats = stats;
   a.B.run_if = run_if;
-  const bool fp8 = FORM == kFormFP8;
+  constexpr bool fp8 = FormTraits<FORM>::kFP8;
   for (int i = 0; i < n; ++i) {
     const FusedItemSpec& f = specs[i];
     const FusedItemPlan& pl = plans[i];
@@ -1120,7 +1145,7 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
     it.q_bound = f.q_bound;
     it.db_step = f.db_step > 1 ? f.db_step : 1;
     it.db_scale_uniform = f.xs_uniform;
-    it.fp8_tail = (fp8 && f.xs_uniform > 0.f) ? (int)fp8_tail_offset(f.d, f.ld8) : 0;
+    it.fp8_tail = FORM == kFormFP8 ? (int)fp8_tail_offset(f.d, f.ld8) : 0;
     it.minima = f.minima;
     it.minima_rows = f.minima_rows;
     CUtensorMap* m = &a.maps[i * kMapsPerItem];
@@ -1139,14 +1164,9 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
       m[kMapQLo] = m[kMapQHi];
       m[kMapXLo] = m[kMapXHi];
     }
-    if (FORM != kFormFP8) {
-      if (!make_map(&m[kMapQTail], f.qh, false, f.nq_pad, f.ld16, kBM, true) ||
-          !make_map(&m[kMapXTail], f.xh, false, f.nb_pad, f.ld16, xrows, true, step))
-        return cudaErrorInvalidValue;
-    } else {
-      m[kMapQTail] = m[kMapQHi];
-      m[kMapXTail] = m[kMapXHi];
-    }
+    if (!make_map(&m[kMapQTail], qh, fp8, f.nq_pad, ldq, kBM, true) ||
+        !make_map(&m[kMapXTail], xh, fp8, f.nb_pad, ldq, xrows, true, step))
+      return cudaErrorInvalidValue;
   }
   if (!PAIR) {
     fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL><<<bp.grid, kNumThreads, smem, st>>>(a);
@@ -1324,36 +1344,29 @@ void plan_fused(int nq, int nb, int num_sms, FusedPlan* out, int split_q4, int f
 
 uint32_t fused_smem_bytes(int form, int d) { return make_layout(form, d).total; }
 
+template <int FORM>
+static cudaError_t prepare_form() {
+  cudaError_t e = ensure_attributes<FORM, 1>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, 1, true>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, 1, false, true>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, 1, true, true>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, 1, false, false, true>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, kFusedMaxItems>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, kFusedMaxItems, false, true>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, kFusedMaxItems, false, false, true>();
+  return e;
+}
+
 cudaError_t prepare_fused_kernels(int form) {
-  cudaError_t e;
   switch (form) {
     case kFormExact:
-      e = ensure_attributes<kFormExact, 1>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormExact, 1, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormExact, 1, false, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormExact, 1, true, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormExact, kFusedMaxItems, false, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormExact, 1, false, false, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormExact, kFusedMaxItems, false, false, true>();
-      return e != cudaSuccess ? e : ensure_attributes<kFormExact, kFusedMaxItems>();
+      return prepare_form<kFormExact>();
     case kFormBF16:
-      e = ensure_attributes<kFormBF16, 1>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormBF16, 1, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormBF16, 1, false, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormBF16, 1, true, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormBF16, kFusedMaxItems, false, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormBF16, 1, false, false, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormBF16, kFusedMaxItems, false, false, true>();
-      return e != cudaSuccess ? e : ensure_attributes<kFormBF16, kFusedMaxItems>();
-    case kFormFP8:
-      e = ensure_attributes<kFormFP8, 1>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormFP8, 1, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormFP8, 1, false, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormFP8, 1, true, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormFP8, kFusedMaxItems, false, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormFP8, 1, false, false, true>();
-      if (e == cudaSuccess) e = ensure_attributes<kFormFP8, kFusedMaxItems, false, false, true>();
-      return e != cudaSuccess ? e : ensure_attributes<kFormFP8, kFusedMaxItems>();
+      return prepare_form<kFormBF16>();
+    case kFormFP8: {
+      const cudaError_t e = prepare_form<kFormFP8>();
+      return e != cudaSuccess ? e : prepare_form<kFormFP8Rows>();
+    }
     default:
       return cudaErrorInvalidValue;
   }
@@ -1373,8 +1386,14 @@ cudaError_t launch_fused_batch(int form, const FusedItemSpec* specs, const Fused
       return launch_form_any<kFormExact>(specs, plans, n, bp, status, stats, smem, st, run_if);
     case kFormBF16:
       return launch_form_any<kFormBF16>(specs, plans, n, bp, status, stats, smem, st, run_if);
-    case kFormFP8:
-      return launch_form_any<kFormFP8>(specs, plans, n, bp, status, stats, smem, st, run_if);
+    case kFormFP8: {
+      // one scale per database for all items of the launch, or per-row scales for all
+      const bool rows = !(specs[0].xs_uniform > 0.f);
+      for (int i = 1; i < n; ++i)
+        if (rows != !(specs[i].xs_uniform > 0.f)) return cudaErrorInvalidValue;
+      return rows ? launch_form_any<kFormFP8Rows>(specs, plans, n, bp, status, stats, smem, st, run_if)
+                  : launch_form_any<kFormFP8>(specs, plans, n, bp, status, stats, smem, st, run_if);
+    }
     default:
       return cudaErrorInvalidValue;
   }

@@ -187,11 +187,11 @@ bool bound_estimate_enabled();
 // rows [b_h b_l b_h] with b = -||x||^2 / (2 fixed_scale) (zeros without a
 // fixed scale).
 enum AugMode : int { kAugNone = 0, kAugDatabase = 1, kAugQuery = 2, kAugF8Query = 3, kAugF8Database = 4 };
-// Byte offset of the FP8 rows' 32-byte BF16 norm tail, round_up(d, 32), when
-// a row of stride ld8 has room for it inside its last 128-byte K chunk; else 0.
+// Byte offset of the FP8 rows' 32-byte BF16 norm tail, round_up(d, 32): inside
+// the last 128-byte K chunk, or a narrow chunk of its own when that is full.
 __host__ __device__ inline long long fp8_tail_offset(long long d, long long ld8) {
   const long long t8 = (d + 31) / 32 * 32;
-  return (t8 % 128 != 0 && t8 + 32 <= ld8) ? t8 : 0;
+  return t8 + 32 <= ld8 ? t8 : 0;
 }
 // `lo_nonzero` (optional) gets a nonzero value when some real row element is
 // not exactly representable in BF16 (its lo part is nonzero).

@@ -97,7 +97,10 @@ int MultiPlan::build(const curplsh_batch_item* items, int n, const std::vector<c
   for (size_t fi = 0; fi < fitems_.size(); ++fi) {
     const FItem& x = fitems_[fi];
     const IndexView& v = views[x.slot];
-    auto key = std::make_pair(x.form, x.d);
+    // FP8 databases with one scale and those with per-row scales have kernels of
+    // their own
+    const int kind = x.form == kFormFP8 && !(v.xs_uniform > 0.f) ? 3 : x.form;
+    auto key = std::make_pair(kind, x.d);
     auto g = gmap.find(key);
     int gi;
     if (g == gmap.end()) {

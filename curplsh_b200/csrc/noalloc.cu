@@ -92,7 +92,7 @@ Layout carve(int form, long long nq_pad, long long ld16, long long ld8, size_t p
     return at;
   };
   L.status = take(sizeof(uint32_t));
-  L.qh = take((size_t)nq_pad * ld16 * 2);
+  L.qh = form != kFormFP8 ? take((size_t)nq_pad * ld16 * 2) : 0;
   L.ql = form == kFormExact ? take((size_t)nq_pad * ld16 * 2) : 0;
   L.q8 = form == kFormFP8 ? take((size_t)nq_pad * ld8) : 0;
   L.qn = take((size_t)nq_pad * 4);

@@ -152,27 +152,48 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, both K-major, kind::f16 (bf16/f16 in, f32 acc).
-__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+// D[tmem] (+)= A[smem] * B[smem]^T over N consecutive 32-byte K steps, both
+// operands K-major, f32 accumulate; F8: e4m3 inputs (kind::f8f6f4), else f16 or
+// bf16 (kind::f16); PAIR: the 256-row MMA of a CTA pair, issued by rank 0 with
+// the offsets of each CTA's halves, the same in both CTAs.  Descriptors are given
+// as their low words and the high word they share; a K step inside the swizzled
+// row is + 2.  One asm block per group keeps the issue loop short: at six cycles
+// an instruction it is what bounds the light FP8 tiles.
+#define CURPLSH_MMA_STEP(I, K, P)                                                                         \
+  "add.u32 x, %1, " #I ";\n\tadd.u32 y, %2, " #I ";\n\tmov.b64 a, {x, %5};\n\tmov.b64 b, {y, %5};\n\t" \
+  "tcgen05.mma." K " [%0], a, b, %3, " P ";\n\t"
+#define CURPLSH_MMA_BLOCK(BODY)                                                                        \
+  asm volatile("{\n\t.reg .pred p, t;\n\t.reg .b32 x, y;\n\t.reg .b64 a, b;\n\t"                       \
+               "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\t" BODY "}" ::"r"(d_tmem),            \
+               "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(hi)                              \
+               : "memory")
+#define CURPLSH_MMA_N(K)                                                                               \
+  if constexpr (N == 1)                                                                                \
+    CURPLSH_MMA_BLOCK(CURPLSH_MMA_STEP(0, K, "p"));                                                    \
+  else if constexpr (N == 2)                                                                           \
+    CURPLSH_MMA_BLOCK(CURPLSH_MMA_STEP(0, K, "p") CURPLSH_MMA_STEP(2, K, "t"));                        \
+  else if constexpr (N == 3)                                                                           \
+    CURPLSH_MMA_BLOCK(CURPLSH_MMA_STEP(0, K, "p") CURPLSH_MMA_STEP(2, K, "t") CURPLSH_MMA_STEP(4, K, "t")); \
+  else                                                                                                 \
+    CURPLSH_MMA_BLOCK(CURPLSH_MMA_STEP(0, K, "p") CURPLSH_MMA_STEP(2, K, "t") CURPLSH_MMA_STEP(4, K, "t")   \
+                          CURPLSH_MMA_STEP(6, K, "t"))
+template <bool F8, bool PAIR, int N>
+__device__ __forceinline__ void mma_steps(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
+  static_assert(N >= 1 && N <= 4, "a 128-byte swizzled chunk has four K steps");
+  if constexpr (F8 && PAIR) {
+    CURPLSH_MMA_N("cta_group::2.kind::f8f6f4");
+  } else if constexpr (F8) {
+    CURPLSH_MMA_N("cta_group::1.kind::f8f6f4");
+  } else if constexpr (PAIR) {
+    CURPLSH_MMA_N("cta_group::2.kind::f16");
+  } else {
+    CURPLSH_MMA_N("cta_group::1.kind::f16");
+  }
 }
-
-// Same for 8-bit floating point inputs (kind::f8f6f4, e4m3 x e4m3 -> f32).
-__device__ __forceinline__ void mma_f8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
+#undef CURPLSH_MMA_N
+#undef CURPLSH_MMA_BLOCK
+#undef CURPLSH_MMA_STEP
 
 // Arrive (once) on an mbarrier when all previously issued tcgen05 async
 // operations of this thread have completed.
@@ -209,18 +230,13 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 //   bits 46-47 descriptor version (1 on sm_100)   bits 61-63 layout (2 = 128-byte swizzle)
 // The tile base must be 1024-byte aligned; a K step inside the 128-byte atom is
 // taken by advancing the start address (32 B per 16 bf16 / 32 fp8 elements).
-__device__ __forceinline__ uint64_t sw128_kmajor_desc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)1u << 16) | ((uint64_t)(1024u >> 4) << 32) |
-         ((uint64_t)1u << 46) | ((uint64_t)2u << 61);
-}
-
-// Same for a K-major tile with the 32-byte swizzle (TMA CU_TENSOR_MAP_SWIZZLE_32B,
-// 32-byte rows, 8-row groups 256 B apart), layout code 6.  One descriptor covers
-// one K step of 16 BF16 elements.  The tile base must be 256-byte aligned.
-__device__ __forceinline__ uint64_t sw32_kmajor_desc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)1u << 16) | ((uint64_t)(256u >> 4) << 32) |
-         ((uint64_t)1u << 46) | ((uint64_t)6u << 61);
-}
+// The low word is desc_lo(address), the high word a constant of the layout.
+constexpr uint32_t kDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);
+// A K-major tile with the 32-byte swizzle (TMA CU_TENSOR_MAP_SWIZZLE_32B, 32-byte
+// rows, 8-row groups 256 B apart), layout code 6.  One descriptor covers one K
+// step of 32 bytes.  The tile base must be 256-byte aligned.
+constexpr uint32_t kDescHiSw32 = (256u >> 4) | (1u << 14) | (6u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return ((saddr >> 4) & 0x3FFFu) | (1u << 16); }
 
 // ---------------------------------------------------------------- CTA pairs
 // A cluster of two CTAs on neighbouring SMs runs the MMA as one 256-row
@@ -283,26 +299,6 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 }
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// 256-row MMA of the pair (issued by rank 0): A and B descriptors give the
-// offsets of each CTA's halves, the same in both CTAs.
-__device__ __forceinline__ void mma_f16_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void mma_f8_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 // Arrive once on the mbarrier at `bar`'s offset in both CTAs of the pair
 // when the issuing thread's earlier tcgen05 operations have completed.

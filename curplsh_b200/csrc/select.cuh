@@ -307,7 +307,9 @@ __device__ __forceinline__ uint64_t warp_select_keep_stream(uint64_t* pool, int 
 }
 
 // Dispatch on the pool capacity: registers up to 1024 entries, else streaming.
-__device__ __forceinline__ uint64_t warp_select_keep_any(uint64_t* pool, int n, int keep, int cap, uint32_t* hist,
+// Not inlined: selections are rare, and their 64 key registers would press the
+// tile loop's values out to local memory.
+static __device__ __noinline__ uint64_t warp_select_keep_any(uint64_t* pool, int n, int keep, int cap, uint32_t* hist,
                                                          int& kept) {
   if (cap <= 512) return warp_select_keep_sampled<16>(pool, n, keep, cap, hist, kept);
   if (cap <= 1024) return warp_select_keep_sampled<32>(pool, n, keep, cap, hist, kept);

@@ -115,14 +115,57 @@ struct DevRes {
 };
 
 // Device memory of indexes and search workspaces comes from one pool per
-// resources and device, which keeps up to kPoolKeep bytes of freed memory for
-// the next index or workspace and goes back to the driver with the resources.
+// device, which keeps up to kPoolKeep bytes of freed memory for the next index
+// or workspace and goes back to the driver with the last resources that use it.
 // cudaMalloc, cudaFree and the pinned read-back took most of a one-shot search
 // (200,000 rows, 1,000 queries: 3.4 to 30 ms a call; 0.39 ms from the pool).
 // Larger buffers come from cudaMalloc: the pool maps and unmaps them at every
 // index (10 GB in 100 to 200 ms, against 25 to 100).
 constexpr uint64_t kPoolKeep = 512ull << 20;
 constexpr size_t kPoolMaxBytes = 256ull << 20;
+
+struct SharedPools {
+  struct Entry {
+    cudaMemPool_t pool = nullptr;
+    int refs = 0;
+  };
+  std::mutex mu;
+  std::map<int, Entry> by_device;
+  cudaError_t take(int device, cudaMemPool_t* out) {
+    std::lock_guard<std::mutex> lk(mu);
+    Entry& p = by_device[device];
+    if (p.refs == 0) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = device;
+      cudaError_t e = cudaMemPoolCreate(&p.pool, &props);
+      if (e != cudaSuccess) return e;
+      uint64_t keep = kPoolKeep;
+      e = cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) {
+        cudaMemPoolDestroy(p.pool);
+        return e;
+      }
+    }
+    ++p.refs;
+    *out = p.pool;
+    return cudaSuccess;
+  }
+  void give(int device) {  // the caller's memory from the pool is freed
+    std::lock_guard<std::mutex> lk(mu);
+    Entry& p = by_device[device];
+    if (--p.refs > 0) return;
+    cudaDeviceSynchronize();
+    cudaMemPoolDestroy(p.pool);
+    p.pool = nullptr;
+  }
+};
+// never destroyed: resources may be released while the process exits
+static SharedPools& shared_pools() {
+  static SharedPools* p = new SharedPools();
+  return *p;
+}
 
 // `st` orders the allocation; only work after it on `st` (or synchronised with
 // it) may use the memory.
@@ -243,13 +286,7 @@ int init_device(curplsh_resources* r, int device, DevRes** out) {
   CUDA_TRY(cudaStreamCreateWithFlags(&d.alt[1], cudaStreamNonBlocking));
   CUDA_TRY(cudaStreamCreateWithFlags(&d.copy, cudaStreamNonBlocking));
   CUDA_TRY(cudaDeviceGetAttribute(&d.num_sms, cudaDevAttrMultiProcessorCount, device));
-  cudaMemPoolProps props = {};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  props.location.id = device;
-  CUDA_TRY(cudaMemPoolCreate(&d.pool, &props));
-  uint64_t keep = kPoolKeep;
-  CUDA_TRY(cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  CUDA_TRY(shared_pools().take(device, &d.pool));
   auto res = r->devs.emplace(device, d);
   *out = &res.first->second;
   return CURPLSH_OK;
@@ -1127,8 +1164,7 @@ static void resources_release(curplsh_resources* r) {
   for (auto& kv : r->devs) {
     DeviceScope scope(kv.first);
     DevRes& d = kv.second;
-    cudaDeviceSynchronize();
-    cudaMemPoolDestroy(d.pool);
+    shared_pools().give(kv.first);
     if (d.def_owned) cudaStreamDestroy(d.def);
     cudaStreamDestroy(d.alt[0]);
     cudaStreamDestroy(d.alt[1]);

@@ -817,6 +817,11 @@ int search_device(curplsh_index* ix, const SearchShape& sh, int nq, const float*
   f.q_bound = b.qbound;
   f.status = ix->status;
   f.plan = plan;
+  // the kernels of one search are launched as programmatic dependents, except
+  // into a capture
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  f.pdl = cap == cudaStreamCaptureStatusNone;
   if (sh.est.on) {
     // sample pass over rows 0, step, 2 step, ...: block minima, no pools
     FusedLaunch e = f;
@@ -835,11 +840,11 @@ int search_device(curplsh_index* ix, const SearchShape& sh, int nq, const float*
     CUDA_TRY(fused_stats_print("sample", e, st));
 #endif
     // the j-th smallest block minimum of every query becomes its starting bound
-    CUDA_TRY(launch_estimate_select(b.minima, sh.est.blocks, nq, sh.est.j, b.qbound, st));
+    CUDA_TRY(launch_estimate_select(b.minima, sh.est.blocks, nq, sh.est.j, b.qbound, st, b.fail, f.pdl));
   } else {
     CUDA_TRY(cudaMemsetAsync(b.qbound, 0xFF, (size_t)nq_pad * sizeof(uint32_t), st));
   }
-  if (b.fail) CUDA_TRY(cudaMemsetAsync(b.fail, 0, 2 * sizeof(int), st));
+  if (b.fail && !sh.est.on) CUDA_TRY(cudaMemsetAsync(b.fail, 0, 2 * sizeof(int), st));
   tm->rec(2, st);
 #ifdef CURPLSH_FUSED_STATS
   CUDA_TRY(fused_stats_begin(&f, st));
@@ -850,6 +855,7 @@ int search_device(curplsh_index* ix, const SearchShape& sh, int nq, const float*
 #endif
   tm->rec(3, st);
   MergeLaunch m{};
+  m.pdl = f.pdl;
   m.nq = nq;
   m.nb = (int)ix->n;
   m.d = d;
@@ -881,8 +887,10 @@ int search_device(curplsh_index* ix, const SearchShape& sh, int nq, const float*
     CUDA_TRY(launch_fill_u32_if(b.qbound, nq_pad, 0xFFFFFFFFu, b.fail, st));
     FusedLaunch f2 = f;
     f2.run_if = b.fail;
+    f2.pdl = false;
     CUDA_TRY(launch_fused(f2, st));
     MergeLaunch m2 = m;
+    m2.pdl = false;
     m2.checks = 0;
     m2.fail_count = nullptr;
     m2.coarse_count = nullptr;

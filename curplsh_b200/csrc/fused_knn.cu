@@ -362,7 +362,10 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
   // a conditional pass (a re-search after a failed check): every thread of
   // every CTA reads the same flag, written by an earlier launch on the stream,
   // and leaves before any barrier or TMEM allocation when it is zero
-  if (B.run_if && *B.run_if == 0) return;
+  if (B.run_if) {
+    griddep_wait();
+    if (*B.run_if == 0) return;
+  }
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int EW = kEpiWarps;
@@ -427,6 +430,10 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
     __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // The prologue above touches nothing an earlier kernel writes.  This kernel does
+  // not let its own successor in early: merge CTAs resident beside the epilogue
+  // slowed it (284 queries, FP8, k' = 480: search 200 -> 260 us).
+  griddep_wait();
 
   const int KC = Tr::kChunkElems;
   auto maps_of = [&](int ii) { return &A.maps[(MAXI == 1 ? 0 : ii) * kMapsPerItem]; };
@@ -434,6 +441,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
+      fence_proxy_async();  // query operands written by the preparation kernel
       const uint64_t pol_db = l2_policy_evict_first();
       const uint64_t pol_q = l2_policy_evict_last();
       // a pair's loads complete on rank 0's barriers, which expect both CTAs' bytes
@@ -1168,24 +1176,9 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
         !make_map(&m[kMapXTail], xh, fp8, f.nb_pad, ldq, xrows, true, step))
       return cudaErrorInvalidValue;
   }
-  if (!PAIR) {
-    fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL><<<bp.grid, kNumThreads, smem, st>>>(a);
-    return cudaGetLastError();
-  }
-  if (bp.grid % 2) return cudaErrorInvalidValue;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)bp.grid, 1, 1);
-  cfg.blockDim = dim3(kNumThreads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL>, a);
+  if (PAIR && bp.grid % 2) return cudaErrorInvalidValue;
+  return launch_dependent(fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL>, (unsigned)bp.grid, kNumThreads, smem, st,
+                          bp.pdl != 0, PAIR ? 2 : 1, a);
 }
 
 template <int FORM>
@@ -1442,6 +1435,7 @@ cudaError_t launch_fused(const FusedLaunch& f, cudaStream_t st) {
   bp.grid = f.plan.grid;
   bp.pair = f.plan.pair;
   bp.dual = f.plan.dual;
+  bp.pdl = f.pdl ? 1 : 0;
   return launch_fused_batch(f.form, &s, &ip, 1, bp, f.status, f.stats, st, f.run_if);
 }
 

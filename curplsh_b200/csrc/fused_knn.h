@@ -71,6 +71,7 @@ struct FusedLaunch {
   uint32_t* status;
   unsigned long long* stats = nullptr;  // instrumented builds only
   const int* run_if = nullptr;          // non-null: the launch does nothing unless *run_if != 0
+  bool pdl = false;                     // a programmatic dependent of the stream's previous kernel
   FusedPlan plan;
 };
 
@@ -126,6 +127,7 @@ struct FusedBatchPlan {
   int grid = 0;
   int pair = 0;  // 1: clusters of two CTAs; work_per_cta is per pair and grid counts CTAs
   int dual = 0;  // 1: each CTA takes query groups of two blocks and 128-row database tiles
+  int pdl = 0;   // 1: launched as a programmatic dependent (launch_dependent)
 };
 // CTA pairs on (1) or off (0, default) for the plans made after the call.
 // CTA pairs: 0 off, 1 on (every grouped pass), kPairsAuto (the default): on
@@ -247,6 +249,7 @@ struct MergeLaunch {
   int* out_idx;
   float* out_dist;
   uint32_t* status;
+  bool pdl = false;  // a programmatic dependent of the stream's previous kernel
 };
 cudaError_t launch_merge_rerank(const MergeLaunch& m, cudaStream_t st);
 
@@ -288,7 +291,7 @@ struct MergeItem {
   float* out_dist;
 };
 cudaError_t launch_merge_batch(MergeItem* items, int n, int d, uint32_t* status, cudaStream_t st,
-                               const int* run_if = nullptr);
+                               const int* run_if = nullptr, bool pdl = false);
 cudaError_t prepare_merge_kernel();
 
 // Fill [n] ints / floats (N == 0 results, padding).
@@ -299,7 +302,9 @@ cudaError_t launch_fill_u32_if(uint32_t* p, long long n, uint32_t v, const int* 
 cudaError_t launch_add_count(unsigned long long* acc, const int* cnt, cudaStream_t st);
 // out[q] = order bits of the j-th smallest (1-based) of minima[q * count ..
 // q * count + count) for q < nq (all ones when count < j).
-cudaError_t launch_estimate_select(const float* minima, int count, int nq, int j, uint32_t* out, cudaStream_t st);
+// Clears fail[0..1] on the way (when not null).
+cudaError_t launch_estimate_select(const float* minima, int count, int nq, int j, uint32_t* out, cudaStream_t st,
+                                   int* fail = nullptr, bool pdl = false);
 // dst[i] = src[rows[i]] for i < n (rows of d floats).
 cudaError_t launch_gather_rows(const float* src, int d, const int* rows, int n, float* dst, cudaStream_t st);
 // out[rows[i]] = in[i] for i < n (result rows of k indices and distances).

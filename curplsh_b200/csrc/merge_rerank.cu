@@ -120,6 +120,8 @@ __device__ uint64_t block_select_bound(Each each, uint32_t keep, uint32_t* hist,
 // 40-register budget.
 template <int NT>
 __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(const __grid_constant__ MergeArgs a) {
+  griddep_launch();
+  griddep_wait();
   if (a.run_if && *a.run_if == 0) return;  // a conditional re-merge whose check passed
   int lo = 0, hi = a.num_items - 1;  // last item with q_begin <= blockIdx.x
   while (lo < hi) {
@@ -435,7 +437,7 @@ cudaError_t prepare_merge_kernel() {
 }
 
 cudaError_t launch_merge_batch(MergeItem* items, int n, int d, uint32_t* status, cudaStream_t st,
-                               const int* run_if) {
+                               const int* run_if, bool pdl) {
   if (n < 1 || n > kMergeMaxItems) return cudaErrorInvalidValue;
   MergeArgs a;
   memset(&a, 0, sizeof(a));
@@ -471,10 +473,8 @@ cudaError_t launch_merge_batch(MergeItem* items, int n, int d, uint32_t* status,
   if (e != cudaSuccess) return e;
   if (smem > 200 * 1024 || qsum > 0x7fffffffLL) return cudaErrorInvalidValue;
   if ((long long)kpmax * d <= kMergeSmallRerank)
-    merge_rerank_kernel<128><<<(unsigned)qsum, 128, smem, st>>>(a);
-  else
-    merge_rerank_kernel<256><<<(unsigned)qsum, 256, smem, st>>>(a);
-  return cudaGetLastError();
+    return launch_dependent(merge_rerank_kernel<128>, (unsigned)qsum, 128, smem, st, pdl, 1, a);
+  return launch_dependent(merge_rerank_kernel<256>, (unsigned)qsum, 256, smem, st, pdl, 1, a);
 }
 
 cudaError_t launch_merge_rerank(const MergeLaunch& m, cudaStream_t st) {
@@ -507,7 +507,7 @@ cudaError_t launch_merge_rerank(const MergeLaunch& m, cudaStream_t st) {
   it.ld16 = m.ld16;
   it.out_idx = m.out_idx;
   it.out_dist = m.out_dist;
-  return launch_merge_batch(&it, 1, m.d, m.status, st, m.run_if);
+  return launch_merge_batch(&it, 1, m.d, m.status, st, m.run_if, m.pdl);
 }
 
 }  // namespace curplsh_b200

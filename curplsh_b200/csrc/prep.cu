@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32) prep_rows_kernel(
     float pad_norm, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, long long ld16,
     uint8_t* __restrict__ f8, float* __restrict__ scale, long long ld8, int vec4, int aug,
     uint32_t* __restrict__ lo_nonzero, float fixed_scale) {
+  griddep_launch();
   const long long r = (long long)blockIdx.x * kPrepWarps + (threadIdx.x >> 5);
   if (r >= nrows_pad) return;
   prep_row(x, ldx, r, nrows, d, norms, pad_norm, hi, lo, ld16, f8, scale, ld8, vec4, aug, lo_nonzero, fixed_scale);
@@ -306,7 +307,11 @@ __global__ void fill_u32_if_kernel(uint32_t* p, long long n, uint32_t v, const i
 // bits, a 256-bin warp histogram in shared memory).
 constexpr int kSelectWarps = 8;
 __global__ void __launch_bounds__(kSelectWarps * 32)
-    estimate_select_kernel(const float* __restrict__ minima, int count, int nq, int j, uint32_t* __restrict__ out) {
+    estimate_select_kernel(const float* minima, int count, int nq, int j, uint32_t* out, int* fail) {  // no __restrict__:
+  // a load may not move above the wait
+  griddep_launch();
+  griddep_wait();
+  if (fail && blockIdx.x == 0 && threadIdx.x < 2) fail[threadIdx.x] = 0;
   __shared__ uint32_t hist_all[kSelectWarps][256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = blockIdx.x * kSelectWarps + warp;
@@ -477,11 +482,11 @@ cudaError_t launch_scatter_results(const int* in_idx, const float* in_dist, cons
   return cudaGetLastError();
 }
 
-cudaError_t launch_estimate_select(const float* minima, int count, int nq, int j, uint32_t* out, cudaStream_t st) {
+cudaError_t launch_estimate_select(const float* minima, int count, int nq, int j, uint32_t* out, cudaStream_t st,
+                                   int* fail, bool pdl) {
   if (nq <= 0) return cudaSuccess;
-  estimate_select_kernel<<<(unsigned)((nq + kSelectWarps - 1) / kSelectWarps), kSelectWarps * 32, 0, st>>>(
-      minima, count, nq, j, out);
-  return cudaGetLastError();
+  return launch_dependent(estimate_select_kernel, (unsigned)((nq + kSelectWarps - 1) / kSelectWarps),
+                          kSelectWarps * 32, 0, st, pdl, 1, minima, count, nq, j, out, fail);
 }
 
 }  // namespace curplsh_b200

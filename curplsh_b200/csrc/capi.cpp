@@ -914,21 +914,27 @@ size_t search_workspace_bytes(const curplsh_index* ix, const SearchShape& sh, in
 }
 
 // Searches again the `nf` queries listed at fail_dev + 2 (device) -- in the
-// exact form, without an estimate, so no check applies -- and writes their
-// results into the full result arrays.
+// exact form -- and writes their results into the full result arrays.  Queries
+// listed for their coarse margin alone may start from an estimate, which is
+// verified on the stream (`allow_est`; some 20 of 10^4 FP8 queries against 10^7
+// rows: re-search 1.13 -> 0.98 ms; all 10^4 of the integer mixture: search 11.9 ->
+// 9.8 ms); one whose estimate failed does not.
 int search_failed(curplsh_index* ix, int nf, const int* fail_dev, const float* q_dev, int k, int rerank_factor,
-                  int* out_idx, float* out_dist, cudaStream_t st, StreamWorkspace& w) {
+                  int* out_idx, float* out_dist, cudaStream_t st, StreamWorkspace& w, bool allow_est) {
   const int d = ix->dim;
   const int form = kFormExact;
   const size_t qbytes = (size_t)round_up((long long)nf * d * sizeof(float), 256);
   const size_t obytes = (size_t)round_up((long long)nf * k * (sizeof(int) + sizeof(float)), 256);
-  const SearchShape sh = search_shape(ix, nf, k, form, rerank_factor, false, false);
-  const size_t core = search_workspace_bytes(ix, sh, nf, form);
-  cudaError_t e = w.fb.ensure(qbytes + obytes + core, ix->dres, st);
-  if (e != cudaSuccess) {
+  SearchShape sh;
+  for (int lean = 0;; ++lean) {  // as in do_search
+    sh = search_shape(ix, nf, k, form, rerank_factor, allow_est && !lean, false, lean != 0);
+    const size_t core = search_workspace_bytes(ix, sh, nf, form);
+    const cudaError_t e = w.fb.ensure(qbytes + obytes + core, ix->dres, st);
+    if (e == cudaSuccess) break;
     cudaGetLastError();
-    return set_error(CURPLSH_ERR_OOM, "re-search workspace of %zu bytes: %s", qbytes + obytes + core,
-                     cudaGetErrorString(e));
+    if (lean)
+      return set_error(CURPLSH_ERR_OOM, "re-search workspace of %zu bytes: %s", qbytes + obytes + core,
+                       cudaGetErrorString(e));
   }
   char* base = static_cast<char*>(w.fb.ptr);
   float* qf = reinterpret_cast<float*>(base);
@@ -937,7 +943,7 @@ int search_failed(curplsh_index* ix, int nf, const int* fail_dev, const float* q
   CUDA_TRY(launch_gather_rows(q_dev, d, fail_dev + 2, nf, qf, st));
   Timing none;
   int* again = nullptr;
-  int rc = search_device(ix, sh, nf, qf, k, form, oif, odf, st, base + qbytes + obytes, &none, &again, false);
+  int rc = search_device(ix, sh, nf, qf, k, form, oif, odf, st, base + qbytes + obytes, &none, &again, true);
   if (rc) return rc;
   CUDA_TRY(launch_scatter_results(oif, odf, fail_dev + 2, nf, k, out_idx, out_dist, st));
   return CURPLSH_OK;
@@ -1056,7 +1062,7 @@ int do_search(curplsh_index* ix, int64_t num, const float* queries, int k, int p
       ix->coarse_queries.fetch_add(nc, std::memory_order_relaxed);
       // queries whose estimated bound was too small, or whose coarse margin
       // failed: search them again in the exact form
-      rc = search_failed(ix, nf, fail, qd, k, rf, oi, od, st, w);
+      rc = search_failed(ix, nf, fail, qd, k, rf, oi, od, st, w, est_on && nf == nc);
       if (rc) return rc;
       rc = copy_out();
       if (rc) return rc;

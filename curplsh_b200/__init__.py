@@ -562,8 +562,8 @@ def get_cta_pairs():
 
 
 def set_dual_blocks(enabled: bool) -> None:
-    """Process-wide switch of dual query blocks (on by default): FP8 fused passes
-    over >= 4 query blocks keep two blocks per CTA against 128-row database tiles
+    """Process-wide switch of dual query blocks (on by default): fused passes over
+    >= 4 query blocks, where two fit shared memory, keep two blocks per CTA against 128-row database tiles
     (results do not depend on it)."""
     _check(_lib.curplsh_set_dual_blocks(1 if enabled else 0))
 

@@ -424,7 +424,7 @@ int build_fp8(curplsh_index* ix, cudaStream_t st) {
       float lo, hi;
       memcpy(&lo, &range[0], sizeof(float));
       memcpy(&hi, &range[1], sizeof(float));
-      if (hi <= kFP8UniformSpan * lo) {
+      if (hi <= kFP8UniformSpan * lo && hi >= kFP8UniformMin) {
         CUDA_TRY(launch_prep_rows(ix->x32, ix->dim, (int)ix->n, ix->n_pad, ix->dim, nullptr, 0.f, nullptr, nullptr,
                                   ix->ld16, ix->x8, ix->xs, ix->ld8, st, kAugF8Database, nullptr, hi));
         ix->xs_uniform = hi;
@@ -791,7 +791,8 @@ int search_device(curplsh_index* ix, const SearchShape& sh, int nq, const float*
 
   tm->rec(1, st);
   CUDA_TRY(launch_prep_rows(q_dev, d, nq, nq_pad, d, b.qn, 0.f, form == kFormFP8 ? nullptr : b.qh, b.ql, ix->ld16,
-                            b.q8, b.qs, ix->ld8, st, form == kFormFP8 ? kAugF8Query : kAugQuery));
+                            b.q8, b.qs, ix->ld8, st, form == kFormFP8 ? kAugF8Query : kAugQuery, nullptr, 0.f,
+                            fp8_query_floor(ix->xs_uniform)));
   FusedLaunch f{};
   f.nq = nq;
   f.nb = (int)ix->n;

@@ -185,7 +185,7 @@ bool bound_estimate_enabled();
 // database rows get [n1 n2 n3 1 1 1] after column d, query rows are stored as -2q
 // followed by [1 1 1 m1 m2 m3]; lo rows get zeros there.  kAugF8Query /
 // kAugF8Database write the FP8 rows' BF16 norm tail (see fp8_tail_offset):
-// query rows (codes stored negated) [a_h a_h a_l] with a = -1/s_q (a zero row takes scale 1), database
+// query rows (codes stored negated) [a_h a_h a_l] with a = -1/s_q (s_q at least min_scale), database
 // rows [b_h b_l b_h] with b = -||x||^2 / (2 fixed_scale) (zeros without a
 // fixed scale).
 enum AugMode : int { kAugNone = 0, kAugDatabase = 1, kAugQuery = 2, kAugF8Query = 3, kAugF8Database = 4 };
@@ -195,12 +195,24 @@ __host__ __device__ inline long long fp8_tail_offset(long long d, long long ld8)
   const long long t8 = (d + 31) / 32 * 32;
   return t8 + 32 <= ld8 ? t8 : 0;
 }
+// The tail form holds ||x||^2 / (2 s_q s) in FP32, s_q and s the scales of the
+// query and of the database, and scales the accumulator by 2 s_q s.  Both stay in
+// FP32's normal range for s >= kFP8UniformMin and s_q >= s * 2^-36: the norm term
+// is then at most 448^2 d 2^35, and 2 s_q s at least 2^-123.  A query whose scale
+// the floor raises keeps its codes to the last bit down to 2^-42 of the rows'
+// magnitude, where its inner products are below the norms' rounding.  Databases
+// of smaller rows take a scale per row, whose kernel multiplies by one scale at a
+// time; the floor there only keeps 1 / s_q finite.
+constexpr float kFP8UniformMin = 1.f / (1ull << 44);
+__host__ __device__ inline float fp8_query_floor(float uniform_scale) {
+  return uniform_scale > 0.f ? uniform_scale * (1.f / (1ull << 36)) : 7.703719778e-34f;  // 2^-110
+}
 // `lo_nonzero` (optional) gets a nonzero value when some real row element is
 // not exactly representable in BF16 (its lo part is nonzero).
 cudaError_t launch_prep_rows(const float* x, long long ldx, int nrows, long long nrows_pad, int d, float* norms,
                              float pad_norm, __nv_bfloat16* hi, __nv_bfloat16* lo, long long ld16, uint8_t* f8,
                              float* scale, long long ld8, cudaStream_t st, int aug = kAugNone,
-                             uint32_t* lo_nonzero = nullptr, float fixed_scale = 0.f);
+                             uint32_t* lo_nonzero = nullptr, float fixed_scale = 0.f, float min_scale = 0.f);
 // out[0] / out[1] = order bits of the smallest / largest positive s[i], i < n
 // (0xFFFFFFFF / 0 when there is none)
 cudaError_t launch_positive_range(const float* s, long long n, uint32_t* out, cudaStream_t st);
@@ -219,6 +231,7 @@ struct PrepSegment {
   __nv_bfloat16* lo;
   uint8_t* f8;
   float* scale;
+  float min_scale;        // kAugF8Query: the query scales' floor (fp8_query_floor)
 };
 cudaError_t launch_prep_segments(PrepSegment* segs, int n, int d, long long ld16, long long ld8, float pad_norm,
                                  int aug, cudaStream_t st);

@@ -57,7 +57,7 @@ __device__ __forceinline__ bool prep_row(const float* __restrict__ x, long long 
                                          float* __restrict__ norms, float pad_norm, __nv_bfloat16* __restrict__ hi,
                                          __nv_bfloat16* __restrict__ lo, long long ld16, uint8_t* __restrict__ f8,
                                          float* __restrict__ scale, long long ld8, int vec4, int aug,
-                                         float fixed_scale = 0.f) {
+                                         float fixed_scale = 0.f, float min_scale = 0.f) {
   const int lane = threadIdx.x & 31;
   if (r >= nrows) {
     if (norms && lane == 0) norms[r] = pad_norm;
@@ -98,11 +98,11 @@ __device__ __forceinline__ bool prep_row(const float* __restrict__ x, long long 
   float inv = 1.f;
   if (f8) {
     m = warp_max(m);
-    // an all-zero row gets scale 0 (its codes are 0 whatever the scale); a
-    // zero query row with a norm tail gets 1, so its tail -1/s_q is finite
+    // an all-zero database row gets scale 0 (its codes are 0 whatever the
+    // scale); a query's is at least min_scale, see fp8_query_floor
     float sc = fixed_scale > 0.f ? fixed_scale : m / kE4M3Max;
     const bool q_tail = aug == kAugF8Query;
-    if (q_tail && !(sc > 0.f)) sc = 1.f;
+    if (q_tail) sc = fmaxf(sc, min_scale);
     inv = sc > 0.f ? 1.f / sc : 0.f;
     // query codes (and their norm tail) are stored negated, so that the FP8
     // accumulator grows with the distance; every rounding is symmetric
@@ -203,12 +203,13 @@ __global__ void __launch_bounds__(kPrepWarps * 32) prep_rows_kernel(
     const float* __restrict__ x, long long ldx, int nrows, long long nrows_pad, int d, float* __restrict__ norms,
     float pad_norm, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, long long ld16,
     uint8_t* __restrict__ f8, float* __restrict__ scale, long long ld8, int vec4, int aug,
-    uint32_t* lo_nonzero, float fixed_scale) {
+    uint32_t* lo_nonzero, float fixed_scale, float min_scale) {
   griddep_launch();
   const long long r = (long long)blockIdx.x * kPrepWarps + (threadIdx.x >> 5);
   bool lo_any = false;
   if (r < nrows_pad)
-    lo_any = prep_row(x, ldx, r, nrows, d, norms, pad_norm, hi, lo, ld16, f8, scale, ld8, vec4, aug, fixed_scale);
+    lo_any = prep_row(x, ldx, r, nrows, d, norms, pad_norm, hi, lo, ld16, f8, scale, ld8, vec4, aug, fixed_scale,
+                      min_scale);
   // One word says whether any row needs its lo part.  An atomic per row on it was
   // most of the preparation of FP32 rows (10^7 x 96: 9.5 ms, 3.4 with one look
   // per block and an atomic only while the word is still zero).
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32) prep_segments_kernel(const __
   const long long r = ((long long)blockIdx.x - g.block_begin) * kPrepWarps + (threadIdx.x >> 5);
   if (r >= g.rows) return;
   prep_row(g.x, a.d, r, g.nrows, a.d, g.norms, a.pad_norm, g.hi, g.lo, a.ld16, g.f8, g.scale, a.ld8, a.vec4[lo_i],
-           a.aug);
+           a.aug, 0.f, g.min_scale);
 }
 
 __global__ void __launch_bounds__(kPrepWarps * 32)
@@ -404,13 +405,13 @@ __global__ void scatter_results_kernel(const int* __restrict__ in_idx, const flo
 cudaError_t launch_prep_rows(const float* x, long long ldx, int nrows, long long nrows_pad, int d, float* norms,
                              float pad_norm, __nv_bfloat16* hi, __nv_bfloat16* lo, long long ld16, uint8_t* f8,
                              float* scale, long long ld8, cudaStream_t st, int aug, uint32_t* lo_nonzero,
-                             float fixed_scale) {
+                             float fixed_scale, float min_scale) {
   if (nrows_pad <= 0) return cudaSuccess;
   const int vec4 = (d % 4 == 0) && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
   const long long blocks = (nrows_pad + kPrepWarps - 1) / kPrepWarps;
   prep_rows_kernel<<<(unsigned)blocks, kPrepWarps * 32, 0, st>>>(x, ldx, nrows, nrows_pad, d, norms, pad_norm, hi,
                                                                  lo, ld16, f8, scale, ld8, vec4, aug, lo_nonzero,
-                                                                 fixed_scale);
+                                                                 fixed_scale, min_scale);
   return cudaGetLastError();
 }
 

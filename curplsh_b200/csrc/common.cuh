@@ -144,8 +144,8 @@ struct FusedItem {
   int db_step;             // database row j of this item is stored row j * db_step (>= 1)
   float db_scale_uniform;  // > 0: every database row has this FP8 scale s (db_scale is not read)
   // FP8 form with one database scale: the byte offset of the 32-byte BF16 norm
-  // tail of the FP8 rows (query rows, codes negated: [a_h a_h a_l], a = -1/s_q;
-  // database rows [b_h b_l b_h], b = -||x||^2 / (2 s)).  One K=16 BF16 MMA over
+  // tail of the FP8 rows (query rows, codes negated: [a1 a1 a2 a2 a1 a3], a = -1/s_q;
+  // database rows [b1 b2 b1 b2 b3 b1], b = -||x||^2 / (2 s)).  One K=16 BF16 MMA over
   // the tails adds ||x||^2 / (2 s_q s) to the FP8 accumulator, which then is
   // (||x||^2 - 2 q.x) / (2 s_q s): no database norm is loaded per tile.
   int fp8_tail;

@@ -185,9 +185,9 @@ bool bound_estimate_enabled();
 // database rows get [n1 n2 n3 1 1 1] after column d, query rows are stored as -2q
 // followed by [1 1 1 m1 m2 m3]; lo rows get zeros there.  kAugF8Query /
 // kAugF8Database write the FP8 rows' BF16 norm tail (see fp8_tail_offset):
-// query rows (codes stored negated) [a_h a_h a_l] with a = -1/s_q (s_q at least min_scale), database
-// rows [b_h b_l b_h] with b = -||x||^2 / (2 fixed_scale) (zeros without a
-// fixed scale).
+// query rows (codes stored negated) [a1 a1 a2 a2 a1 a3] with a = -1/s_q = a1 + a2 + a3 (s_q
+// at least min_scale), database rows [b1 b2 b1 b2 b3 b1] with b = -||x||^2 /
+// (2 fixed_scale) (zeros without a fixed scale).
 enum AugMode : int { kAugNone = 0, kAugDatabase = 1, kAugQuery = 2, kAugF8Query = 3, kAugF8Database = 4 };
 // Byte offset of the FP8 rows' 32-byte BF16 norm tail, round_up(d, 32): inside
 // the last 128-byte K chunk, or a narrow chunk of its own when that is full.

@@ -176,8 +176,11 @@ __device__ __forceinline__ bool prep_row(const float* __restrict__ x, long long 
       }
   }
   if (f8 && (aug == kAugF8Query || aug == kAugF8Database)) {
-    // the BF16 norm tail at byte t8 (a 32-byte K step of the last 128-byte
-    // chunk): a_h b_h + a_h b_l + a_l b_h = a b to ~2^-16 relative
+    // The BF16 norm tail at byte t8, a K step of 16 columns.  a and b are three
+    // BF16 terms each (all 24 bits), and six columns hold the products above
+    // 2^-24: a1 b1 + a1 b2 + a2 b1 + a2 b2 + a1 b3 + a3 b1.  A K step costs the
+    // same with six columns as with the three of a two-term split, which kept
+    // 16 bits of the norm.
     const long long t8 = fp8_tail_offset(d, ld8);
     if (t8 > 0) {
       __syncwarp();  // after the zero fill above, which covers these bytes
@@ -186,13 +189,11 @@ __device__ __forceinline__ bool prep_row(const float* __restrict__ x, long long 
         v = inv;  // -1 / s_q
       else if (fixed_scale > 0.f)
         v = -0.5f * s / fixed_scale;  // -||x||^2 / (2 s)
-      const float vh = __bfloat162float(__float2bfloat16_rn(v));
-      const float vl = v - vh;  // exact
-      float e = 0.f;
-      if (aug == kAugF8Query)
-        e = lane < 2 ? vh : (lane == 2 ? vl : 0.f);
-      else
-        e = lane == 1 ? vl : (lane == 0 || lane == 2 ? vh : 0.f);
+      const float t1 = __bfloat162float(__float2bfloat16_rn(v));
+      const float r1 = v - t1;  // exact, as is r1 - t2
+      const float t2 = __bfloat162float(__float2bfloat16_rn(r1));
+      const int term = ((aug == kAugF8Query ? 0x201100 : 0x021010) >> (4 * (lane & 7))) & 15;
+      const float e = lane >= 6 ? 0.f : term == 0 ? t1 : term == 1 ? t2 : r1 - t2;
       if (lane < 16) reinterpret_cast<__nv_bfloat16*>(f8 + r * ld8 + t8)[lane] = __float2bfloat16_rn(e);
     }
   }

@@ -86,3 +86,33 @@ def test_rows_at_the_ends_of_the_range(env, d, scale):
     for entry, (dist, idx) in _every_entry(env, base, queries, 10).items():
         assert (idx >= 0).all(), entry
         assert_knn_matches(base, queries, dist, idx, rd, ri)
+
+
+# Rows whose codes are exact, with norms around 8e5 that differ by a few units
+# (2^-18 of them): 16 bits of a norm hold 4 units of half of it, so all rows would
+# tie and the lowest rows -- not the nearest, which come last -- be taken as the
+# 480 candidates.  The distances of the 10 nearest are at most 1.5 and those of the
+# other rows at least 2.5, and FP32 resolves 0.06 there.  `top` 448 and 300: a
+# query scale of one, and one whose reciprocal is no short binary fraction.
+@pytest.mark.parametrize("d", [128, 256])
+@pytest.mark.parametrize("top", [448.0, 300.0])
+def test_norms_keep_fp32_bits(env, d, top):
+    cb, torch, res = env
+    n, k = 2000, 10
+    rng = np.random.default_rng(d)
+    row = np.zeros(d, np.float32)
+    row[:4] = 448.0
+    row[4:8] = 40.0, 13.0, 4.0, 2.0  # half of the norm is 401,408 + 894.5
+    base = np.tile(row, (n, 1))
+    far = np.array([[1.5, 0.5, 0, 0], [1.5, 0.5, 0.5, 0], [1, 1, 0.5, 0.5], [1.5, 1, 0, 0], [2, 0.5, 0, 0]], np.float32)
+    near = np.array([[0.5, 0, 0, 0], [0.5, 0.5, 0, 0], [1, 0, 0, 0], [1, 0.5, 0, 0], [1, 0.5, 0.5, 0]], np.float32)
+    base[:, d - 4:] = far[rng.integers(0, 5, n)]
+    base[n - k:, d - 4:] = np.repeat(near, 2, axis=0)
+    queries = np.tile(row * np.float32(top / 448.0), (3, 1))
+    rd, ri = oracle.knn(base, queries, k)
+    cb.set_coarse_check(False)
+    out = _every_entry(env, base, queries, k)
+    cb.set_coarse_check(True)
+    for entry, (_, idx) in out.items():
+        np.testing.assert_array_equal(np.sort(idx, axis=1), np.tile(np.arange(n - k, n), (3, 1)), err_msg=entry)
+    assert (np.sort(ri, axis=1) == np.arange(n - k, n)).all()

@@ -721,6 +721,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       const int S = OWN ? 1 : pool_sync_tiles(P, p.kprime);
       if (u_ord < 0 || u_ord >= U) {  // identical in every epilogue warp: both of a pair leave here
         raise_abort(abort_flag, B.status, kErrBadSchedule);
+        ok = false;
         break;
       }
       const int qbw = DUAL ? qb + g : qb;  // this warp's query block
@@ -1022,6 +1023,23 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
         if (gap) p.pool_counts[list_of(row) - kLists] = 0;
       }
       if constexpr (!OWN) bar_sync_named(pair_bar, kGroupThreads);  // the counts are read before the next unit resets them
+    }
+    // After an abort the lists of the current unit and of those not reached are
+    // written as empty: the merge still runs, and the workspace's memory may have
+    // held anything before.
+    if constexpr (!MINIMA) {
+      if (!ok) {
+        do {
+          const FusedItem& p = A.items[MAXI == 1 ? 0 : ii];
+          const int U = p.units_per_block;
+          const long long q = (long long)(DUAL ? qb + g : qb) * kBM + row;
+          if (u_ord >= 0 && u_ord < U && q < p.nq && (OWN || g == 0)) {
+            const size_t l = ((size_t)q * U + (size_t)u_ord) * kLists + (kLists > 1 ? g : 0);
+            p.pool_counts[l] = 0;
+            if (gap) p.pool_counts[l - kLists] = 0;
+          }
+        } while (walk.next(A, ii, qb, t0, t1, u_ord, gap, rot));
+      }
     }
     if (lane == 0) {
       STAT_FLUSH(kStatEpiWaitAccFull, st_wait);

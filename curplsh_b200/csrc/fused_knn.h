@@ -239,6 +239,10 @@ cudaError_t launch_prep_segments(PrepSegment* segs, int n, int d, long long ld16
 // Plain squared (or not) L2 norms, as computeL2Norm.
 cudaError_t launch_l2_norms(const float* x, long long n, int d, float* norms, int squared, cudaStream_t st);
 
+// Whether a candidate list's length is one the fused pass writes.  The merge
+// reads no key of any other list: the lengths are sums and bounds of its reads.
+__host__ __device__ inline bool pool_count_valid(int count, int cap) { return count >= 0 && count <= cap; }
+
 // Checks of the merge pass that list a query for a search again (MergeItem::checks).
 constexpr int kCheckEstimate = 1;  // the fused pass started from estimated bounds: verify them
 constexpr int kCheckCoarse = 2;    // coarse (BF16/FP8) distances: verify the candidate margin

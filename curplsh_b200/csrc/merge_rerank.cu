@@ -177,7 +177,10 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   int total = 0;
   for (int l0 = 0; l0 < nlists; l0 += NT) {
     const int l = l0 + tid;
-    const uint32_t c = l < nlists ? (uint32_t)m.pool_counts[list0 + l] : 0u;
+    const int written = l < nlists ? m.pool_counts[list0 + l] : 0;
+    const bool valid = pool_count_valid(written, m.pool_cap);
+    if (!valid) atomicOr(a.status, kErrBadSchedule);
+    const uint32_t c = valid ? (uint32_t)written : 0u;
     const uint32_t incl = block_incl_scan(c, warp_tot);
     if (l < nlists) loff[l] = total + (int)(incl - c);
     if (tid == NT - 1) misc[1] = incl;

@@ -581,11 +581,12 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       STAT_DECL(st_full);
       STAT_DECL(st_acc);
       while (ok && walk.next(A, ii, qb, t0, t1, u_ord, gap, rot)) {
+        // The lanes wait one by one and may disagree at a time-out or an abort;
+        // the vote at the end of every chunk makes them leave together (a lane
+        // that left alone would strand the others at their next warp barrier).
+        bool got = true;
         if (!L.a_stream) {
-          if (!wait_or_abort(a_full, unit & 1, abort_flag)) {
-            raise_abort(abort_flag, B.status, kErrWaitTimeout);
-            break;
-          }
+          got = wait_or_abort(a_full, unit & 1, abort_flag);
           tc_fence_after();
         }
         // The norm columns' K step (hi x hi alone carries them: lo rows are zero
@@ -604,28 +605,20 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
         for (int t = t0; t < t1 && ok; ++t, ++tc) {
           const uint32_t slot = tc & 1u, use = tc >> 1;
           STAT_BEGIN(ta);
-          if (!wait_or_abort(&acc_empty[slot], (use & 1u) ^ 1u, abort_flag, pair)) {
-            raise_abort(abort_flag, B.status, kErrWaitTimeout);
-            ok = false;
-            break;
-          }
+          got = got && wait_or_abort(&acc_empty[slot], (use & 1u) ^ 1u, abort_flag, pair);
           STAT_END(ta, st_acc);
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + slot * kBN;
           uint32_t a_lo = a_first;
           for (int kc = 0; kc < nreg; ++kc) {
             STAT_BEGIN(tf);
-            if (!wait_or_abort(&full[s], sphase, abort_flag)) {
-              raise_abort(abort_flag, B.status, kErrWaitTimeout);
-              ok = false;
-              break;
-            }
+            got = got && wait_or_abort(&full[s], sphase, abort_flag);
             STAT_END(tf, st_full);
             tc_fence_after();
             if (L.a_stream) a_lo = b_lo + a_in_stage;
             const bool last = kc == nreg - 1;
             const int n = last ? last_steps : kSteps;
-            if (leader) {
+            if (leader && got) {
 #pragma unroll
               for (int j = 0; j < kQB; ++j) {  // dual: block j accumulates into columns j * 128 of the slot
                 const uint32_t dj = d_tmem + (uint32_t)j * (kBN / 2);
@@ -640,7 +633,11 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
               commit(&empty[s]);
               if (last) commit(&acc_full[slot]);
             }
-            __syncwarp();
+            if (__any_sync(0xffffffffu, !got)) {
+              if (!got) raise_abort(abort_flag, B.status, kErrWaitTimeout);
+              ok = false;
+              break;
+            }
             a_lo += Tr::kAParts * kA16;
             b_lo += stage16;
             if (++s == S) {
@@ -659,6 +656,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       if (leader) commit(drain);
       __syncwarp();
       mbar_wait(drain, 0);
+      __syncwarp();
       if (lane == 0) {
         STAT_FLUSH(kStatMmaWaitFull, st_full);
         STAT_FLUSH(kStatMmaWaitAccEmpty, st_acc);
@@ -858,7 +856,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
           }
         }
         STAT_BEGIN(tw);
-        const bool got = wait_or_abort(&acc_full[slot], use & 1u, abort_flag);
+        // the same for the whole warp: what follows is warp-wide
+        const bool got = __all_sync(0xffffffffu, wait_or_abort(&acc_full[slot], use & 1u, abort_flag));
         if (!got) raise_abort(abort_flag, B.status, kErrWaitTimeout);
         STAT_END(tw, st_wait);
         // an aborting warp skips the tile but still meets its partner below

@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       UnitWalk walk(blockIdx.x, B, rank);
       int ii, qb, t0, t1, u_ord, rot, unit = 0;
       bool gap;
-      uint32_t it = 0;
+      uint32_t it = 0, q_loads = 0;  // stages and query blocks loaded
       bool ok = true;
       STAT_DECL(st_wait);
       while (ok && walk.next(A, ii, qb, t0, t1, u_ord, gap, rot)) {
@@ -474,6 +474,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
             break;
           }
           const int nreg = L.nkc - (L.tail_narrow ? 1 : 0);
+          ++q_loads;
           if (issuer)
             mbar_arrive_expect_tx(a_full, tx_mul * (uint32_t)kQB *
                                               ((uint32_t)nreg * Tr::kAParts * kAChunkBytes +
@@ -521,6 +522,15 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
           }
         }
         ++unit;
+      }
+      // After an abort nobody consumes the last loads, so this role waits for
+      // their bytes itself (a pair's complete on rank 0's barriers): the shared
+      // memory must not change hands under a copy.  Otherwise it has nothing
+      // else to do until the MMAs are through.
+      if (issuer) {
+        bool landed = q_loads == 0 || mbar_wait(a_full, (q_loads - 1) & 1u);
+        for (uint32_t i = it > (uint32_t)S ? it - (uint32_t)S : 0u; landed && i < it; ++i)
+          landed = mbar_wait(&full[i % (uint32_t)S], (i / (uint32_t)S) & 1u);
       }
       STAT_FLUSH(kStatProducerWaitEmpty, st_wait);
     }

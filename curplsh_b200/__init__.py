@@ -145,6 +145,8 @@ def _load():
         "curplsh_index_get_fallback_count": (i32, [vp, ctypes.POINTER(ctypes.c_int64)]),
         "curplsh_estimate_plan_shape": (i32, [i64, i64, i32, i32, ctypes.POINTER(ctypes.c_int),
                                               ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
+        "curplsh_index_estimate_sample": (i32, [vp, i64, i32, i32, i32] + [ctypes.POINTER(ctypes.c_int)] * 4),
+        "curplsh_estimate_sample_shape": (i32, [i64, i64, i32, i32] + [ctypes.POINTER(ctypes.c_int)] * 4),
     }
     for name, (res, args) in sig.items():
         fn = getattr(lib, name)
@@ -173,6 +175,7 @@ EXPORTED_SYMBOLS = (
     "curplsh_index_get_fallback_count", "curplsh_estimate_plan_shape", "curplsh_set_coarse_check",
     "curplsh_get_coarse_check", "curplsh_index_get_coarse_fallback_count", "curplsh_set_cta_pairs",
     "curplsh_get_cta_pairs", "curplsh_set_dual_blocks", "curplsh_get_dual_blocks",
+    "curplsh_index_estimate_sample", "curplsh_estimate_sample_shape",
 )
 
 
@@ -381,14 +384,23 @@ class IndexBF:
         return self._res
 
     def estimate_plan(self, num_queries: int, k: int, precision: int = -1, rerank_factor: int = -1):
-        """(sample_rows, step, rank) of the sampled bound estimate a search of this
-        shape would use (rank among the sample_rows / 128 block minima);
-        sample_rows == 0 when it uses none."""
+        """(sample_rows, step, rank) of the regular sampled bound estimate a search of
+        this shape would use (rank among the sample_rows / 128 block minima);
+        sample_rows == 0 when it uses none or a light one (estimate_sample)."""
         a, b, c = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
         _check(_lib.curplsh_index_estimate_plan(self._h, int(num_queries), int(k), int(precision),
                                                 int(rerank_factor), ctypes.byref(a), ctypes.byref(b),
                                                 ctypes.byref(c)))
         return a.value, b.value, c.value
+
+    def estimate_sample(self, num_queries: int, k: int, precision: int = -1, rerank_factor: int = -1):
+        """(sample_rows, step, block_rows, rank) of the estimate a search of this shape
+        starts from, regular or light (rank among the sample_rows / block_rows block
+        minima); sample_rows == 0 when it uses none."""
+        v = [ctypes.c_int(0) for _ in range(4)]
+        _check(_lib.curplsh_index_estimate_sample(self._h, int(num_queries), int(k), int(precision),
+                                                  int(rerank_factor), *map(ctypes.byref, v)))
+        return tuple(x.value for x in v)
 
     def fallback_count(self) -> int:
         """Queries searched again after their estimated bound failed (since creation)."""
@@ -517,13 +529,22 @@ def set_bound_estimate(enabled: bool) -> None:
 
 
 def estimate_plan_shape(num_rows: int, num_queries: int, kprime: int, num_sms: int = 148):
-    """(sample_rows, step, rank) of the sampled bound estimate for a bare search shape
-    (no index or device needed); sample_rows == 0 when that shape uses none, or only the
-    light sample of a small k'."""
+    """(sample_rows, step, rank) of the regular sampled bound estimate for a bare search
+    shape (no index or device needed); sample_rows == 0 when that shape uses none or a
+    light one (estimate_sample_shape)."""
     a, b, c = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
     _check(_lib.curplsh_estimate_plan_shape(int(num_rows), int(num_queries), int(kprime), int(num_sms),
                                             ctypes.byref(a), ctypes.byref(b), ctypes.byref(c)))
     return a.value, b.value, c.value
+
+
+def estimate_sample_shape(num_rows: int, num_queries: int, kprime: int, num_sms: int = 148):
+    """(sample_rows, step, block_rows, rank) of the estimate, regular or light, of a bare
+    search shape; sample_rows == 0 when it uses none."""
+    v = [ctypes.c_int(0) for _ in range(4)]
+    _check(_lib.curplsh_estimate_sample_shape(int(num_rows), int(num_queries), int(kprime), int(num_sms),
+                                              *map(ctypes.byref, v)))
+    return tuple(x.value for x in v)
 
 
 def get_bound_estimate() -> bool:

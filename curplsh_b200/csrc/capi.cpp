@@ -1472,45 +1472,79 @@ int curplsh_get_dual_blocks(int* enabled) {
   return CURPLSH_OK;
 }
 
-int curplsh_index_estimate_plan(curplsh_index* ix, int64_t num, int k, int precision, int rerank_factor,
-                                int* sample_rows, int* step, int* rank) {
-  if (!ix || !sample_rows || !step || !rank) return set_error(CURPLSH_ERR_INVALID_ARG, "null argument");
+// The plan of the estimate a search of this shape uses (on == false: none).
+static int index_estimate(curplsh_index* ix, int64_t num, int k, int precision, int rerank_factor, EstimatePlan* out) {
+  *out = EstimatePlan();
   if (k < 1 || k > 1024 || num < 0 || num > (int64_t)1 << 30)
     return set_error(CURPLSH_ERR_INVALID_ARG, "bad k or number of queries");
   const int form = precision < 0 ? ix->cfg.precision : precision;
   if (form < 0 || form > 2) return set_error(CURPLSH_ERR_INVALID_ARG, "unknown precision %d", precision);
   const int rf = rerank_factor > 0 ? rerank_factor : ix->cfg.rerank_factor;
   std::shared_lock<std::shared_mutex> lk(ix->mu);
-  *sample_rows = 0;
-  *step = 1;
-  *rank = 0;
   if (ix->n == 0 || !g_bound_estimate.load(std::memory_order_relaxed)) return CURPLSH_OK;
   const bool coarse_on = g_coarse_check.load(std::memory_order_relaxed) != 0;
-  const EstimatePlan e = plan_estimate((int)num, ix->n, kprime_for(form, k, rf, ix->n, coarse_on), ix->dres->num_sms);
-  if (e.on && !e.light) {
-    *sample_rows = e.rows;
-    *step = e.step;
-    *rank = e.j;
-  }
+  *out = plan_estimate((int)num, ix->n, kprime_for(form, k, rf, ix->n, coarse_on), ix->dres->num_sms);
   return CURPLSH_OK;
+}
+
+static int shape_estimate(int64_t num_rows, int64_t num_queries, int kprime, int num_sms, EstimatePlan* out) {
+  if (num_rows < 0 || num_rows > INT32_MAX || num_queries < 0 || num_queries > (int64_t)1 << 30 || kprime < 0 ||
+      num_sms < 1)
+    return set_error(CURPLSH_ERR_INVALID_ARG, "bad shape");
+  *out = plan_estimate((int)num_queries, num_rows, kprime, num_sms);
+  return CURPLSH_OK;
+}
+
+// What the plan calls report: the regular samples.
+static void put_plan(const EstimatePlan& e, int* sample_rows, int* step, int* rank) {
+  const bool on = e.on && !e.light;
+  *sample_rows = on ? e.rows : 0;
+  *step = on ? e.step : 1;
+  *rank = on ? e.j : 0;
+}
+
+// What the sample calls report: every sample.
+static void put_sample(const EstimatePlan& e, int* sample_rows, int* step, int* block_rows, int* rank) {
+  *sample_rows = e.on ? e.rows : 0;
+  *step = e.on ? e.step : 1;
+  *block_rows = e.on ? e.block_rows : 0;
+  *rank = e.on ? e.j : 0;
+}
+
+int curplsh_index_estimate_plan(curplsh_index* ix, int64_t num, int k, int precision, int rerank_factor,
+                                int* sample_rows, int* step, int* rank) {
+  if (!ix || !sample_rows || !step || !rank) return set_error(CURPLSH_ERR_INVALID_ARG, "null argument");
+  EstimatePlan e;
+  int rc = index_estimate(ix, num, k, precision, rerank_factor, &e);
+  if (!rc) put_plan(e, sample_rows, step, rank);
+  return rc;
 }
 
 int curplsh_estimate_plan_shape(int64_t num_rows, int64_t num_queries, int kprime, int num_sms, int* sample_rows,
                                 int* step, int* rank) {
   if (!sample_rows || !step || !rank) return set_error(CURPLSH_ERR_INVALID_ARG, "null argument");
-  if (num_rows < 0 || num_rows > INT32_MAX || num_queries < 0 || num_queries > (int64_t)1 << 30 || kprime < 0 ||
-      num_sms < 1)
-    return set_error(CURPLSH_ERR_INVALID_ARG, "bad shape");
-  *sample_rows = 0;
-  *step = 1;
-  *rank = 0;
-  const EstimatePlan e = plan_estimate((int)num_queries, num_rows, kprime, num_sms);
-  if (e.on && !e.light) {
-    *sample_rows = e.rows;
-    *step = e.step;
-    *rank = e.j;
-  }
-  return CURPLSH_OK;
+  EstimatePlan e;
+  int rc = shape_estimate(num_rows, num_queries, kprime, num_sms, &e);
+  if (!rc) put_plan(e, sample_rows, step, rank);
+  return rc;
+}
+
+int curplsh_index_estimate_sample(curplsh_index* ix, int64_t num, int k, int precision, int rerank_factor,
+                                  int* sample_rows, int* step, int* block_rows, int* rank) {
+  if (!ix || !sample_rows || !step || !block_rows || !rank) return set_error(CURPLSH_ERR_INVALID_ARG, "null argument");
+  EstimatePlan e;
+  int rc = index_estimate(ix, num, k, precision, rerank_factor, &e);
+  if (!rc) put_sample(e, sample_rows, step, block_rows, rank);
+  return rc;
+}
+
+int curplsh_estimate_sample_shape(int64_t num_rows, int64_t num_queries, int kprime, int num_sms, int* sample_rows,
+                                  int* step, int* block_rows, int* rank) {
+  if (!sample_rows || !step || !block_rows || !rank) return set_error(CURPLSH_ERR_INVALID_ARG, "null argument");
+  EstimatePlan e;
+  int rc = shape_estimate(num_rows, num_queries, kprime, num_sms, &e);
+  if (!rc) put_sample(e, sample_rows, step, block_rows, rank);
+  return rc;
 }
 
 int curplsh_index_get_fallback_count(curplsh_index* ix, int64_t* count) {

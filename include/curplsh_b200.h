@@ -299,10 +299,12 @@ int curplsh_tuning_clear(void);
  * and the call returns synchronised.  The switch is process-wide; on (1) by default. */
 int curplsh_set_bound_estimate(int enabled);
 int curplsh_get_bound_estimate(int* enabled);
-/* The estimate a search of num_queries queries with this k / precision / rerank factor would
- * use: the sample size, its row step and the rank j among the sample_rows / 128 block minima;
- * *sample_rows = 0 when it uses none, or only the light sample of a small k' (fewer than 8
- * expected rows among the k' nearest). */
+/* The regular estimate a search of num_queries queries with this k / precision / rerank factor
+ * would use: the sample size, its row step and the rank j among the sample_rows / 128 block
+ * minima; *sample_rows = 0 when it uses none or a light one (curplsh_index_estimate_sample).  A
+ * regular sample has 8 to 12 expected rows among the k' nearest and at most a tenth of the
+ * database, of 65,536 rows or more; searches for which no such sample holds a rank use a light
+ * one, sized by its cost. */
 int curplsh_index_estimate_plan(curplsh_index* index, int64_t num_queries, int k, int precision,
                                 int rerank_factor, int* sample_rows, int* step, int* rank);
 /* The same plan for a bare shape (N rows, num_queries queries, k' candidates, num_sms SMs),
@@ -310,6 +312,13 @@ int curplsh_index_estimate_plan(curplsh_index* index, int64_t num_queries, int k
  * on. */
 int curplsh_estimate_plan_shape(int64_t num_rows, int64_t num_queries, int kprime, int num_sms, int* sample_rows,
                                 int* step, int* rank);
+/* The estimate such a search starts from, regular or light: *rank is that among the
+ * sample_rows / block_rows block minima, and *sample_rows = 0 means that it uses none.  Sample
+ * row i is database row i * step. */
+int curplsh_index_estimate_sample(curplsh_index* index, int64_t num_queries, int k, int precision,
+                                  int rerank_factor, int* sample_rows, int* step, int* block_rows, int* rank);
+int curplsh_estimate_sample_shape(int64_t num_rows, int64_t num_queries, int kprime, int num_sms, int* sample_rows,
+                                  int* step, int* block_rows, int* rank);
 /* Number of queries this index searched again after their estimate failed (since creation). */
 int curplsh_index_get_fallback_count(curplsh_index* index, int64_t* count);
 

@@ -1,0 +1,51 @@
+"""GPU: samples of rows that were added in some order.  A light sample must hold
+its rank when a query's neighbours all lie in one part of the rows: the search
+answers as without a sample, and (almost) no query is searched again.  Run with
+-m gpu on a B200."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def env():
+    import torch
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    import curplsh_b200 as cb
+    res = cb.DeviceResources(0)
+    yield cb, res
+    cb.set_bound_estimate(True)
+    res.close()
+
+
+def _check(env, base, queries, k):
+    """Results with and without a sample are equal and no query fails its estimate
+    (the rank's failure probability is at most 1e-6 a query)."""
+    cb, res = env
+    n, d = base.shape
+    ix = cb.IndexBF(res, d, cb.IndexBFConfig(precision=0))
+    ix.add(n, base)
+    assert ix.estimate_plan(len(queries), k)[0] == 0 and ix.estimate_sample(len(queries), k)[0] > 0
+    d1, i1 = ix.search_array(queries, k)
+    failed = ix.fallback_count()
+    cb.set_bound_estimate(False)
+    d0, i0 = ix.search_array(queries, k)
+    cb.set_bound_estimate(True)
+    ix.close()
+    np.testing.assert_array_equal(i1, i0)
+    np.testing.assert_array_equal(d1, d0)
+    assert failed == 0
+
+
+# (rows, queries, k): sample blocks of 8 and of 128 rows, whose step used to be 1 and 3
+SHAPES = [(30_000, 1000, 100), (300_000, 200, 1024), (100_000, 100, 10)]
+
+
+@pytest.mark.parametrize("n,nq,k", SHAPES)
+@pytest.mark.parametrize("first", [0.3, 0.5, 0.75, 1.0])
+def test_two_sets_added_one_after_the_other(env, n, nq, k, first):
+    rng = np.random.default_rng(n)
+    base = rng.random((n, 48), dtype=np.float32)
+    base[int(n * first):] += 3.0
+    _check(env, base, rng.random((nq, 48), dtype=np.float32), k)

@@ -839,6 +839,7 @@ int search_device(curplsh_index* ix, const SearchShape& sh, int nq, const float*
     e.nb = sh.est.rows;
     e.nb_pad = sh.est.rows;
     e.db_step = sh.est.step;
+    e.db_phased = sh.est.light;
     e.kprime = 1;
     e.minima = b.minima;
     e.minima_rows = sh.est.block_rows;

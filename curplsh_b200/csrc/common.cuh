@@ -141,7 +141,9 @@ struct FusedItem {
   uint64_t* pools;         // [G_i*128][U_i][pool_cap]
   int* pool_counts;        // [G_i*128][U_i]
   uint32_t* q_bound;       // [nq_pad] shared per-query bound (ordered bits), init kOrdInf or an estimate
-  int db_step;             // database row j of this item is stored row j * db_step (>= 1)
+  // Database row j of this item is stored row j * db_step (>= 1; > 1 in
+  // block-minimum mode only), plus sample_phase(j / 256, db_step) when db_phased.
+  int db_step, db_phased;
   float db_scale_uniform;  // > 0: every database row has this FP8 scale s (db_scale is not read)
   // FP8 form with one database scale: the byte offset of the 32-byte BF16 norm
   // tail of the FP8 rows (query rows, codes negated: [a1 a1 a2 a2 a1 a3], a = -1/s_q;
@@ -155,6 +157,13 @@ struct FusedItem {
   float* minima;
   int minima_rows;         // 128 or 8
 };
+
+// Which of the db_step rows after its first each row of a phased sample's tile is:
+// the fractions t * (sqrt(5) - 1) / 2 mod 1 spread the tiles evenly over them, so
+// rows stored with a period that divides the step are sampled alike.
+__host__ __device__ inline int sample_phase(int tile, int step) {
+  return (int)(((unsigned long long)((uint32_t)tile * 2654435769u) * (uint32_t)step) >> 32);
+}
 
 // Tensor maps of one item, in this order.
 enum FusedMap : int { kMapQHi = 0, kMapQLo, kMapXHi, kMapXLo, kMapQTail, kMapXTail, kMapsPerItem };

@@ -61,6 +61,7 @@ struct FusedLaunch {
   float xs_uniform = 0.f;   // > 0: one FP8 scale for every database row
   // database row j of this pass is stored row j * db_step (a strided sample when > 1)
   int db_step = 1;
+  int db_phased = 0;  // FusedItem::db_phased
   // non-null: block-minimum mode, see FusedItem::minima (pools are not used)
   float* minima = nullptr;
   int minima_rows = 128;
@@ -112,6 +113,7 @@ struct FusedItemSpec {
   int* pool_counts;         // [G*128][U]
   uint32_t* q_bound;        // [nq_pad], initialised to all ones (or to estimated bounds)
   int db_step;              // database row j is stored row j * db_step (0 or 1: contiguous)
+  int db_phased;            // FusedItem::db_phased
   float* minima;            // non-null: block-minimum mode (FusedItem::minima)
   int minima_rows;          // its block rows: 128 or 8
 };
@@ -160,7 +162,7 @@ struct EstimatePlan {
   bool on = false;
   bool light = false;  // sized by cost, not by expected rows (see capi.cpp)
   int rows = 0;    // sample rows (a multiple of 256)
-  int step = 1;    // sample row j is database row j * step
+  int step = 1;    // sample row j is database row j * step, plus, in a light sample, its tile's sample_phase
   int block_rows = 128;  // or 8
   int blocks = 0;  // B = rows / block_rows block minima per query
   int j = 0;       // rank of the estimate among the block minima

@@ -49,3 +49,35 @@ def test_two_sets_added_one_after_the_other(env, n, nq, k, first):
     base = rng.random((n, 48), dtype=np.float32)
     base[int(n * first):] += 3.0
     _check(env, base, rng.random((nq, 48), dtype=np.float32), k)
+
+
+# periods that divide the old steps (2, 3, 4) and some that do not; the FP8 forms of
+# one scale and of a scale per row read norms and scales at the sampled rows too
+@pytest.mark.parametrize("n,nq,k", SHAPES)
+@pytest.mark.parametrize("period", [2, 3, 4, 10])
+def test_rows_interleaved_with_a_period(env, n, nq, k, period):
+    rng = np.random.default_rng(n + period)
+    base = rng.random((n, 48), dtype=np.float32) + np.float32(3.0) * (np.arange(n) % period)[:, None].astype(np.float32)
+    _check(env, base, rng.random((nq, 48), dtype=np.float32), k)
+
+
+@pytest.mark.parametrize("form,spread", [(0, 1.0), (1, 1.0), (2, 1.0), (2, 1000.0)])
+@pytest.mark.parametrize("n,nq,k", [(2048, 600, 20), (20_011, 70, 50)])
+def test_forms_agree_with_and_without_a_light_sample(env, form, spread, n, nq, k):
+    cb, res = env
+    rng = np.random.default_rng(n + form)
+    base = rng.standard_normal((n, 72)).astype(np.float32)
+    base[rng.random(n) < 0.5] *= np.float32(spread)
+    queries = base[rng.choice(n, nq)] + rng.normal(0.0, 0.1, (nq, 72)).astype(np.float32)
+    ix = cb.IndexBF(res, 72, cb.IndexBFConfig(precision=form, rerankFactor=6 if form else 0))
+    ix.add(n, base)
+    assert ix.estimate_plan(nq, k)[0] == 0 and ix.estimate_sample(nq, k)[0] > 0
+    d1, i1 = ix.search_array(queries.astype(np.float32), k)
+    failed = ix.fallback_count()
+    cb.set_bound_estimate(False)
+    d0, i0 = ix.search_array(queries.astype(np.float32), k)
+    cb.set_bound_estimate(True)
+    ix.close()
+    np.testing.assert_array_equal(i1, i0)
+    np.testing.assert_array_equal(d1, d0)
+    assert failed == 0

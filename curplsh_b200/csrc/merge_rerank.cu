@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   // smallest k'-th of any pool, or the estimate the pass started from.  When
   // it comes from a pool, every key of the k' smallest has a distance <= it.
   uint32_t qbound = 0xFFFFFFFFu;
-  if (m.q_bound && T > 0) qbound = m.q_bound[prow];
+  if (m.q_bound && T > 0 && a.pre_cap > 0) qbound = m.q_bound[prow];
 
   for (int i = tid; i < d; i += NT) qv[i] = m.queries[(size_t)q * d + i];
   if (tid == 0) {
@@ -169,11 +169,13 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
     misc[6] = 0xFFFFFFFFu;   // min of the same
     misc[7] = 0u;            // largest coarse distance among the candidates, order bits
   }
-  // The lists are read as one flattened sequence (list of key i by binary
-  // search in the offsets), four loads in flight per thread: list by list, each
-  // of the up to 148 short lists of a few-query search was a load latency of
-  // its own (merge of 16 queries against 2 x 10^6 rows 164 -> 23 us, of one
-  // query against 10^4 rows 56 -> 19, of 1,000 queries with k = 1,024 312 -> 212).
+  // The lists are read as one flattened sequence, four loads in flight per thread:
+  // list by list, each of the up to 148 short lists of a few-query search was a
+  // load latency of its own (merge of 16 queries against 2 x 10^6 rows 164 -> 23
+  // us, of one query against 10^4 rows 56 -> 19, of 1,000 queries with k = 1,024
+  // 312 -> 212).  A thread's list only moves forward; with a binary search per key
+  // long lists took three times as long (k' = 1,024, 10^6 rows, one query without a
+  // bound: 3.47 -> 1.20 ms, 1.76 list by list).
   int total = 0;
   for (int l0 = 0; l0 < nlists; l0 += NT) {
     const int l = l0 + tid;
@@ -194,6 +196,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   // f(key, on) for this thread's share of the keys, called by whole warps (on =
   // false past the end and for keys above the final bound)
   auto each_pool_key = [&](auto f) {
+    int l = 0, lo = 0, hi = loff[nlists > 0 ? 1 : 0];  // list l holds the keys [lo, hi); it only moves forward
     for (int i0 = tid; i0 - tid < total; i0 += kLoads * NT) {
       uint64_t key[kLoads];
 #pragma unroll
@@ -201,15 +204,11 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
         const int i = i0 + u * NT;
         key[u] = kKeyEmpty;
         if (i < total) {
-          int l = 0, h = nlists;  // loff[l] <= i < loff[h]
-          while (h - l > 1) {
-            const int mid = (l + h) >> 1;
-            if (loff[mid] <= i)
-              l = mid;
-            else
-              h = mid;
+          while (i >= hi) {
+            lo = hi;
+            hi = loff[++l + 1];
           }
-          key[u] = m.pools[(list0 + (size_t)l) * (size_t)m.pool_cap + (size_t)(i - loff[l])];
+          key[u] = m.pools[(list0 + (size_t)l) * (size_t)m.pool_cap + (size_t)(i - lo)];
         }
       }
 #pragma unroll
@@ -226,10 +225,14 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
     if (on && pos < (uint32_t)cap) buf[pos] = key;
   };
 
-  // ---- 1. keys under the final bound, compacted into shared memory
-  each_pool_key([&](uint64_t key, bool on) { append(key, on, pre, a.pre_cap, &misc[0]); });
-  __syncthreads();
-  const int cnt = (int)misc[0];
+  // ---- 1. keys under the final bound, compacted into shared memory (when this
+  // launch has room for them)
+  int cnt = total;
+  if (a.pre_cap > 0) {
+    each_pool_key([&](uint64_t key, bool on) { append(key, on, pre, a.pre_cap, &misc[0]); });
+    __syncthreads();
+    cnt = (int)misc[0];
+  }
   // Started from an estimate E: every row with a key under E was admitted, so
   // k' keys under the final bound (<= E) prove that the k' smallest keys of
   // the whole database are among the candidates (their k'-th is then <= E, and
@@ -461,10 +464,25 @@ cudaError_t launch_merge_batch(MergeItem* items, int n, int d, uint32_t* status,
   int kp2 = 32;  // >= 32 keeps the shared-memory carve 16-byte aligned
   while (kp2 < kpmax) kp2 <<= 1;
   a.kp2 = kp2;
+  // Whether some pool can have bounded the k'-th distance: a unit covers at least
+  // k' rows, or the pools started from an estimate (whose check counts the keys
+  // under the final bound).
+  bool bounded = false;
+  long long keys = 0;  // the most that one query's lists hold
+  for (int i = 0; i < n; ++i) {
+    long long len = std::min<long long>(items[i].split_tiles, items[i].work_per_cta);
+    len = std::min<long long>(len, items[i].num_tiles);
+    bounded = bounded || (items[i].q_bound && len * kBN >= items[i].kprime) || (items[i].checks & kCheckEstimate);
+    keys = std::max(keys, std::min<long long>(items[i].nb_total,
+                                              (long long)items[i].units_per_block * items[i].lists * items[i].pool_cap));
+  }
   // Room for the keys that pass the final bound: two k', at least 1,024 (8 KB,
   // which 12 CTAs per SM still have) so that searches with small k' select from
-  // shared memory too.
-  a.pre_cap = std::max(2 * kp2, 1024);
+  // shared memory too.  Without a bound every key passes and the selection reads
+  // the lists themselves: a first pass that only found too many keys cost a search
+  // of 3,000 rows with k' = 480 a tenth, and room for all of them took residency
+  // (k' = 480, 2,048 rows, 150 queries: merge 60 us, 56 without).
+  a.pre_cap = bounded ? (int)std::min<long long>(std::max(2 * kp2, 1024), (keys + 31) / 32 * 32) : 0;
   a.lcnt_n = (umax + 1 + 3) & ~3;
   bool vec4 = d % 4 == 0;
   for (int i = 0; i < n; ++i)

@@ -699,7 +699,7 @@ SearchShape search_shape(const curplsh_index* ix, int nq, int k, int form, int r
   sh.P = pool_capacity(sh.kp, tp.headroom);
   if (allow_est) sh.est = plan_estimate(nq, ix->n, sh.kp, ix->dres->num_sms, lean);
   plan_fused(nq, (int)ix->n, ix->dres->num_sms, &sh.plan, default_split_q4(tp, sh.P), form, ix->dim,
-             lean ? kFillSingle : sh.est.on ? 0 : sh.kp);
+             sh.est.on ? 0 : sh.kp, lean);
   sh.nq_pad = round_up(nq, kBM);
   sh.pool_lists = (size_t)sh.plan.pool_rows() * sh.plan.units_per_block * sh.plan.lists_per_unit();
   sh.coarse = coarse_check_applies(ix, form, sh.kp, coarse_on);

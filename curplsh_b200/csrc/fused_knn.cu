@@ -88,6 +88,10 @@ struct FormTraits<kFormFP8Rows> : FP8Traits {
   static constexpr bool kRowScales = true;
 };
 
+// FILL: eights of a warp's 16 with survivors from which 32 columns are taken at a
+// time (one query, 100,000 rows, k' = 1,024: pass 43 -> 25 us; 6 and 9 alike).
+constexpr int kDenseEights = 6;
+
 constexpr uint32_t kAChunkBytes = kBM * kChunkBytes;  // 16 KB
 constexpr uint32_t kBChunkBytes = kBN * kChunkBytes;  // 32 KB
 // A narrow tail chunk holds the last <= 16 BF16 columns (the augmented norm
@@ -344,6 +348,13 @@ __device__ __forceinline__ float select8(const float* x, int j) {
   return (j & 1) ? b1 : b0;
 }
 
+// x[j] for a runtime j in [0, 32)
+__device__ __forceinline__ float select32(const float* x, int j) {
+  const float a = (j & 8) ? select8(x + 8, j & 7) : select8(x, j & 7);
+  const float b = (j & 8) ? select8(x + 24, j & 7) : select8(x + 16, j & 7);
+  return (j & 16) ? b : a;
+}
+
 // ------------------------------------------------------------------ kernel
 // MINIMA selects the block-minimum mode (FusedItem::minima, the sample pass of
 // the bound estimate) at compile time, so the candidate-pool kernel carries
@@ -354,9 +365,16 @@ __device__ __forceinline__ float select8(const float* x, int j) {
 // DUAL: two query blocks resident per CTA; each 128-row database tile feeds two
 // 128 x 128 MMAs (one per block), so a tile crosses L2 -> SM once per 256
 // queries without coupling CTAs; warp g of a lane group filters block g.
-template <int FORM, int MAXI, bool MINIMA = false, bool PAIR = false, bool DUAL = false>
+// FILL: pools that start without a bound (few rows, the estimate off, the
+// allocation-free call).  Most eights of a tile then hold survivors until the
+// pools' own bounds are tight, so the survivor code takes 32 columns at a time,
+// and a bound that another CTA found is worth asking for at every tile.  An
+// instance of its own: within the bounded kernel this code cost the FP8 sphere's
+// pass 1.3 %.
+template <int FORM, int MAXI, bool MINIMA = false, bool PAIR = false, bool DUAL = false, bool FILL = false>
 __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_constant__ FusedArgs<MAXI> A) {
   static_assert(!(PAIR && DUAL) && !(DUAL && MINIMA), "dual blocks: single CTAs, candidate pools");
+  static_assert(!(FILL && MINIMA), "block minima have no pools");
   using Tr = FormTraits<FORM>;
   const FusedBatch& B = A.B;
   // a conditional pass (a re-search after a failed check): every thread of
@@ -704,9 +722,12 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
     // warps meet nowhere.  CTA pairs do the same with two pools per query, one
     // per warp (kLists): an accumulator waits for both CTAs' warps, so what the
     // warps wait for each other is paid twice (FP32-exact integer mixture as
-    // pairs: full pass 5.30 -> 4.72 ms).  Block minima need no pool at all.
-    constexpr bool OWN = DUAL || PAIR || MINIMA;
-    constexpr int kLists = PAIR ? 2 : 1;
+    // pairs: full pass 5.30 -> 4.72 ms).  Pairs whose pools start without a bound
+    // share them all the same: two pools fill with twice the keys (FP32-exact, d =
+    // 256, k' = 32, 3,000 rows, 1,000 queries: pass 106 us, 281 with two).  Block
+    // minima need no pool at all.
+    constexpr bool OWN = DUAL || (PAIR && !FILL) || MINIMA;
+    constexpr int kLists = PAIR && !FILL ? 2 : 1;
     const int ew = warp - 2;       // 0..EW-1
     const int g = ew >> 2;         // this warp's index within its lane group
     const int lg = warp & 3;       // TMEM lane group this warp may access
@@ -739,6 +760,11 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       const int P = p.pool_cap;
       const int U = p.units_per_block;
       const int S = OWN ? 1 : pool_sync_tiles(P, p.kprime);
+      // At a unit's end pools above k' are selected, so that the merge reads little
+      // beyond what it needs.  Short units end with some more in every pool, and
+      // a selection of most of its keys frees nothing for its 10 us (k' = 224, 3,000
+      // rows, 1,000 queries: pass 256 us, 44 without).
+      const int end_lim = FILL ? p.kprime + p.kprime / 4 : p.kprime;
       if (u_ord < 0 || u_ord >= U) {  // identical in every epilogue warp: both of a pair leave here
         raise_abort(abort_flag, B.status, kErrBadSchedule);
         ok = false;
@@ -849,13 +875,13 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       if (tphys < 0) tphys += T_i;
       int until_sync = S;    // tiles until the pair meets
       // The shared bound is an L2 round trip and moves rarely: it is asked for
-      // at one tile and used four tiles later
+      // at one tile and used four tiles later (FILL: at the next)
       uint32_t nb_ob = kOrdInf;
       if (valid) nb_ob = ld_relaxed_u32(&p.q_bound[q]);
       for (int t = t0; t < t1; ++t, ++tc) {
         const uint32_t slot = tc & 1u, use = tc >> 1;
         if constexpr (!OWN) thr = fminf(thr, thr_s[row]);
-        if (((t - t0) & 3) == 0) {
+        if (FILL || ((t - t0) & 3) == 0) {
           if (nb_ob != kOrdInf) thr = fminf(thr, thr_from<Tr::kFolded>(ord2f(nb_ob), qn));
           if (valid) nb_ob = ld_relaxed_u32(&p.q_bound[q]);
         }
@@ -951,6 +977,47 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
           // missed the instruction caches)
           uint32_t hit = __reduce_or_sync(
               0xffffffffu, survive_mask<8>(gm, km, thr_up) | survive_mask<8>(gm + 8, km, thr_up) << 8);
+          if (FILL && __popc(hit) >= kDenseEights) {
+#pragma unroll 1
+            for (int c32 = 0; c32 < kHalfN; c32 += 32) {
+              uint32_t w[32];
+              float x[32];
+              tmem_ld_32x32b_x32(t_src + c32, w);
+              tmem_ld_wait();
+              dist_of(w, c32, x, 32);
+              const int c0 = tcol + c32;
+              uint32_t m = survive_mask<32>(x, km, thr_up);
+              if (c0 + 32 > p.nb) m &= c0 >= p.nb ? 0u : (1u << (p.nb - c0)) - 1u;
+              const int c = __popc(m);
+              int n = reserve(c);
+              STAT_INC(st_surv, c);
+              if (m == ~0u) {  // every column (no bound yet)
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                  if (n + j < P) pool[n + j] = make_key(key_d(x[j]), (uint32_t)(c0 + j));
+                m = 0u;
+              }
+              if (__any_sync(0xffffffffu, __popc(m) > 4)) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                  const bool take = (m >> j) & 1u;
+                  if (take && n < P) pool[n] = make_key(key_d(x[j]), (uint32_t)(c0 + j));
+                  n += take ? 1 : 0;
+                }
+                continue;
+              }
+#pragma unroll 1
+              while (__any_sync(0xffffffffu, m != 0u)) {
+                STAT_INC(st_iters, 1);
+                const int j = __ffs(m) - 1;  // -1: none left
+                const float xs = select32(x, j);
+                m &= m - 1u;
+                if (j >= 0 && n < P) pool[n] = make_key(key_d(xs), (uint32_t)(c0 + j));
+                ++n;
+              }
+            }
+            hit = 0u;
+          }
 #pragma unroll 1
           while (hit) {
             const int e = __ffs(hit) - 1;
@@ -1005,9 +1072,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
             break;
           }
           // pools that may not have room for the next tile, or, at the unit's
-          // end, every pool above k' (the merge pass reads at most k' keys'
-          // worth beyond what it needs)
-          const int lim = t + 1 < t1 ? P - kHalfN : p.kprime;
+          // end, every pool above the end's limit
+          const int lim = t + 1 < t1 ? P - kHalfN : end_lim;
           const uint32_t need = __ballot_sync(0xffffffffu, valid && own_cnt > lim);
           if (need) {
             if (own_cnt > P) atomicOr(B.status, kErrPoolOverflow);
@@ -1028,7 +1094,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
           break;
         }
         // as above, for the next S tiles (both halves)
-        const int lim = t + 1 < t1 ? P - S * kTileRows : p.kprime;
+        const int lim = t + 1 < t1 ? P - S * kTileRows : end_lim;
         const bool mine = (lane & 1) == g;
         const int cn = mine ? cnt_s[row] : 0;
         if (cn > P) atomicOr(B.status, kErrPoolOverflow);
@@ -1140,13 +1206,13 @@ bool make_map(CUtensorMap* m, const void* base, bool fp8, long long rows, long l
 }
 
 // Raises the kernel's dynamic shared memory limit once per device.
-template <int FORM, int MAXI, bool MINIMA = false, bool PAIR = false, bool DUAL = false>
+template <int FORM, int MAXI, bool MINIMA = false, bool PAIR = false, bool DUAL = false, bool FILL = false>
 cudaError_t ensure_attributes() {
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_done[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL>,
+    cudaError_t e = cudaFuncSetAttribute(fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL, FILL>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          227 * 1024);
     if (e != cudaSuccess) return e;
@@ -1155,11 +1221,11 @@ cudaError_t ensure_attributes() {
   return cudaSuccess;
 }
 
-template <int FORM, int MAXI, bool MINIMA = false, bool PAIR = false, bool DUAL = false>
+template <int FORM, int MAXI, bool MINIMA = false, bool PAIR = false, bool DUAL = false, bool FILL = false>
 cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, int n, const FusedBatchPlan& bp,
                         uint32_t* status, unsigned long long* stats, uint32_t smem, cudaStream_t st,
                         const int* run_if) {
-  cudaError_t e = ensure_attributes<FORM, MAXI, MINIMA, PAIR, DUAL>();
+  cudaError_t e = ensure_attributes<FORM, MAXI, MINIMA, PAIR, DUAL, FILL>();
   if (e != cudaSuccess) return e;
   smem = make_layout(FORM, specs[0].d, PAIR ? 1 : 0, kEpiWarps, DUAL ? 1 : 0).total;  // this instance's
   FusedArgs<MAXI> a;
@@ -1225,8 +1291,27 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
       return cudaErrorInvalidValue;
   }
   if (PAIR && bp.grid % 2) return cudaErrorInvalidValue;
-  return launch_dependent(fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL>, (unsigned)bp.grid, kNumThreads, smem, st,
+  return launch_dependent(fused_knn_kernel<FORM, MAXI, MINIMA, PAIR, DUAL, FILL>, (unsigned)bp.grid, kNumThreads, smem, st,
                           bp.pdl != 0, PAIR ? 2 : 1, a);
+}
+
+// The candidate-pool instance of a plan.  Dual blocks without bounds are planned
+// for FP8 alone (plan_fused_batch).
+template <int FORM, int MAXI>
+cudaError_t launch_pools(const FusedItemSpec* specs, const FusedItemPlan* plans, int n, const FusedBatchPlan& bp,
+                         uint32_t* status, unsigned long long* stats, uint32_t smem, cudaStream_t st,
+                         const int* run_if) {
+  if (bp.dual) {
+    if constexpr (FormTraits<FORM>::kFP8)
+      if (bp.fill)
+        return launch_form<FORM, MAXI, false, false, true, true>(specs, plans, n, bp, status, stats, smem, st, run_if);
+    return launch_form<FORM, MAXI, false, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if);
+  }
+  if (bp.pair)
+    return bp.fill ? launch_form<FORM, MAXI, false, true, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
+                   : launch_form<FORM, MAXI, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if);
+  return bp.fill ? launch_form<FORM, MAXI, false, false, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
+                 : launch_form<FORM, MAXI>(specs, plans, n, bp, status, stats, smem, st, run_if);
 }
 
 template <int FORM>
@@ -1238,15 +1323,8 @@ cudaError_t launch_form_any(const FusedItemSpec* specs, const FusedItemPlan* pla
                    : launch_form<FORM, 1, true>(specs, plans, n, bp, status, stats, smem, st, run_if);
   for (int i = 0; i < n; ++i)
     if (specs[i].minima) return cudaErrorInvalidValue;  // block-minimum mode is single-item
-  if (bp.dual)
-    return n == 1 ? launch_form<FORM, 1, false, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
-                    : launch_form<FORM, kFusedMaxItems, false, false, true>(specs, plans, n, bp, status, stats, smem,
-                                                                          st, run_if);
-  if (n == 1)
-    return bp.pair ? launch_form<FORM, 1, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
-                   : launch_form<FORM, 1>(specs, plans, n, bp, status, stats, smem, st, run_if);
-  return bp.pair ? launch_form<FORM, kFusedMaxItems, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
-                 : launch_form<FORM, kFusedMaxItems>(specs, plans, n, bp, status, stats, smem, st, run_if);
+  if (n == 1) return launch_pools<FORM, 1>(specs, plans, n, bp, status, stats, smem, st, run_if);
+  return launch_pools<FORM, kFusedMaxItems>(specs, plans, n, bp, status, stats, smem, st, run_if);
 }
 
 }  // namespace
@@ -1265,8 +1343,6 @@ std::atomic<int> g_dual{CURPLSH_DUAL_DEFAULT};
 // 3.43, 192 4.75 -> 4.36, 256 6.10 -> 5.55, 512 11.5 -> 9.9 (identical results).
 constexpr int kPairMinDimBF16 = 320;
 constexpr int kPairMinDimExact = 192;
-// Dual blocks need units of this many times k' rows when pools start unbounded.
-constexpr int kDualFillRows = 64;
 }  // namespace
 
 void set_cta_pairs(int mode) {
@@ -1298,31 +1374,28 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
     const SmemLayout DL = make_layout(form, specs[0].d, 0, kEpiWarps, 1);
     dual_fits = !DL.a_stream && DL.stages >= (form == kFormExact ? 2 : 3);
   }
-  // Pools that start without a bound fill to k' keys in every unit; a dual
-  // unit has half the rows at the same CTA range, so there are twice as many.
-  // With an estimate (fill_kprime = 0), or with units of many times k' rows,
-  // that is nothing; where it is not, single blocks stay (1,000 queries,
-  // k = 1,024, 300,000 rows without an estimate: 5.7 against 8.4 ms).
-  bool short_units = false;
-  {
-    long long work = 0;
-    for (int i = 0; i < n; ++i)
-      if (specs[i].nb > 0)
-        work += (long long)((specs[i].nq + 2 * kBM - 1) / (2 * kBM)) * ((specs[i].nb + kBN / 2 - 1) / (kBN / 2));
-    const long long w = std::max<long long>(1, work / std::max(1, max_ctas));
-    for (int i = 0; i < n; ++i)
-      short_units = short_units || w * (kBN / 2) < (long long)kDualFillRows * specs[i].fill_kprime;
+  // Pools that start without a bound fill to k' keys in every unit, and a dual
+  // unit has half the rows at the same CTA range, so there are twice as many and
+  // the bounds tighten later.  BF16 and FP32-exact keep single blocks then (1,000
+  // queries, k' = 32, single -> dual: FP32-exact, 100,000 rows 472 -> 686 us;
+  // BF16, 10^6 rows 1,042 -> 1,311; k' = 200 1,877 -> 2,024); FP8, whose MMAs are
+  // light, does not (k' = 480, 8,000 rows 254 -> 63 us).
+  bool fill = false, lean = false;
+  int kp_min = 1 << 30;
+  for (int i = 0; i < n; ++i) {
+    fill = fill || specs[i].fill_kprime > 0;
+    if (specs[i].fill_kprime > 0) kp_min = std::min(kp_min, specs[i].fill_kprime);
+    lean = lean || specs[i].lean;
   }
+  const bool dual_pays = !fill || form == kFormFP8;
   // Two query blocks per CTA: a database tile crosses L2 -> SM once per 256
   // queries, and every query's pool belongs to one lane (full pass, single ->
   // dual blocks: BF16 integer mixture 3.50 -> 2.84 ms, FP32-exact 5.64 -> 4.70)
-  const int dual = (grouped && dual_fits && !short_units && get_dual_blocks()) ? 1 : 0;
+  const int dual = (grouped && dual_fits && dual_pays && !lean && get_dual_blocks()) ? 1 : 0;
   const int pm = get_cta_pairs();
   const int d0 = n > 0 ? specs[0].d : 0;
   const bool want_pair = pm == 1 || (pm == kPairsAuto && ((form == kFormBF16 && d0 >= kPairMinDimBF16) ||
                                                           (form == kFormExact && d0 >= kPairMinDimExact)));
-  bool lean = false;
-  for (int i = 0; i < n; ++i) lean = lean || specs[i].fill_kprime >= kFillSingle;
   const int pair = (!dual && !lean && grouped && want_pair && max_ctas >= 2) ? 1 : 0;
   const int rows = kBM << (pair | dual);
   const int tile_rows = dual ? kBN / 2 : kBN;
@@ -1348,8 +1421,13 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
   out->work_per_cta = total > 0 ? (total + grid - 1) / grid : 1;
   out->grid = total > 0 ? (int)((total + out->work_per_cta - 1) / out->work_per_cta) << pair : 0;
   const long long W = out->work_per_cta;
+  // Pairs whose units are single tiles never fill pools of 128 keys and more, one
+  // per warp, to k': no bound, no selection (FP32-exact, d = 512, k' = 128, 2,000
+  // rows, 1,000 queries: pass 50 us, 146 with shared pools).
+  out->fill = fill && !(pair && W == 1 && kp_min >= kHalfN) ? 1 : 0;
   for (int i = 0; i < n; ++i) {
     FusedItemPlan& pl = plans[i];
+    pl.fill = out->fill;
     int U = 1;
     for (int qb = 0; qb < pl.num_qblocks; ++qb) {
       const long long base = pl.work_begin + (long long)qb * pl.num_tiles;
@@ -1360,12 +1438,13 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
   }
 }
 
-void plan_fused(int nq, int nb, int num_sms, FusedPlan* out, int split_q4, int form, int d, int fill_kprime) {
+void plan_fused(int nq, int nb, int num_sms, FusedPlan* out, int split_q4, int form, int d, int fill_kprime, bool lean) {
   FusedItemSpec s{};
   s.nq = nq;
   s.nb = nb;
   s.d = d;
   s.fill_kprime = fill_kprime;
+  s.lean = lean;
   FusedItemPlan ip;
   FusedBatchPlan bp;
   plan_fused_batch(&s, 1, num_sms, &ip, &bp, form);
@@ -1379,22 +1458,31 @@ void plan_fused(int nq, int nb, int num_sms, FusedPlan* out, int split_q4, int f
   out->grid = bp.grid;
   out->pair = bp.pair;
   out->dual = bp.dual;
+  out->fill = bp.fill;
   out->units_per_block = ip.units_per_block;
   out->split_tiles = ip.split_tiles;
 }
 
 uint32_t fused_smem_bytes(int form, int d) { return make_layout(form, d).total; }
 
+template <int FORM, int MAXI>
+static cudaError_t prepare_pools() {
+  cudaError_t e = ensure_attributes<FORM, MAXI>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, MAXI, false, true>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, MAXI, false, false, true>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, MAXI, false, false, false, true>();
+  if (e == cudaSuccess) e = ensure_attributes<FORM, MAXI, false, true, false, true>();
+  if constexpr (FormTraits<FORM>::kFP8)
+    if (e == cudaSuccess) e = ensure_attributes<FORM, MAXI, false, false, true, true>();
+  return e;
+}
+
 template <int FORM>
 static cudaError_t prepare_form() {
-  cudaError_t e = ensure_attributes<FORM, 1>();
+  cudaError_t e = prepare_pools<FORM, 1>();
+  if (e == cudaSuccess) e = prepare_pools<FORM, kFusedMaxItems>();
   if (e == cudaSuccess) e = ensure_attributes<FORM, 1, true>();
-  if (e == cudaSuccess) e = ensure_attributes<FORM, 1, false, true>();
   if (e == cudaSuccess) e = ensure_attributes<FORM, 1, true, true>();
-  if (e == cudaSuccess) e = ensure_attributes<FORM, 1, false, false, true>();
-  if (e == cudaSuccess) e = ensure_attributes<FORM, kFusedMaxItems>();
-  if (e == cudaSuccess) e = ensure_attributes<FORM, kFusedMaxItems, false, true>();
-  if (e == cudaSuccess) e = ensure_attributes<FORM, kFusedMaxItems, false, false, true>();
   return e;
 }
 
@@ -1478,12 +1566,14 @@ cudaError_t launch_fused(const FusedLaunch& f, cudaStream_t st) {
   ip.work_end = (long long)f.plan.num_qblocks * f.plan.num_tiles;
   ip.pair = f.plan.pair;
   ip.dual = f.plan.dual;
+  ip.fill = f.plan.fill;
   FusedBatchPlan bp;
   bp.total_work = ip.work_end;
   bp.work_per_cta = f.plan.work_per_cta;
   bp.grid = f.plan.grid;
   bp.pair = f.plan.pair;
   bp.dual = f.plan.dual;
+  bp.fill = f.plan.fill;
   bp.pdl = f.pdl ? 1 : 0;
   return launch_fused_batch(f.form, &s, &ip, 1, bp, f.status, f.stats, st, f.run_if);
 }

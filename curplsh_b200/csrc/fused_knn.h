@@ -7,6 +7,10 @@
 
 namespace curplsh_b200 {
 
+// Candidate pools of one query in one unit: the two warps of a lane group have
+// one each in CTA pairs, unless the pools start without a bound.
+constexpr int pool_lists(int pair, int fill) { return pair && !fill ? 2 : 1; }
+
 struct FusedPlan {
   int num_qblocks = 0;        // G = ceil(nq / (128 << pair)): query blocks, or groups of two with CTA pairs
   int num_tiles = 0;          // T = ceil(nb / 256)
@@ -16,9 +20,10 @@ struct FusedPlan {
   int split_tiles = 1;        // L: resolved unit length limit
   int pair = 0;               // 1: clusters of two CTAs share each 256-row MMA (two query blocks)
   int dual = 0;               // 1: one CTA holds two query blocks against 128-row database tiles
+  int fill = 0;               // 1: the pools start without a bound
   // pool rows of the plan (pools and counts are indexed by query row)
   long long pool_rows() const { return (long long)num_qblocks * (128LL << (pair | dual)); }
-  int lists_per_unit() const { return pair ? 2 : 1; }  // candidate pools of one query in one unit
+  int lists_per_unit() const { return pool_lists(pair, fill); }
 };
 
 // Tuned launch parameters for one (form, d, k, Q) bucket (tuning.cpp).
@@ -78,11 +83,10 @@ struct FusedLaunch {
 
 // One search over at most num_sms CTAs.  split_q4 < 4 cuts units shorter than
 // the CTA ranges (split_tiles_for(W, split_q4)); >= 4 leaves the ranges whole.
-// `form` (-1: unknown) decides whether dual blocks may be used, and
-// `fill_kprime` > 0 says that pools start without a bound and fill to that many
-// keys first (FusedItemSpec::fill_kprime).
+// `form` (-1: unknown) decides whether dual blocks may be used; `fill_kprime`
+// and `lean` as in FusedItemSpec.
 void plan_fused(int nq, int nb, int num_sms, FusedPlan* out, int split_q4 = 4, int form = -1, int d = 0,
-                int fill_kprime = 0);
+                int fill_kprime = 0, bool lean = false);
 uint32_t fused_smem_bytes(int form, int d);
 cudaError_t launch_fused(const FusedLaunch& f, cudaStream_t st);
 
@@ -95,7 +99,9 @@ constexpr int kFusedMaxItems = 16;
 
 struct FusedItemSpec {
   int nq, nb, d, kprime, pool_cap;
-  int fill_kprime;  // planning: k' when the pools start without a bound, 0 when an estimate bounds them
+  int fill_kprime;  // planning: k' when the pools start without a bound (no estimate), else 0
+  bool lean;        // planning: single query blocks, which need the least pool memory (dual blocks and CTA
+                    // pairs round the pools up to 256 queries, and pairs have two per query and unit)
   int split_tiles;  // max tiles per unit (<= 0: no limit beyond the CTA ranges)
   long long nq_pad, nb_pad, ld16, ld8;
   const __nv_bfloat16* qh;
@@ -123,12 +129,14 @@ struct FusedItemPlan {
   long long work_begin, work_end;
   int pair;         // the launch's FusedBatchPlan::pair
   int dual;         // the launch's FusedBatchPlan::dual
+  int fill;         // the launch's FusedBatchPlan::fill
 };
 struct FusedBatchPlan {
   long long total_work = 0, work_per_cta = 1;
   int grid = 0;
   int pair = 0;  // 1: clusters of two CTAs; work_per_cta is per pair and grid counts CTAs
   int dual = 0;  // 1: each CTA takes query groups of two blocks and 128-row database tiles
+  int fill = 0;  // 1: some item's pools start without a bound
   int pdl = 0;   // 1: launched as a programmatic dependent (launch_dependent)
 };
 // CTA pairs on (1) or off (0, default) for the plans made after the call.
@@ -140,7 +148,7 @@ int get_cta_pairs();
 // Dual query blocks on or off for the plans made after the call.
 void set_dual_blocks(int on);
 int get_dual_blocks();
-// Plans `n` items over at most `max_ctas` CTAs.  Only nq, nb, d, fill_kprime and
+// Plans `n` items over at most `max_ctas` CTAs.  Only nq, nb, d, fill_kprime, lean and
 // split_tiles of the specs are read, so pool sizes (which depend on units_per_block) can be computed
 // from the plan before the pools are carved.
 void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItemPlan* plans, FusedBatchPlan* out,
@@ -173,10 +181,6 @@ struct EstimatePlan {
 // `lean`: only the estimates of at most a tenth of the rows among 128-row blocks,
 // for callers short of working memory.
 EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms, bool lean = false);
-// FusedItemSpec::fill_kprime of a lean plan, which keeps single query blocks:
-// dual blocks and CTA pairs round the pools up to 256 queries and pairs have two
-// pools per query and unit.
-constexpr int kFillSingle = 1 << 30;
 // The process-wide switch (curplsh_set_bound_estimate).
 bool bound_estimate_enabled();
 

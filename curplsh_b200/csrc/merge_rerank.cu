@@ -173,9 +173,10 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   // list by list, each of the up to 148 short lists of a few-query search was a
   // load latency of its own (merge of 16 queries against 2 x 10^6 rows 164 -> 23
   // us, of one query against 10^4 rows 56 -> 19, of 1,000 queries with k = 1,024
-  // 312 -> 212).  A thread's list only moves forward; with a binary search per key
-  // long lists took three times as long (k' = 1,024, 10^6 rows, one query without a
-  // bound: 3.47 -> 1.20 ms, 1.76 list by list).
+  // 312 -> 212).  A thread's list only moves forward, a few at a time or by a binary
+  // search in the offsets; with the search for every key long lists took three
+  // times as long (k' = 1,024, 10^6 rows, one query without a bound: 3.47 -> 1.20
+  // ms, 1.76 list by list).
   int total = 0;
   for (int l0 = 0; l0 < nlists; l0 += NT) {
     const int l = l0 + tid;
@@ -204,9 +205,25 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
         const int i = i0 + u * NT;
         key[u] = kKeyEmpty;
         if (i < total) {
-          while (i >= hi) {
-            lo = hi;
-            hi = loff[++l + 1];
+          if (i >= hi) {
+            int steps = 4;
+            do {
+              lo = hi;
+              hi = loff[++l + 1];
+            } while (i >= hi && --steps);
+            if (i >= hi) {  // short lists: loff[l] <= i < loff[h]
+              int h = nlists;
+              ++l;
+              while (h - l > 1) {
+                const int mid = (l + h) >> 1;
+                if (loff[mid] <= i)
+                  l = mid;
+                else
+                  h = mid;
+              }
+              lo = loff[l];
+              hi = loff[l + 1];
+            }
           }
           key[u] = m.pools[(list0 + (size_t)l) * (size_t)m.pool_cap + (size_t)(i - lo)];
         }

@@ -164,7 +164,8 @@ int MultiPlan::build(const curplsh_batch_item* items, int n, const std::vector<c
         specs[j].d = G.d;
         if (use_est) x.est = plan_estimate(x.nq, views[x.slot].n, x.kp, num_sms, lean);
         FL.est_any = FL.est_any || x.est.on;
-        specs[j].fill_kprime = lean ? kFillSingle : x.est.on ? 0 : x.kp;
+        specs[j].fill_kprime = x.est.on ? 0 : x.kp;
+        specs[j].lean = lean;
         // units as long as the item's own CTA ranges would be if it were
         // searched alone (scaled by the tuned split, at most the whole range,
         // as alone), so its in-pool selection work stays what it is alone
@@ -216,7 +217,7 @@ int MultiPlan::build(const curplsh_batch_item* items, int n, const std::vector<c
     bcur += (size_t)x.nq_pad;
     if (v.n == 0) continue;
     const size_t lists = (size_t)x.plan.num_qblocks * ((size_t)kBM << (x.plan.pair | x.plan.dual)) *
-                         x.plan.units_per_block * (x.plan.pair ? 2 : 1);
+                         x.plan.units_per_block * pool_lists(x.plan.pair, x.plan.fill);
     if (x.form != kFormFP8) x.o_qh = take((size_t)x.nq_pad * v.ld16 * 2);
     if (x.form == kFormExact) x.o_ql = take((size_t)x.nq_pad * v.ld16 * 2);
     if (x.form == kFormFP8) x.o_q8 = take((size_t)x.nq_pad * v.ld8);
@@ -404,7 +405,7 @@ int MultiPlan::enqueue(cudaStream_t main, const std::vector<cudaStream_t>* branc
           m.num_tiles = v.n > 0 ? x.plan.num_tiles : 0;
           m.units_per_block = v.n > 0 ? x.plan.units_per_block : 1;
           m.pair = x.plan.pair | x.plan.dual;
-          m.lists = x.plan.pair ? 2 : 1;
+          m.lists = pool_lists(x.plan.pair, x.plan.fill);
           m.row0 = x.row0[j];
           m.split_tiles = v.n > 0 ? x.plan.split_tiles : 1;
           m.work_begin = x.plan.work_begin;

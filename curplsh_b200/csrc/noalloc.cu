@@ -151,14 +151,14 @@ int search_noalloc_locked(const IndexView& v, int nq, const float* q, int k, int
   FusedPlan plan{};
   Layout L{};
   int cap = v.num_sms;
-  int fill = kp;  // dual blocks where the schedule fits them whole, else the lean plan
+  bool lean = false;  // dual blocks or pairs where the schedule fits them whole, else the lean plan
   for (;;) {
-    plan_fused(nq, (int)v.n, cap, &plan, 4, form, v.dim, fill);
+    plan_fused(nq, (int)v.n, cap, &plan, 4, form, v.dim, kp, lean);
     const size_t lists = (size_t)plan.pool_rows() * plan.units_per_block * plan.lists_per_unit();
     L = carve(form, nq_pad, v.ld16, v.ld8, lists, P);
-    if (L.total <= kNoAllocScratchBytes || (cap == 1 && fill != kp)) break;
-    if (fill == kp)
-      fill = kFillSingle;
+    if (L.total <= kNoAllocScratchBytes || (cap == 1 && lean)) break;
+    if (!lean)
+      lean = true;
     else
       cap = cap * 3 / 4 > 1 ? cap * 3 / 4 : 1;
   }

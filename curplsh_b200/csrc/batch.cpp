@@ -119,14 +119,14 @@ int plan_batch(curplsh_batch* b) {
                          num_sms);
   if (rc) return rc;
   b->ws_bytes = b->plan.bytes();
-  if (cudaMalloc(&b->ws, b->ws_bytes) != cudaSuccess) {  // short of memory: a plan with less
+  if (device_malloc(b->device, &b->ws, b->ws_bytes) != cudaSuccess) {  // short of memory: a plan with less
     cudaGetLastError();
     b->ws = nullptr;
     rc = b->plan.build(b->items.data(), (int)b->items.size(), b->uniq, b->views, b->precision, b->rerank_factor,
                        num_sms, true);
     if (rc) return rc;
     b->ws_bytes = b->plan.bytes();
-    BT_TRY(cudaMalloc(&b->ws, b->ws_bytes));
+    BT_TRY(device_malloc(b->device, &b->ws, b->ws_bytes));
   }
   b->plan.bind(b->ws);
   b->status = b->plan.status();

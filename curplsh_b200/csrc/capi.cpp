@@ -111,6 +111,7 @@ struct DevRes {
   cudaStream_t alt[2] = {nullptr, nullptr};
   cudaStream_t copy = nullptr;
   int num_sms = 0;
+  int device = 0;
   cudaMemPool_t pool = nullptr;
 };
 
@@ -154,6 +155,11 @@ struct SharedPools {
     *out = p.pool;
     return cudaSuccess;
   }
+  void trim(int device) {
+    std::lock_guard<std::mutex> lk(mu);
+    auto p = by_device.find(device);
+    if (p != by_device.end() && p->second.pool) cudaMemPoolTrimTo(p->second.pool, 0);
+  }
   void give(int device) {  // the caller's memory from the pool is freed
     std::lock_guard<std::mutex> lk(mu);
     Entry& p = by_device[device];
@@ -169,32 +175,38 @@ static SharedPools& shared_pools() {
   return *p;
 }
 
+static bool is_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return cap != cudaStreamCaptureStatusNone;
+}
+
+// `alloc()`, and once more with what the current device's pool keeps given back
+// when memory is short.  Memory freed in a stream's order counts as kept only
+// once that stream's work is done, hence the wait.
+template <class Alloc>
+static cudaError_t alloc_or_trim(int device, Alloc alloc) {
+  cudaError_t e = alloc();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
+  shared_pools().trim(device);
+  return alloc();
+}
+
 // `st` orders the allocation; only work after it on `st` (or synchronised with
 // it) may use the memory.
 static cudaError_t pool_alloc(DevRes* d, void** p, size_t bytes, cudaStream_t st, bool* pooled) {
   *pooled = false;
-  if (bytes > kPoolMaxBytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation) {  // give back what the pool keeps, once
-      cudaGetLastError();
-      cudaMemPoolTrimTo(d->pool, 0);
-      e = cudaMalloc(p, bytes);
-    }
-    return e;
-  }
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return cudaMalloc(p, bytes);  // an allocation recorded into a graph would belong to the graph
-  }
-  *pooled = true;
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
-  if (e == cudaErrorMemoryAllocation) {  // give back what the pool keeps, once
-    cudaGetLastError();
-    cudaMemPoolTrimTo(d->pool, 0);
-    e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
-  }
-  return e;
+  // an allocation recorded into a graph would belong to the graph
+  if (is_capturing(st)) return cudaMalloc(p, bytes);
+  *pooled = bytes <= kPoolMaxBytes;
+  return alloc_or_trim(d->device, [&]() {
+    return *pooled ? cudaMallocFromPoolAsync(p, bytes, d->pool, st) : cudaMalloc(p, bytes);
+  });
 }
 
 // Device buffer that only grows.
@@ -215,7 +227,8 @@ struct DevBuf {
     return e;
   }
   void release(cudaStream_t st) {
-    if (ptr && (!pooled || cudaFreeAsync(ptr, st) != cudaSuccess)) cudaFree(ptr);
+    // (a free recorded into a graph would have to be of the graph's own memory)
+    if (ptr && (!pooled || is_capturing(st) || cudaFreeAsync(ptr, st) != cudaSuccess)) cudaFree(ptr);
     ptr = nullptr;
     cap = 0;
   }
@@ -288,6 +301,7 @@ int init_device(curplsh_resources* r, int device, DevRes** out) {
   CUDA_TRY(cudaStreamCreateWithFlags(&d.alt[1], cudaStreamNonBlocking));
   CUDA_TRY(cudaStreamCreateWithFlags(&d.copy, cudaStreamNonBlocking));
   CUDA_TRY(cudaDeviceGetAttribute(&d.num_sms, cudaDevAttrMultiProcessorCount, device));
+  d.device = device;
   CUDA_TRY(shared_pools().take(device, &d.pool));
   auto res = r->devs.emplace(device, d);
   *out = &res.first->second;
@@ -1107,6 +1121,9 @@ int do_search(curplsh_index* ix, int64_t num, const float* queries, int k, int p
 
 // ================================================================== internals
 namespace curplsh_b200 {
+cudaError_t device_malloc(int device, void** p, size_t bytes) {
+  return alloc_or_trim(device, [&]() { return cudaMalloc(p, bytes); });
+}
 int index_lock_view(curplsh_index* ix, IndexView* v) {
   if (!ix || !v) return set_error(CURPLSH_ERR_INVALID_ARG, "null argument");
   ix->mu.lock_shared();
@@ -1357,7 +1374,7 @@ int curplsh_index_add(curplsh_index* ix, int64_t num, const float* data) {
     x32 = const_cast<float*>(data);
   } else {
     if (ix->cfg.memory_space == CURPLSH_MEMORY_UNIFIED)
-      CUDA_TRY(cudaMallocManaged(&x32, (size_t)n_new * d * sizeof(float)));
+      CUDA_TRY(alloc_or_trim(ix->cfg.device, [&]() { return cudaMallocManaged(&x32, (size_t)n_new * d * sizeof(float)); }));
     else
       CUDA_TRY(ix->alloc(&x32, (size_t)n_new * d * sizeof(float), st));
     if (n_old) CUDA_TRY(cudaMemcpyAsync(x32, ix->x32, (size_t)n_old * d * sizeof(float), cudaMemcpyDeviceToDevice, st));

@@ -356,6 +356,9 @@ struct IndexView {
   cudaStream_t stream;   // the index's default stream
   cudaEvent_t fp8_ready; // recorded after the FP8 copy (x8, xs) was written; wait on it before reading them
 };
+// cudaMalloc on the current device `device`, and once more with what the library's
+// pool there keeps given back when memory is short (capi.cpp).
+cudaError_t device_malloc(int device, void** p, size_t bytes);
 // Locks the index (same lock as search/add) and fills `out`; unlock with index_unlock.
 int index_lock_view(curplsh_index* index, IndexView* out);
 void index_unlock(curplsh_index* index);

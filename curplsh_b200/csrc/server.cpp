@@ -449,7 +449,7 @@ int curplsh_server_create(curplsh_index* index, const curplsh_server_config* cfg
   cudaSetDevice(s->device);
   auto restore = [&]() { cudaSetDevice(prev); };
   cudaError_t e = cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, s->device);
-  if (e == cudaSuccess) e = cudaMalloc(&s->arena_mem, (size_t)c.memory_budget);
+  if (e == cudaSuccess) e = device_malloc(s->device, &s->arena_mem, (size_t)c.memory_budget);
   for (int i = 0; i < c.max_inflight && e == cudaSuccess; ++i) {
     Slot sl;
     e = cudaStreamCreateWithFlags(&sl.st, cudaStreamNonBlocking);

@@ -81,3 +81,50 @@ def test_forms_agree_with_and_without_a_light_sample(env, form, spread, n, nq, k
     np.testing.assert_array_equal(i1, i0)
     np.testing.assert_array_equal(d1, d0)
     assert failed == 0
+
+
+def _sampled_rows(rows, step):
+    """Database rows of a light sample (curplsh_index_estimate_sample)."""
+    i = np.arange(rows, dtype=np.uint64)
+    phase = ((i // 256 * 2654435769) % 2**32 * step) >> np.uint64(32)
+    return (i * step + phase).astype(np.int64)
+
+
+# sample blocks of 8 and of 128 rows; host arrays (the host searches failed queries
+# again) and device arrays (the stream does)
+@pytest.mark.parametrize("n,nq,k", [(10_000, 2, 10), (300_000, 200, 10)])
+@pytest.mark.parametrize("host", [True, False])
+def test_a_light_sample_that_fails(env, n, nq, k, host):
+    """Only the sampled rows are near the queries and the rank is below k' = 32, so
+    every bound is too small."""
+    import torch
+    cb, res = env
+    rng = np.random.default_rng(n)
+    base = rng.random((n, 32), dtype=np.float32) + np.float32(50.0)
+    queries = rng.random((nq, 32), dtype=np.float32)
+    ix = cb.IndexBF(res, 32, cb.IndexBFConfig(precision=0))
+    ix.add(n, base)
+    assert ix.estimate_plan(nq, k)[0] == 0
+    rows, step, _, rank = ix.estimate_sample(nq, k)
+    at = _sampled_rows(rows, step)
+    assert 0 < rank < 24 and at.max() < n and len(np.unique(at)) == rows
+    ix.reset()
+    base[at] -= np.float32(50.0)
+    ix.add(n, base)
+
+    def search():
+        if host:
+            return [np.asarray(a) for a in ix.search_array(queries, k)]
+        i, x = torch.empty((nq, k), dtype=torch.int32, device="cuda"), torch.empty((nq, k), device="cuda")
+        ix.search(nq, torch.tensor(queries).cuda(), k, i, x)
+        torch.cuda.synchronize()
+        return [x.cpu().numpy(), i.cpu().numpy()]
+
+    d1, i1 = search()
+    assert ix.fallback_count() == nq
+    cb.set_bound_estimate(False)
+    d0, i0 = search()
+    cb.set_bound_estimate(True)
+    ix.close()
+    np.testing.assert_array_equal(i1, i0)
+    np.testing.assert_array_equal(d1, d0)

@@ -1335,12 +1335,14 @@ cudaError_t launch_form_any(const FusedItemSpec* specs, const FusedItemPlan* pla
 namespace {
 std::atomic<int> g_cta_pairs{kPairsAuto};
 std::atomic<int> g_dual{CURPLSH_DUAL_DEFAULT};
-// Automatic CTA pairs: from these dimensions on, the MMAs of a tile are heavy
-// enough that halving each SM's database bytes per query pays.  Measured on
-// 10^6 N(0,1) BF16-valued rows, 4,096 queries (k = 10) and 2,048 (k = 100),
-// single CTAs -> pairs: BF16 d = 128 2.33 -> 2.93 ms, 256 3.15 -> 3.44, 320
-// 3.59 -> 3.48, 384 4.67 -> 3.83, 512 5.98 -> 4.54; FP32-exact d = 128 3.44 ->
-// 3.43, 192 4.75 -> 4.36, 256 6.10 -> 5.55, 512 11.5 -> 9.9 (identical results).
+// Automatic CTA pairs: BF16 and FP32-exact from these dimensions on, where two
+// query blocks no longer fit one CTA and the MMAs of a tile are heavy enough that
+// halving each SM's database bytes per query pays (500,000 N(0,1) rows, 4,096
+// queries, k = 10, pass with single blocks -> pairs: BF16 d = 320 1,381 -> 986 us,
+// 384 2,160 -> 1,144, 512 2,641 -> 1,377; FP32-exact 192 2,047 -> 1,272, 256 2,478
+// -> 1,795, 384 3,498 -> 2,650; identical results).  Below the lines dual blocks
+// are the rule; between the last of them and the line (FP32-exact d = 123 to 191,
+// BF16 315 to 319) pairs measure ahead too (FP32-exact 144: 2,218 -> 1,067).
 constexpr int kPairMinDimBF16 = 320;
 constexpr int kPairMinDimExact = 192;
 }  // namespace
@@ -1394,8 +1396,14 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
   const int dual = (grouped && dual_fits && dual_pays && !lean && get_dual_blocks()) ? 1 : 0;
   const int pm = get_cta_pairs();
   const int d0 = n > 0 ? specs[0].d : 0;
+  // FP8 pairs where a CTA's own ring is down to two stages, which no longer cover
+  // the load latency: the norm tail's chunk took the third at d = 768 (pass, single
+  // -> pairs: 1,842 -> 1,425 us, 1,620 before there was a tail; 1,024 2,376 ->
+  // 1,714; with three stages, d = 704, 1,385 -> 1,477)
+  const bool fp8_pair = form == kFormFP8 && d0 > 0 && make_layout(form, d0).stages < 3;
   const bool want_pair = pm == 1 || (pm == kPairsAuto && ((form == kFormBF16 && d0 >= kPairMinDimBF16) ||
-                                                          (form == kFormExact && d0 >= kPairMinDimExact)));
+                                                          (form == kFormExact && d0 >= kPairMinDimExact) ||
+                                                          (form == kFormFP8 && fp8_pair)));
   const int pair = (!dual && !lean && grouped && want_pair && max_ctas >= 2) ? 1 : 0;
   const int rows = kBM << (pair | dual);
   const int tile_rows = dual ? kBN / 2 : kBN;

@@ -33,6 +33,8 @@ namespace {
 // at k' = 224, d = 128, 0.32 -> 0.28 ms); 256 win where it is large (the
 // batched workload, d up to 512: 93 -> 74 ms per graph replay).
 constexpr int kMergeSmallRerank = 65536;
+// Keys per list from which a thread walks from list to list.
+constexpr int kMergeWalkKeys = 64;
 // Candidates one warp reranks at once: each lane keeps this many database rows
 // in flight (a row of d = 128 is one 16-byte load per lane).
 #ifndef CURPLSH_RERANK_ROWS
@@ -173,10 +175,11 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   // list by list, each of the up to 148 short lists of a few-query search was a
   // load latency of its own (merge of 16 queries against 2 x 10^6 rows 164 -> 23
   // us, of one query against 10^4 rows 56 -> 19, of 1,000 queries with k = 1,024
-  // 312 -> 212).  A thread's list only moves forward, a few at a time or by a binary
-  // search in the offsets; with the search for every key long lists took three
-  // times as long (k' = 1,024, 10^6 rows, one query without a bound: 3.47 -> 1.20
-  // ms, 1.76 list by list).
+  // 312 -> 212).  A key's list comes from a binary search
+  // in the offsets, four at once, or, where the lists are long, from a walk (a
+  // thread's list only moves forward).  k' = 1,024, 10^6 rows, one query without a
+  // bound: 3.47 ms by searches, 1.20 by walking, 1.76 list by list; k' = 32, 2.3 x
+  // 10^6 rows, one query, nine keys a list: 23 us by searches, 43 by walking.
   int total = 0;
   for (int l0 = 0; l0 < nlists; l0 += NT) {
     const int l = l0 + tid;
@@ -196,36 +199,40 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   constexpr int kLoads = 4;
   // f(key, on) for this thread's share of the keys, called by whole warps (on =
   // false past the end and for keys above the final bound)
+  const bool walk = total >= kMergeWalkKeys * nlists;
   auto each_pool_key = [&](auto f) {
-    int l = 0, lo = 0, hi = loff[nlists > 0 ? 1 : 0];  // list l holds the keys [lo, hi); it only moves forward
+    int l = 0, lo = 0, hi = loff[nlists > 0 ? 1 : 0];  // list l holds the keys [lo, hi)
     for (int i0 = tid; i0 - tid < total; i0 += kLoads * NT) {
       uint64_t key[kLoads];
+      if (walk) {
 #pragma unroll
-      for (int u = 0; u < kLoads; ++u) {
-        const int i = i0 + u * NT;
-        key[u] = kKeyEmpty;
-        if (i < total) {
-          if (i >= hi) {
-            int steps = 4;
-            do {
+        for (int u = 0; u < kLoads; ++u) {
+          const int i = i0 + u * NT;
+          key[u] = kKeyEmpty;
+          if (i < total) {
+            while (i >= hi) {
               lo = hi;
               hi = loff[++l + 1];
-            } while (i >= hi && --steps);
-            if (i >= hi) {  // short lists: loff[l] <= i < loff[h]
-              int h = nlists;
-              ++l;
-              while (h - l > 1) {
-                const int mid = (l + h) >> 1;
-                if (loff[mid] <= i)
-                  l = mid;
-                else
-                  h = mid;
-              }
-              lo = loff[l];
-              hi = loff[l + 1];
             }
+            key[u] = m.pools[(list0 + (size_t)l) * (size_t)m.pool_cap + (size_t)(i - lo)];
           }
-          key[u] = m.pools[(list0 + (size_t)l) * (size_t)m.pool_cap + (size_t)(i - lo)];
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < kLoads; ++u) {
+          const int i = i0 + u * NT;
+          key[u] = kKeyEmpty;
+          if (i < total) {
+            int a0 = 0, a1 = nlists;  // loff[a0] <= i < loff[a1]
+            while (a1 - a0 > 1) {
+              const int mid = (a0 + a1) >> 1;
+              if (loff[mid] <= i)
+                a0 = mid;
+              else
+                a1 = mid;
+            }
+            key[u] = m.pools[(list0 + (size_t)a0) * (size_t)m.pool_cap + (size_t)(i - loff[a0])];
+          }
         }
       }
 #pragma unroll

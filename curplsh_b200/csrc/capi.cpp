@@ -576,21 +576,28 @@ int binomial_rank(int n, double q) {
   return hi;
 }
 
-// Smallest rank j <= most * n with exp(-n KL(j / n || q)) <= kEstimateFailure, a
-// bound of P(X >= j) for j / n >= q that costs two logarithms (one or two ranks
-// above the exact tail's); 0 if there is none.
+// Whether exp(-n KL(j / n || q)) <= kEstimateFailure, a bound of P(X >= j) for
+// j / n >= q that costs two logarithms (one or two ranks above the exact tail's).
+bool chernoff_small(int n, double q, int j) {
+  const double p = (double)j / n;
+  if (p <= q) return false;
+  const double kl = p * std::log(p / q) + (p < 1.0 ? (1.0 - p) * std::log((1.0 - p) / (1.0 - q)) : 0.0);
+  return n * kl >= -std::log(kEstimateFailure);
+}
+// Smallest such rank j <= most * n; 0 if there is none.
 int chernoff_rank(int n, double q, double most) {
-  auto small = [&](int j) {
-    const double p = (double)j / n;
-    if (p <= q) return false;
-    const double kl = p * std::log(p / q) + (p < 1.0 ? (1.0 - p) * std::log((1.0 - p) / (1.0 - q)) : 0.0);
-    return n * kl >= -std::log(kEstimateFailure);
-  };
   int lo = (int)(q * n), hi = (int)(most * n);  // small(hi) and not small(lo)
-  if (hi < 1 || hi <= lo || !small(hi)) return 0;
+  if (hi < 1 || hi <= lo || !chernoff_small(n, q, hi)) return 0;
+  for (int step = 4; lo + step < hi; step *= 2) {  // the rank is a few deviations above the mean
+    if (chernoff_small(n, q, lo + step)) {
+      hi = lo + step;
+      break;
+    }
+    lo += step;
+  }
   while (hi - lo > 1) {
     const int mid = (lo + hi) / 2;
-    (small(mid) ? hi : lo) = mid;
+    (chernoff_small(n, q, mid) ? hi : lo) = mid;
   }
   return hi;
 }
@@ -650,27 +657,29 @@ EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms, bool lean) 
     for (int den = 2; den <= 640; den *= 2) {
       const long long t = n / ((long long)kBN * den);
       if (t < 1) break;
+      int br = kEstimateBlockRows;
+      double most = 0.5, p = (double)kp / (double)n;
+      int r = chernoff_rank((int)(t * kBN / br), under(br, p), most);
+      if (r == 0 && t <= kEstimateFineMaxTiles)
+        r = chernoff_rank((int)(t * kBN / kEstimateFineRows), under(br = kEstimateFineRows, p), most = 0.9);
+      if (r == 0) continue;
+      const int blocks = (int)(t * kBN / br);
+      const double admitted = (double)n * -std::expm1(std::log1p(-(double)r / blocks) / br);
+      const double cost = (double)t * kBN + kLightSurvivorRows * std::min(1.0, nq / (double)kBM) * admitted;
+      if (j != 0 && cost >= best) continue;
       // The sample is spread over the first t * kBN * step rows, four fifths of the
       // database at the least (t = T / den had a step of 1 or 3 where n is just
       // short of the next step, and took the leading half or three quarters).  All
       // k' may lie among them, so the rank goes by their share of those rows: rows
       // added in order then keep the failure probability (1,000 of 1,000 queries
       // near the first half of 30,000 rows failed before).
-      const double p = (double)kp / (double)(t * kBN * (n / (t * kBN)));
-      int br = kEstimateBlockRows;
-      int r = chernoff_rank((int)(t * kBN / br), under(br, p), 0.5);
-      if (r == 0 && t <= kEstimateFineMaxTiles)
-        r = chernoff_rank((int)(t * kBN / kEstimateFineRows), under(br = kEstimateFineRows, p), 0.9);
-      if (r == 0) continue;
-      const double blocks = (double)(t * kBN / br);
-      const double admitted = (double)n * -std::expm1(std::log1p(-r / blocks) / br);
-      const double cost = (double)t * kBN + kLightSurvivorRows * std::min(1.0, nq / (double)kBM) * admitted;
-      if (j == 0 || cost < best) {
-        best = cost;
-        tiles = t;
-        block_rows = br;
-        j = r;
-      }
+      const double q = under(br, (double)kp / (double)(t * kBN * (n / (t * kBN))));
+      while (r <= most * blocks && !chernoff_small(blocks, q, r)) ++r;
+      if (r > most * blocks) continue;
+      best = cost;
+      tiles = t;
+      block_rows = br;
+      j = r;
     }
     if (j == 0) return e;
   }

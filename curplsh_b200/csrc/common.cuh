@@ -142,7 +142,8 @@ struct FusedItem {
   int* pool_counts;        // [G_i*128][U_i]
   uint32_t* q_bound;       // [nq_pad] shared per-query bound (ordered bits), init kOrdInf or an estimate
   // Database row j of this item is stored row j * db_step (>= 1; > 1 in
-  // block-minimum mode only), plus sample_phase(j / 256, db_step) when db_phased.
+  // block-minimum mode only), plus sample_phase(j / 256, db_step) when db_phased,
+  // which then is the columns of a stored row.
   int db_step, db_phased;
   float db_scale_uniform;  // > 0: every database row has this FP8 scale s (db_scale is not read)
   // FP8 form with one database scale: the byte offset of the 32-byte BF16 norm

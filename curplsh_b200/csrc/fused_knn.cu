@@ -469,15 +469,6 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
         else
           tma_load_2d(dst, m, bar, c0, c1, pol);
       };
-      // database tiles; a sample's map is 3-D: (column, phase, sample row)
-      auto load_x = [&](void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int phase, int row, uint64_t pol) {
-        if constexpr (MINIMA && PAIR)
-          tma_load_3d_pair(dst, m, bar, c0, phase, row, pol);
-        else if constexpr (MINIMA)
-          tma_load_3d(dst, m, bar, c0, phase, row, pol);
-        else
-          load(dst, m, bar, c0, row, pol);
-      };
       const uint32_t tx_mul = pair ? 2u : 1u;
       const int half_row = pair ? (int)rank * (kBN / 2) : 0;  // this CTA's rows of a tile
       UnitWalk walk(blockIdx.x, B, rank);
@@ -523,7 +514,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
           const int tile = (t - rot + T_i) % T_i;  // database tile of position t
           const int tx_row = tile * kTileRows + half_row;
           const FusedItem& p = A.items[MAXI == 1 ? 0 : ii];
-          const int phase = MINIMA && p.db_phased ? sample_phase(tile, p.db_step) : 0;
+          // column of a phased sample's row in its map (make_map)
+          const int col0 = MINIMA && p.db_phased ? sample_phase(tile, p.db_step) * p.db_phased : 0;
           for (int kc = 0; kc < nreg; ++kc, ++it) {
             const int s = (int)(it % (uint32_t)S);
             STAT_BEGIN(tw);
@@ -539,14 +531,14 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
             if (with_tail) tx += L.b_tail + (L.a_stream ? kATailBytes : 0u);
             if (issuer) mbar_arrive_expect_tx(&full[s], tx_mul * tx);
             for (int part = 0; part < Tr::kBParts; ++part)
-              load_x(st + part * L.b_chunk, part ? &tm_x_lo : &tm_x_hi, &full[s], kc * KC, phase, tx_row, pol_db);
+              load(st + part * L.b_chunk, part ? &tm_x_lo : &tm_x_hi, &full[s], col0 + kc * KC, tx_row, pol_db);
             if (L.a_stream)
               for (int part = 0; part < Tr::kAParts; ++part)
                 load(st + stage_a_off<Tr::kAParts, Tr::kBParts>(L, part), part ? &tm_q_lo : &tm_q_hi, &full[s],
                      kc * KC, qb * kBM, pol_q);
             if (with_tail) {
               uint8_t* tl = st + stage_tail_off<Tr::kAParts, Tr::kBParts>(L);
-              load_x(tl, &tm_x_tail, &full[s], nreg * KC, phase, tx_row, pol_db);
+              load(tl, &tm_x_tail, &full[s], col0 + nreg * KC, tx_row, pol_db);
               if (L.a_stream) load(tl + L.b_tail, &tm_q_tail, &full[s], nreg * KC, qb * kBM, pol_q);
             }
           }
@@ -1183,22 +1175,21 @@ EncodeTiledFn get_encode_fn() {
 
 // 2-D K-major operand map: rows x ld elements, box = (128 bytes of K) x box_rows
 // with the 128-byte swizzle, or (narrow) 32 bytes of K with the 32-byte
-// swizzle; zero fill out of bounds.  sample_step > 0: the 3-D map of a sample,
-// (column, phase, sample row), whose row j at phase f is stored row j *
-// sample_step + f.
+// swizzle; zero fill out of bounds.  Map row j is stored row j * row_step; with
+// `phased` it is the row_step stored rows from there on, one after another: row f
+// of them starts at column f * ld_elems, and a box that reaches past it holds the
+// next row's first columns, which meet zeros of the query rows.
 bool make_map(CUtensorMap* m, const void* base, bool fp8, long long rows, long long ld_elems, int box_rows,
-              bool narrow = false, int sample_step = 0) {
+              bool narrow = false, int row_step = 1, bool phased = false) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return false;
-  const int esz = fp8 ? 1 : 2, at = sample_step > 0 ? 2 : 1;  // the rows' dimension
-  const cuuint64_t row_bytes = (cuuint64_t)(ld_elems * esz);
-  cuuint64_t dims[3] = {(cuuint64_t)ld_elems, (cuuint64_t)sample_step, 0};
-  cuuint64_t strides[2] = {row_bytes, row_bytes * (cuuint64_t)sample_step};
-  cuuint32_t box[3] = {(cuuint32_t)((narrow ? kTailRowBytes : kChunkBytes) / esz), 1, 0};
-  cuuint32_t estr[3] = {1, 1, 1};
-  dims[at] = (cuuint64_t)rows;
-  box[at] = (cuuint32_t)box_rows;
-  CUresult r = fn(m, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)at + 1,
+  const int esz = fp8 ? 1 : 2;
+  const cuuint64_t step = (cuuint64_t)(row_step > 1 ? row_step : 1);
+  cuuint64_t dims[2] = {(cuuint64_t)ld_elems * (phased ? step : 1), (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)(ld_elems * esz) * step};
+  cuuint32_t box[2] = {(cuuint32_t)((narrow ? kTailRowBytes : kChunkBytes) / esz), (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(m, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   narrow ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1264,7 +1255,7 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
     it.pool_counts = f.pool_counts;
     it.q_bound = f.q_bound;
     it.db_step = f.db_step > 1 ? f.db_step : 1;
-    it.db_phased = f.db_phased ? 1 : 0;
+    it.db_phased = f.db_phased ? (int)(fp8 ? f.ld8 : f.ld16) : 0;
     it.db_scale_uniform = f.xs_uniform;
     it.fp8_tail = FORM == kFormFP8 ? (int)fp8_tail_offset(f.d, f.ld8) : 0;
     it.minima = f.minima;
@@ -1274,20 +1265,21 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
     const void* xh = fp8 ? (const void*)f.x8 : (const void*)f.xh;
     const long long ldq = fp8 ? f.ld8 : f.ld16;
     if (!MINIMA && it.db_step > 1) return cudaErrorInvalidValue;  // samples are block-minimum passes
-    const int step = MINIMA ? it.db_step : 0;
+    const int step = it.db_step;
+    const bool phased = it.db_phased != 0;
     if (!make_map(&m[kMapQHi], qh, fp8, f.nq_pad, ldq, kBM) ||
-        !make_map(&m[kMapXHi], xh, fp8, f.nb_pad, ldq, xrows, false, step))
+        !make_map(&m[kMapXHi], xh, fp8, f.nb_pad, ldq, xrows, false, step, phased))
       return cudaErrorInvalidValue;
     if (FORM == kFormExact) {
       if (!make_map(&m[kMapQLo], f.ql, false, f.nq_pad, f.ld16, kBM) ||
-          !make_map(&m[kMapXLo], f.xl, false, f.nb_pad, f.ld16, xrows, false, step))
+          !make_map(&m[kMapXLo], f.xl, false, f.nb_pad, f.ld16, xrows, false, step, phased))
         return cudaErrorInvalidValue;
     } else {
       m[kMapQLo] = m[kMapQHi];
       m[kMapXLo] = m[kMapXHi];
     }
     if (!make_map(&m[kMapQTail], qh, fp8, f.nq_pad, ldq, kBM, true) ||
-        !make_map(&m[kMapXTail], xh, fp8, f.nb_pad, ldq, xrows, true, step))
+        !make_map(&m[kMapXTail], xh, fp8, f.nb_pad, ldq, xrows, true, step, phased))
       return cudaErrorInvalidValue;
   }
   if (PAIR && bp.grid % 2) return cudaErrorInvalidValue;

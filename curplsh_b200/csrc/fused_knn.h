@@ -66,7 +66,7 @@ struct FusedLaunch {
   float xs_uniform = 0.f;   // > 0: one FP8 scale for every database row
   // database row j of this pass is stored row j * db_step (a strided sample when > 1)
   int db_step = 1;
-  int db_phased = 0;  // FusedItem::db_phased
+  int db_phased = 0;  // 1: a phased sample, see FusedItem::db_phased
   // non-null: block-minimum mode, see FusedItem::minima (pools are not used)
   float* minima = nullptr;
   int minima_rows = 128;
@@ -119,7 +119,7 @@ struct FusedItemSpec {
   int* pool_counts;         // [G*128][U]
   uint32_t* q_bound;        // [nq_pad], initialised to all ones (or to estimated bounds)
   int db_step;              // database row j is stored row j * db_step (0 or 1: contiguous)
-  int db_phased;            // FusedItem::db_phased
+  int db_phased;            // 1: a phased sample, see FusedItem::db_phased
   float* minima;            // non-null: block-minimum mode (FusedItem::minima)
   int minima_rows;          // its block rows: 128 or 8
 };

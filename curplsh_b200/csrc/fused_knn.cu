@@ -1391,8 +1391,12 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
   // FP8 pairs where a CTA's own ring is down to two stages, which no longer cover
   // the load latency: the norm tail's chunk took the third at d = 768 (pass, single
   // -> pairs: 1,842 -> 1,425 us, 1,620 before there was a tail; 1,024 2,376 ->
-  // 1,714; with three stages, d = 704, 1,385 -> 1,477)
-  const bool fp8_pair = form == kFormFP8 && d0 > 0 && make_layout(form, d0).stages < 3;
+  // 1,714; with three stages, d = 704, 1,385 -> 1,477).  Passes of a few tiles per
+  // CTA do not pay for the pair's barriers (963 rows, 708 queries, d = 960: 35 -> 41).
+  long long single_work = 0;
+  for (int i = 0; i < n; ++i)
+    single_work += (long long)((specs[i].nq + kBM - 1) / kBM) * ((specs[i].nb + kBN - 1) / kBN);
+  const bool fp8_pair = form == kFormFP8 && d0 > 0 && single_work >= 4LL * max_ctas && make_layout(form, d0).stages < 3;
   const bool want_pair = pm == 1 || (pm == kPairsAuto && ((form == kFormBF16 && d0 >= kPairMinDimBF16) ||
                                                           (form == kFormExact && d0 >= kPairMinDimExact) ||
                                                           (form == kFormFP8 && fp8_pair)));

@@ -26,7 +26,7 @@ def env():
 def test_wide_rows(env, d, estimate):
     cb, res = env
     rng = np.random.default_rng(d)
-    n, nq, k = 9001, 513, 10
+    n, nq, k = 40_001, 513, 10
     base = rng.standard_normal((n, d)).astype(np.float32)
     queries = (base[rng.choice(n, nq)] + rng.normal(0.0, 0.2, (nq, d))).astype(np.float32)
     ix = cb.IndexBF(res, d, cb.IndexBFConfig(precision=2))

@@ -782,12 +782,12 @@ cudaError_t fused_stats_print(const char* label, const FusedLaunch& f, cudaStrea
           h[kStatEpiFilter] / ctas / 8 / 1e6, h[kStatEpiRefresh] / ctas / 8 / 1e6, h[kStatRefreshes],
           h[kStatSurvivors]);
   fprintf(stderr,
-          "[fused-stats2 %s] radix passes/refresh %.2f | slow chunks %llu (%.1f%% of warp-chunks) | loop iters/slow "
-          "chunk %.2f | tmem Mcycles/warp %.2f | pair barriers Mcycles/warp %.2f\n",
+          "[fused-stats2 %s] radix passes/refresh %.2f | survivor visits %llu (%.1f%% of warp-tiles) | loop iters/visit "
+          "%.2f | pair barriers Mcycles/warp %.2f\n",
           label, h[kStatRefreshes] ? (double)h[kStatRadixPasses] / h[kStatRefreshes] : 0.0, h[kStatSlowChunks],
-          100.0 * h[kStatSlowChunks] / (ctas * 8 * (double)plan.work_per_cta * 4),
+          100.0 * h[kStatSlowChunks] / (ctas * 8 * (double)plan.work_per_cta),
           h[kStatSlowChunks] ? (double)h[kStatLoopIters] / h[kStatSlowChunks] : 0.0,
-          h[kStatTmemCycles] / ctas / 8 / 1e6, h[kStatPairBarrier] / ctas / 8 / 1e6);
+          h[kStatPairBarrier] / ctas / 8 / 1e6);
   return cudaSuccess;
 }
 #endif

@@ -128,8 +128,8 @@ struct FusedItem {
   int nb;                  // real number of database rows
   int kprime;              // candidates kept per query (before the FP32 rerank)
   int pool_cap;            // capacity of one candidate pool (entries)
-  int num_qblocks;         // G_i = ceil(nq / 128)
-  int num_tiles;           // T_i = ceil(nb / 256)
+  int num_qblocks;         // G_i = ceil(nq / R), R = 128 query rows, 256 with dual blocks and CTA pairs
+  int num_tiles;           // T_i = ceil(nb / 256), or / 128 with dual blocks
   int units_per_block;     // U_i: max units (pool lists) of one query block of this item
   int split_tiles;         // L_i: a unit never crosses a multiple of L_i tiles within its block
   long long work_begin;    // flattened offset of this item's first (block, tile)
@@ -138,8 +138,8 @@ struct FusedItem {
   const float* db_scale;   // [nb_pad] fp8 per-vector scales (FP8 form)
   const float* q_norms;    // [nq_pad]
   const float* q_scale;    // [nq_pad] (FP8 form)
-  uint64_t* pools;         // [G_i*128][U_i][pool_cap]
-  int* pool_counts;        // [G_i*128][U_i]
+  uint64_t* pools;         // [G_i*R][U_i][pool_lists][pool_cap]
+  int* pool_counts;        // [G_i*R][U_i][pool_lists]
   uint32_t* q_bound;       // [nq_pad] shared per-query bound (ordered bits), init kOrdInf or an estimate
   // Database row j of this item is stored row j * db_step (>= 1; > 1 in
   // block-minimum mode only), plus sample_phase(j / 256, db_step) when db_phased,
@@ -195,9 +195,8 @@ enum FusedStat : int {
   kStatSurvivors,              // candidates appended to pools
   kStatCtaCycles,              // sum over CTAs of kernel cycles
   kStatRadixPasses,            // histogram passes run by pool refreshes
-  kStatSlowChunks,             // warp-chunks (32 columns) that entered the survivor path
+  kStatSlowChunks,             // warp-tiles (a warp's 128 columns) that entered the survivor path
   kStatLoopIters,              // survivor-append loop iterations executed by warps
-  kStatTmemCycles,             // epilogue warps (lane 0): cycles in TMEM loads + waits
   kStatPairBarrier,            // epilogue warps (lane 0): cycles in the pair barriers
   kStatCount
 };

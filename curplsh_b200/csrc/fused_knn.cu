@@ -742,7 +742,6 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
     STAT_DECL(st_surv);
     STAT_DECL(st_slow);
     STAT_DECL(st_iters);
-    STAT_DECL(st_tmem);
     STAT_DECL(st_bar);
 #ifdef CURPLSH_FUSED_STATS
     if (threadIdx.x == 64 && B.stats) g_radix_pass_counter = &B.stats[kStatRadixPasses];
@@ -1129,7 +1128,6 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       STAT_FLUSH(kStatRefreshes, st_nref);
       STAT_FLUSH(kStatSlowChunks, st_slow);
       STAT_FLUSH(kStatLoopIters, st_iters);
-      STAT_FLUSH(kStatTmemCycles, st_tmem);
       STAT_FLUSH(kStatPairBarrier, st_bar);
     }
     STAT_FLUSH(kStatSurvivors, st_surv);
@@ -1214,11 +1212,12 @@ cudaError_t ensure_attributes() {
 
 template <int FORM, int MAXI, bool MINIMA = false, bool PAIR = false, bool DUAL = false, bool FILL = false>
 cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, int n, const FusedBatchPlan& bp,
-                        uint32_t* status, unsigned long long* stats, uint32_t smem, cudaStream_t st,
+                        uint32_t* status, unsigned long long* stats, cudaStream_t st,
                         const int* run_if) {
   cudaError_t e = ensure_attributes<FORM, MAXI, MINIMA, PAIR, DUAL, FILL>();
   if (e != cudaSuccess) return e;
-  smem = make_layout(FORM, specs[0].d, PAIR ? 1 : 0, kEpiWarps, DUAL ? 1 : 0).total;  // this instance's
+  const uint32_t smem = make_layout(FORM, specs[0].d, PAIR ? 1 : 0, kEpiWarps, DUAL ? 1 : 0).total;
+  if (smem > 227u * 1024u) return cudaErrorInvalidConfiguration;  // a layout bug, not a caller error
   FusedArgs<MAXI> a;
   memset(&a, 0, sizeof(a));
   a.B.num_items = n;
@@ -1291,32 +1290,32 @@ cudaError_t launch_form(const FusedItemSpec* specs, const FusedItemPlan* plans, 
 // for FP8 alone (plan_fused_batch).
 template <int FORM, int MAXI>
 cudaError_t launch_pools(const FusedItemSpec* specs, const FusedItemPlan* plans, int n, const FusedBatchPlan& bp,
-                         uint32_t* status, unsigned long long* stats, uint32_t smem, cudaStream_t st,
+                         uint32_t* status, unsigned long long* stats, cudaStream_t st,
                          const int* run_if) {
   if (bp.dual) {
     if constexpr (FormTraits<FORM>::kFP8)
       if (bp.fill)
-        return launch_form<FORM, MAXI, false, false, true, true>(specs, plans, n, bp, status, stats, smem, st, run_if);
-    return launch_form<FORM, MAXI, false, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if);
+        return launch_form<FORM, MAXI, false, false, true, true>(specs, plans, n, bp, status, stats, st, run_if);
+    return launch_form<FORM, MAXI, false, false, true>(specs, plans, n, bp, status, stats, st, run_if);
   }
   if (bp.pair)
-    return bp.fill ? launch_form<FORM, MAXI, false, true, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
-                   : launch_form<FORM, MAXI, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if);
-  return bp.fill ? launch_form<FORM, MAXI, false, false, false, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
-                 : launch_form<FORM, MAXI>(specs, plans, n, bp, status, stats, smem, st, run_if);
+    return bp.fill ? launch_form<FORM, MAXI, false, true, false, true>(specs, plans, n, bp, status, stats, st, run_if)
+                   : launch_form<FORM, MAXI, false, true>(specs, plans, n, bp, status, stats, st, run_if);
+  return bp.fill ? launch_form<FORM, MAXI, false, false, false, true>(specs, plans, n, bp, status, stats, st, run_if)
+                 : launch_form<FORM, MAXI>(specs, plans, n, bp, status, stats, st, run_if);
 }
 
 template <int FORM>
 cudaError_t launch_form_any(const FusedItemSpec* specs, const FusedItemPlan* plans, int n, const FusedBatchPlan& bp,
-                            uint32_t* status, unsigned long long* stats, uint32_t smem, cudaStream_t st,
+                            uint32_t* status, unsigned long long* stats, cudaStream_t st,
                             const int* run_if) {
   if (n == 1 && specs[0].minima)
-    return bp.pair ? launch_form<FORM, 1, true, true>(specs, plans, n, bp, status, stats, smem, st, run_if)
-                   : launch_form<FORM, 1, true>(specs, plans, n, bp, status, stats, smem, st, run_if);
+    return bp.pair ? launch_form<FORM, 1, true, true>(specs, plans, n, bp, status, stats, st, run_if)
+                   : launch_form<FORM, 1, true>(specs, plans, n, bp, status, stats, st, run_if);
   for (int i = 0; i < n; ++i)
     if (specs[i].minima) return cudaErrorInvalidValue;  // block-minimum mode is single-item
-  if (n == 1) return launch_pools<FORM, 1>(specs, plans, n, bp, status, stats, smem, st, run_if);
-  return launch_pools<FORM, kFusedMaxItems>(specs, plans, n, bp, status, stats, smem, st, run_if);
+  if (n == 1) return launch_pools<FORM, 1>(specs, plans, n, bp, status, stats, st, run_if);
+  return launch_pools<FORM, kFusedMaxItems>(specs, plans, n, bp, status, stats, st, run_if);
 }
 
 }  // namespace
@@ -1512,20 +1511,18 @@ cudaError_t launch_fused_batch(int form, const FusedItemSpec* specs, const Fused
   for (int i = 1; i < n; ++i)
     if (specs[i].d != specs[0].d) return cudaErrorInvalidValue;
   if (bp.grid == 0) return cudaSuccess;
-  const uint32_t smem = make_layout(form, specs[0].d, bp.pair).total;
-  if (smem > 227u * 1024u) return cudaErrorInvalidConfiguration;  // a layout bug, not a caller error
   switch (form) {
     case kFormExact:
-      return launch_form_any<kFormExact>(specs, plans, n, bp, status, stats, smem, st, run_if);
+      return launch_form_any<kFormExact>(specs, plans, n, bp, status, stats, st, run_if);
     case kFormBF16:
-      return launch_form_any<kFormBF16>(specs, plans, n, bp, status, stats, smem, st, run_if);
+      return launch_form_any<kFormBF16>(specs, plans, n, bp, status, stats, st, run_if);
     case kFormFP8: {
       // one scale per database for all items of the launch, or per-row scales for all
       const bool rows = !(specs[0].xs_uniform > 0.f);
       for (int i = 1; i < n; ++i)
         if (rows != !(specs[i].xs_uniform > 0.f)) return cudaErrorInvalidValue;
-      return rows ? launch_form_any<kFormFP8Rows>(specs, plans, n, bp, status, stats, smem, st, run_if)
-                  : launch_form_any<kFormFP8>(specs, plans, n, bp, status, stats, smem, st, run_if);
+      return rows ? launch_form_any<kFormFP8Rows>(specs, plans, n, bp, status, stats, st, run_if)
+                  : launch_form_any<kFormFP8>(specs, plans, n, bp, status, stats, st, run_if);
     }
     default:
       return cudaErrorInvalidValue;

@@ -115,8 +115,8 @@ struct FusedItemSpec {
   const float* xn;
   const float* xs;
   float xs_uniform;         // > 0: one FP8 scale for every database row
-  uint64_t* pools;          // [G*128][U][pool_cap]
-  int* pool_counts;         // [G*128][U]
+  uint64_t* pools;          // [G*R][U][pool_lists][pool_cap], see FusedItem
+  int* pool_counts;         // [G*R][U][pool_lists]
   uint32_t* q_bound;        // [nq_pad], initialised to all ones (or to estimated bounds)
   int db_step;              // database row j is stored row j * db_step (0 or 1: contiguous)
   int db_phased;            // 1: a phased sample, see FusedItem::db_phased
@@ -284,7 +284,7 @@ constexpr int kMergeMaxItems = 128;
 struct MergeItem {
   int nq, k, kprime, pool_cap, num_tiles, units_per_block;
   int pair;                // the fused launch ran CTA pairs (query groups of 256 rows)
-  int lists;               // pools of one query in one unit (2 with CTA pairs)
+  int lists;               // pools of one query in one unit (pool_lists)
   int row0;                // first pool row of this item within its fused item
   int split_tiles;         // the fused item's resolved split length L
   long long work_begin;    // the fused item's offset in its launch's flattened work space

@@ -46,14 +46,8 @@ __device__ __forceinline__ bool bar_red_or(int id, int count, bool v) {
   return r != 0;
 }
 
-// Packed FP32 pairs (sm_100): one instruction, two IEEE results rounded as
-// the scalar mul.rn / fma.rn would round them.
-__device__ __forceinline__ void mul2_f32(float& d0, float& d1, float a0, float a1, float b0, float b1) {
-  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-      "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d0), "=f"(d1)
-      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
+// A packed FP32 pair (sm_100): one instruction, two IEEE results rounded as the
+// scalar fma.rn would round them.
 __device__ __forceinline__ void fma2_f32(float& d0, float& d1, float a0, float a1, float b0, float b1, float c0,
                                          float c1) {
   asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"

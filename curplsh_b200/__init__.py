@@ -569,8 +569,9 @@ def get_coarse_check() -> bool:
 def set_cta_pairs(mode) -> None:
     """Process-wide CTA pairs mode: fused passes over >= 4 query blocks run as
     clusters of two CTAs sharing one 256-row tensor-core MMA.  True: every such
-    pass; False: none; "auto" (the default): BF16 passes with d >= 320 and
-    FP32-exact passes with d >= 192.  Results do not depend on it."""
+    pass; False: none; "auto" (the default): BF16 passes with d >= 320,
+    FP32-exact passes with d >= 192 and long FP8 passes of d = 737 to 768 and 865 to
+    1,120.  Results do not depend on it."""
     v = 2 if mode == "auto" else (1 if mode else 0)
     _check(_lib.curplsh_set_cta_pairs(v))
 

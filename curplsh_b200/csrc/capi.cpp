@@ -119,7 +119,7 @@ struct DevRes {
 // device, which keeps up to kPoolKeep bytes of freed memory for the next index
 // or workspace and goes back to the driver with the last resources that use it.
 // cudaMalloc, cudaFree and the pinned read-back took most of a one-shot search
-// (200,000 rows, 1,000 queries: 3.4 to 30 ms a call; 0.39 ms from the pool).
+// (200,000 rows, 1,000 queries: 3.4 to 30 ms a call; 0.31 ms from the pool).
 // Larger buffers come from cudaMalloc: the pool maps and unmaps them at every
 // index (10 GB in 100 to 200 ms, against 25 to 100).
 // At 512 MB three indexes of 10^6 rows opened and closed in turn had it give
@@ -626,8 +626,8 @@ constexpr int kEstimateFineRows = 8;
 constexpr int kEstimateFineMaxTiles = 64;  // 2,048 minima per query
 // Shorter searches are one or two tiles per CTA either way; from about here on the
 // sample pays (FP32-exact, d = 128, k = 10, with -> without: 3,000 rows 1 query
-// 70 -> 65 us, 16 queries 70 -> 100; 10^4 rows 66 -> 70 and 71 -> 129, 100
-// queries 76 -> 182; 40,000 rows 1 query 76 -> 151).
+// 66 -> 59 us, 16 queries 66 -> 85, 150 queries 66 -> 132; 20,000 rows 67 -> 95,
+// 69 -> 121 and 70 -> 182).
 constexpr long long kEstimateMinRows = 2048;
 
 }  // namespace

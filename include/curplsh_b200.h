@@ -288,7 +288,7 @@ int curplsh_tuning_clear(void);
 /* ------------------------------------------------------------ sampled bound estimate */
 /* No counterpart in the reference.  A search of many queries against a large database
  * (curplsh_index_search / _ex / _profiled) may first run the fused pass over a strided sample of
- * the database, keeping per query the smallest distance of every 128-row block of the sample,
+ * the database, keeping per query the smallest distance of every block of 128 (or 8) of its rows,
  * and start every candidate pool of the full pass at the j-th smallest of those block minima,
  * so far fewer rows survive the filter.  The merge pass verifies the estimate exactly (k'
  * candidates under the final bound prove the result complete); queries it fails are searched
@@ -343,13 +343,14 @@ int curplsh_get_coarse_check(int* enabled);
  * (tcgen05 cta_group::2) over two query blocks, so every database tile crosses from L2 once per
  * 256 queries instead of once per 128.  0 = off, 1 = on for every such pass, 2 = automatic (the
  * default): on for BF16 passes with d >= 320 and FP32-exact passes with d >= 192, where the
- * tensor work per tile is heavy enough for the halved tile bytes to pay (BF16 at d = 512: 5.98 ->
- * 4.54 ms for 4,096 queries over 10^6 rows; at d = 128 pairs are slower).  Results do not depend
- * on it.  Applies to searches, batches and servers planned after the call.  Process-wide. */
+ * tensor work per tile is heavy enough for the halved tile bytes to pay (BF16 at d = 512: pass
+ * 2.64 -> 1.38 ms for 4,096 queries over 500,000 rows), and for FP8 passes of d = 737 to 768 and
+ * 865 to 1,120 with four tiles per SM or more.  Results do not depend on it.  Applies to searches, batches and servers planned after the call.  Process-wide. */
 int curplsh_set_cta_pairs(int enabled);
 int curplsh_get_cta_pairs(int* enabled);
 /* Dual query blocks (engine-specific, no counterpart in cuRPLSH; on by default): a fused pass
- * over at least four 128-query blocks, where two fit shared memory, keeps two resident in each CTA and feeds each
+ * over at least four 128-query blocks, where two fit shared memory and (BF16 and FP32-exact) the
+ * pools start from an estimate, keeps two resident in each CTA and feeds each
  * 128-row database tile to two 128 x 128 tensor-core MMAs, so a tile crosses from L2 once per 256
  * queries.  Results do not depend on it.  Applies to plans made after the call; process-wide. */
 int curplsh_set_dual_blocks(int enabled);

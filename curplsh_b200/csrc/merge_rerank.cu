@@ -33,8 +33,11 @@ namespace {
 // at k' = 224, d = 128, 0.32 -> 0.28 ms); 256 win where it is large (the
 // batched workload, d up to 512: 93 -> 74 ms per graph replay).
 constexpr int kMergeSmallRerank = 65536;
-// Keys per list from which a thread walks from list to list.
-constexpr int kMergeWalkKeys = 64;
+// Lists per step of a thread (NT keys) up to which it walks from list to list
+// instead of searching: both take about as many shared-memory reads there (merge
+// of 16 queries without a bound, 10^6 rows, k' = 32, 36 keys a list: 169 us by
+// searches, 94 by walking; 9 alike).
+constexpr int kMergeWalkLists = 5;
 // Candidates one warp reranks at once: each lane keeps this many database rows
 // in flight (a row of d = 128 is one 16-byte load per lane).
 #ifndef CURPLSH_RERANK_ROWS
@@ -178,8 +181,8 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   // 312 -> 212).  A key's list comes from a binary search
   // in the offsets, four at once, or, where the lists are long, from a walk (a
   // thread's list only moves forward).  k' = 1,024, 10^6 rows, one query without a
-  // bound: 3.47 ms by searches, 1.20 by walking, 1.76 list by list; k' = 32, 2.3 x
-  // 10^6 rows, one query, nine keys a list: 23 us by searches, 43 by walking.
+  // bound: 3.47 ms by searches, 1.20 by walking, 1.76 list by list; 10^4 rows, one
+  // query, some ten keys a list: search 61.4 us with searches, 62.4 walking.
   int total = 0;
   for (int l0 = 0; l0 < nlists; l0 += NT) {
     const int l = l0 + tid;
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 12 : 6) merge_rerank_kernel(co
   constexpr int kLoads = 4;
   // f(key, on) for this thread's share of the keys, called by whole warps (on =
   // false past the end and for keys above the final bound)
-  const bool walk = total >= kMergeWalkKeys * nlists;
+  const bool walk = (long long)total * kMergeWalkLists >= (long long)NT * nlists;
   auto each_pool_key = [&](auto f) {
     int l = 0, lo = 0, hi = loff[nlists > 0 ? 1 : 0];  // list l holds the keys [lo, hi)
     for (int i0 = tid; i0 - tid < total; i0 += kLoads * NT) {

@@ -91,6 +91,8 @@ struct FormTraits<kFormFP8Rows> : FP8Traits {
 // FILL: eights of a warp's 16 with survivors from which 32 columns are taken at a
 // time (one query, 100,000 rows, k' = 1,024: pass 43 -> 25 us; 6 and 9 alike).
 constexpr int kDenseEights = 6;
+// FILL: keys that a pool may end its unit with.
+__host__ __device__ constexpr int end_limit(int kprime) { return kprime + kprime / 4; }
 
 constexpr uint32_t kAChunkBytes = kBM * kChunkBytes;  // 16 KB
 constexpr uint32_t kBChunkBytes = kBN * kChunkBytes;  // 32 KB
@@ -755,7 +757,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
       // beyond what it needs.  Short units end with some more in every pool, and
       // a selection of most of its keys frees nothing for its 10 us (k' = 224, 3,000
       // rows, 1,000 queries: pass 256 us, 44 without).
-      const int end_lim = FILL ? p.kprime + p.kprime / 4 : p.kprime;
+      const int end_lim = FILL ? end_limit(p.kprime) : p.kprime;
       if (u_ord < 0 || u_ord >= U) {  // identical in every epilogue warp: both of a pair leave here
         raise_abort(abort_flag, B.status, kErrBadSchedule);
         ok = false;
@@ -987,15 +989,6 @@ __global__ void __launch_bounds__(kNumThreads, 1) fused_knn_kernel(const __grid_
                 for (int j = 0; j < 32; ++j)
                   if (n + j < P) pool[n + j] = make_key(key_d(x[j]), (uint32_t)(c0 + j));
                 m = 0u;
-              }
-              if (__any_sync(0xffffffffu, __popc(m) > 4)) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                  const bool take = (m >> j) & 1u;
-                  if (take && n < P) pool[n] = make_key(key_d(x[j]), (uint32_t)(c0 + j));
-                  n += take ? 1 : 0;
-                }
-                continue;
               }
 #pragma unroll 1
               while (__any_sync(0xffffffffu, m != 0u)) {
@@ -1369,10 +1362,11 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
   }
   // Pools that start without a bound fill to k' keys in every unit, and a dual
   // unit has half the rows at the same CTA range, so there are twice as many and
-  // the bounds tighten later.  BF16 and FP32-exact keep single blocks then (1,000
-  // queries, k' = 32, single -> dual: FP32-exact, 100,000 rows 472 -> 686 us;
-  // BF16, 10^6 rows 1,042 -> 1,311; k' = 200 1,877 -> 2,024); FP8, whose MMAs are
-  // light, does not (k' = 480, 8,000 rows 254 -> 63 us).
+  // the bounds tighten later: such passes keep single blocks (1,000 queries, single
+  // -> dual: FP32-exact, k' = 32, 100,000 rows 472 -> 686 us; BF16, 10^6 rows 1,042
+  // -> 1,311; FP8, k' = 480, 100,000 rows 697 -> 877).  FP8's light MMAs pay for dual
+  // blocks where the half unit alone ends without a selection (k' = 480, 3,000 rows,
+  // 4,000 queries: 166 -> 82; k' = 1,216, 100,000 rows, 1,000: 2,728 -> 1,719).
   bool fill = false, lean = false;
   int kp_min = 1 << 30;
   for (int i = 0; i < n; ++i) {
@@ -1380,7 +1374,18 @@ void plan_fused_batch(const FusedItemSpec* specs, int n, int max_ctas, FusedItem
     if (specs[i].fill_kprime > 0) kp_min = std::min(kp_min, specs[i].fill_kprime);
     lean = lean || specs[i].lean;
   }
-  const bool dual_pays = !fill || form == kFormFP8;
+  bool dual_pays = !fill;
+  if (fill && form == kFormFP8) {
+    long long work = 0;
+    for (int i = 0; i < n; ++i)
+      work += (long long)((specs[i].nq + kBM - 1) / kBM) * ((specs[i].nb + kBN - 1) / kBN);
+    const long long w = (work + max_ctas - 1) / max_ctas;
+    for (int i = 0; i < n; ++i) {
+      const long long rows = kBN * (specs[i].split_tiles > 0 ? std::min<long long>(w, specs[i].split_tiles) : w);
+      const int lim = end_limit(specs[i].fill_kprime);
+      dual_pays = dual_pays || (specs[i].fill_kprime > 0 && rows > lim && rows <= 2LL * lim);
+    }
+  }
   // Two query blocks per CTA: a database tile crosses L2 -> SM once per 256
   // queries, and every query's pool belongs to one lane (full pass, single ->
   // dual blocks: BF16 integer mixture 3.50 -> 2.84 ms, FP32-exact 5.64 -> 4.70)

@@ -349,8 +349,8 @@ int curplsh_get_coarse_check(int* enabled);
 int curplsh_set_cta_pairs(int enabled);
 int curplsh_get_cta_pairs(int* enabled);
 /* Dual query blocks (engine-specific, no counterpart in cuRPLSH; on by default): a fused pass
- * over at least four 128-query blocks, where two fit shared memory and (BF16 and FP32-exact) the
- * pools start from an estimate, keeps two resident in each CTA and feeds each
+ * over at least four 128-query blocks, where two fit shared memory and the pools start
+ * from an estimate (FP8: not only then), keeps two resident in each CTA and feeds each
  * 128-row database tile to two 128 x 128 tensor-core MMAs, so a tile crosses from L2 once per 256
  * queries.  Results do not depend on it.  Applies to plans made after the call; process-wide. */
 int curplsh_set_dual_blocks(int enabled);

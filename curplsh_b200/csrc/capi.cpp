@@ -629,6 +629,11 @@ constexpr int kEstimateFineMaxTiles = 64;  // 2,048 minima per query
 // 66 -> 59 us, 16 queries 66 -> 85, 150 queries 66 -> 132; 20,000 rows 67 -> 95,
 // 69 -> 121 and 70 -> 182).
 constexpr long long kEstimateMinRows = 2048;
+// Light samples are phased from here on.  Where half of a sample's tiles start off a
+// 32-byte boundary their loads take longer (10^4 rows, 100 queries: 64.0 -> 65.2 us
+// a search), and below this a pass that runs again for rows stored with a period is
+// short.
+constexpr long long kEstimatePhasedTiles = 64;
 
 }  // namespace
 
@@ -682,6 +687,7 @@ EstimatePlan plan_estimate(int nq, long long n, int kp, int num_sms, bool lean) 
       j = r;
     }
     if (j == 0) return e;
+    e.phased = T >= kEstimatePhasedTiles;
   }
   e.rows = (int)(tiles * kBN);
   e.step = (int)(n / e.rows);  // rows i * step < n for every i < rows
@@ -862,7 +868,7 @@ int search_device(curplsh_index* ix, const SearchShape& sh, int nq, const float*
     e.nb = sh.est.rows;
     e.nb_pad = sh.est.rows;
     e.db_step = sh.est.step;
-    e.db_phased = sh.est.light;
+    e.db_phased = sh.est.phased;
     e.kprime = 1;
     e.minima = b.minima;
     e.minima_rows = sh.est.block_rows;

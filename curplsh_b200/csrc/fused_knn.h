@@ -169,8 +169,9 @@ cudaError_t launch_fused_batch(int form, const FusedItemSpec* specs, const Fused
 struct EstimatePlan {
   bool on = false;
   bool light = false;  // sized by cost, not by expected rows (see capi.cpp)
+  bool phased = false;  // each tile's rows start at another of the step's rows (sample_phase)
   int rows = 0;    // sample rows (a multiple of 256)
-  int step = 1;    // sample row j is database row j * step, plus, in a light sample, its tile's sample_phase
+  int step = 1;    // sample row j is database row j * step, plus, when phased, its tile's sample_phase
   int block_rows = 128;  // or 8
   int blocks = 0;  // B = rows / block_rows block minima per query
   int j = 0;       // rank of the estimate among the block minima

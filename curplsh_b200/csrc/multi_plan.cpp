@@ -353,7 +353,7 @@ int MultiPlan::enqueue(cudaStream_t main, const std::vector<cudaStream_t>* branc
       e.xs = s.xs;
       e.xs_uniform = s.xs_uniform;
       e.db_step = x.est.step;
-      e.db_phased = x.est.light;
+      e.db_phased = x.est.phased;
       e.minima = reinterpret_cast<float*>(base_ + x.o_minima);
       e.minima_rows = x.est.block_rows;
       e.pools = s.pools;

@@ -314,8 +314,8 @@ int curplsh_estimate_plan_shape(int64_t num_rows, int64_t num_queries, int kprim
                                 int* step, int* rank);
 /* The estimate such a search starts from, regular or light: *rank is that among the
  * sample_rows / block_rows block minima, and *sample_rows = 0 means that it uses none.  Sample
- * row i is database row i * step of a regular sample; a light one adds the next digit of a
- * golden-ratio sequence, floor(frac(floor(i / 256) * 2654435769 / 2^32) * step), so that rows
+ * row i is database row i * step of a regular sample; a light one of 16,129 database rows and more adds the next
+ * term of a golden-ratio sequence, floor(frac(floor(i / 256) * 2654435769 / 2^32) * step), so that rows
  * stored with a period that divides the step are sampled alike. */
 int curplsh_index_estimate_sample(curplsh_index* index, int64_t num_queries, int k, int precision,
                                   int rerank_factor, int* sample_rows, int* step, int* block_rows, int* rank);

@@ -83,10 +83,10 @@ def test_forms_agree_with_and_without_a_light_sample(env, form, spread, n, nq, k
     assert failed == 0
 
 
-def _sampled_rows(rows, step):
+def _sampled_rows(n, rows, step):
     """Database rows of a light sample (curplsh_index_estimate_sample)."""
     i = np.arange(rows, dtype=np.uint64)
-    phase = ((i // 256 * 2654435769) % 2**32 * step) >> np.uint64(32)
+    phase = ((i // 256 * 2654435769) % 2**32 * step) >> np.uint64(32) if n > 63 * 256 else 0
     return (i * step + phase).astype(np.int64)
 
 
@@ -106,7 +106,7 @@ def test_a_light_sample_that_fails(env, n, nq, k, host):
     ix.add(n, base)
     assert ix.estimate_plan(nq, k)[0] == 0
     rows, step, _, rank = ix.estimate_sample(nq, k)
-    at = _sampled_rows(rows, step)
+    at = _sampled_rows(n, rows, step)
     assert 0 < rank < 24 and at.max() < n and len(np.unique(at)) == rows
     ix.reset()
     base[at] -= np.float32(50.0)
